@@ -108,12 +108,19 @@ class GPT(nn.Module):
         cfg, be = self.cfg, self.backend
         ids_flat = ids.reshape(-1)
         aux_total = None
+        whole_layer = getattr(be, "dense_layer", None)
         for bi, blk in enumerate(self.blocks):
             l = blk.layer
             if self.grad_bucket_cb is not None and l in self.grad_bucket_boundaries and x.requires_grad:
                 cb, b = self.grad_bucket_cb, self.grad_bucket_boundaries[l]
                 x.register_hook(lambda g, cb=cb, b=b: cb(b))
             with nvtx_range(f"layer {l}"):
+                if whole_layer is not None:
+                    y = whole_layer(x, x0, self.resid_lambdas, self.x0_lambdas, bi, blk, ids_flat, B, T, cfg, self.rope_cos,
+                                    self.rope_sin, cfg.window(l))
+                    if y is not None:
+                        x = y
+                        continue
                 x, xn = be.resid_scale_norm(x, x0, self.resid_lambdas, self.x0_lambdas, bi)
                 a = be.attention_block(xn, blk, ids_flat, B, T, cfg, self.rope_cos, self.rope_sin,
                                        cfg.window(l))

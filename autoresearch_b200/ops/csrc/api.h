@@ -236,4 +236,21 @@ int arb_moe_combine_bwd(const void* d_out, void* const* y_bufs, const void* y_ro
                         const int* idx, const int* row, const float* gates, float* d_gates, long long N, int K, int D,
                         int E, cudaStream_t s);
 
+// ---- one dense layer per call (layer.cu): the same kernels as the entry points above, started from native code ----
+typedef struct {
+  // forward: inputs, parameters, the buffer for what the layer keeps (bf16 [N, 8 D + M] then four times
+  // fp32 [N, H], each rounded up to 4 floats), output [N, D]
+  const void *x, *x0, *lam_r, *lam_0, *wqkv, *wo, *wfc, *wdn, *ve, *gate_w, *ids, *cos_t, *sin_t;
+  void *kept, *out, *err;
+  // backward: incoming gradient [N, D], scratch, input gradients (d_x0_acc as in arb_resid_scale_norm_bwd), fp32 gradients
+  const void* g;
+  void *work, *d_x, *d_x0;
+  const void* d_x0_acc;
+  void *g_lam_r, *g_lam_0, *g_wqkv, *g_wo, *g_wfc, *g_wdn, *g_gate;
+  long long B, T, H, M, window, idx, gate_ch, fuse_post;
+  double eps, scale;
+} ArbLayer;
+int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s);
+int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s);
+
 }  // extern "C"

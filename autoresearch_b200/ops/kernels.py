@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from typing import Optional
 
 import torch
@@ -107,6 +108,8 @@ def _signatures() -> dict:
         "arb_moe_finish_dispatch": [vp, vp, vp, i32, i32, i32, i32, i32, vp],
         "arb_moe_combine_fwd": [vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, vp],
         "arb_moe_combine_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, vp],
+        "arb_layer_fwd": [vp, vp, vp],
+        "arb_layer_bwd": [vp, vp, vp],
     }
 
 
@@ -294,6 +297,18 @@ def flush_pending_pulls() -> None:
     dst = (C.c_void_p * n)(*[k for k, _ in items])
     nb = (C.c_longlong * n)(*[v[1] for _, v in items])
     _check(lib().arb_pull_ranges(src, dst, nb, n, _stream()), "pull_ranges")
+
+
+_LAYER = struct.Struct("=36q2d")        # ArbLayer of csrc/api.h: 28 pointers, 8 sizes, eps and scale
+
+
+def layer_call(entry: str, pointers, sizes, eps: float, scale: float) -> None:
+    """arb_layer_fwd / arb_layer_bwd with the fields of ArbLayer in order (absent pointers are 0)."""
+    global launch_count
+    n = C.c_int(0)
+    rc = getattr(lib(), entry)(_LAYER.pack(*pointers, *sizes, eps, scale), C.addressof(n), _stream())
+    launch_count += max(0, n.value - 1)
+    _check(rc, entry)
 
 
 def attn_set_mode(mode: int) -> None:

@@ -399,6 +399,67 @@ class AttentionFn(torch.autograd.Function):
         return d_qkv, None, None, None, None
 
 
+class DenseLayerFn(torch.autograd.Function):
+    """A whole dense layer, launched by one native call per direction (csrc/layer.cu): the kernels, their order and their
+    arguments are those of ResidScaleNormFn, AttnPreFn, AttentionFn, LinearAddNormFn and MLPFn in a row.  What the layer
+    keeps for its backward pass is one buffer."""
+
+    @staticmethod
+    def forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, B, T, window, idx, gate_ch, eps, chain):
+        N, D = x.shape
+        M, H = wfc.shape[0], D // 128
+        stat = (N * H + 3) // 4 * 8                            # fp32 [N, H] in bf16 elements; lse, rstd of q and k, gate
+        kept = torch.empty(N * (8 * D + M) + 4 * stat, dtype=torch.bfloat16, device=x.device)
+        out = torch.empty_like(x)
+        sizes = (B, T, H, M, window, idx, gate_ch, int(K.qkv_post_fusable(N, 3 * D)))
+        ptrs = [t.data_ptr() for t in (x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn)]
+        ptrs += (ve.data_ptr(), gate_w.data_ptr()) if ve is not None else (0, 0)
+        ptrs += (ids.data_ptr(), cos.data_ptr(), sin.data_ptr(), kept.data_ptr(), out.data_ptr(), K.err_flag(x.device).data_ptr())
+        K.layer_call("arb_layer_fwd", ptrs + [0] * 12, sizes, eps, 1.0 / math.sqrt(128.0))
+        ctx.save_for_backward(x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept)
+        ctx.sizes, ctx.eps, ctx.chain = sizes, eps, chain
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept = ctx.saved_tensors
+        B, T, H, M, _, idx, gate_ch, _ = ctx.sizes
+        chain = ctx.chain
+        N, D = x.shape
+        dev = x.device
+        if K.pending_pulls:
+            K.flush_pending_pulls()
+        g = g.contiguous()
+        params = (lam_r, lam_0, wqkv, wo, wfc, wdn) + ((gate_w,) if ve is not None else ())
+        mains = [_main_grad(p) for p in params]
+        accs = [m if m is not None else torch.zeros(p.shape, dtype=torch.float32, device=dev) for m, p in zip(mains, params)]
+        wide = max(M, 4 * D)
+        work = torch.empty(N * (wide + 2 * D + gate_ch) + 8 + 2 * ((N * H + 3) // 4 * 8), dtype=torch.bfloat16, device=dev)
+        dx = torch.empty_like(x)
+        acc0 = chain.buf
+        dx0 = acc0 if acc0 is not None else torch.empty_like(x)
+        ptrs = [t.data_ptr() for t in (x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn)]
+        ptrs += (ve.data_ptr(), gate_w.data_ptr()) if ve is not None else (0, 0)
+        ptrs += (ids.data_ptr(), cos.data_ptr(), sin.data_ptr(), kept.data_ptr(), 0, K.err_flag(dev).data_ptr(),
+                 g.data_ptr(), work.data_ptr(), dx.data_ptr(), dx0.data_ptr(), dx0.data_ptr() if acc0 is not None else 0)
+        ptrs += [t.data_ptr() for t in accs] + ([0] if ve is None else [])
+        K.layer_call("arb_layer_bwd", ptrs, ctx.sizes, ctx.eps, 1.0 / math.sqrt(128.0))
+        g_ve = None
+        if ve is not None:
+            d_ve = work[3 * N * D:4 * N * D].view(N, D)
+            mgv = _main_grad(ve)
+            acc = mgv if mgv is not None else torch.zeros(ve.shape, dtype=torch.float32, device=dev)
+            K.embedding_bwd(ids, d_ve, acc)
+            g_ve = None if mgv is not None else acc.to(ve.dtype)
+        chain.buf = dx0
+        if idx != 0:
+            dx0 = None              # still being summed; layer 0 of the stage returns it
+        else:
+            chain.buf = None
+        gp = [None if m is not None else a.to(p.dtype) for m, a, p in zip(mains, accs, params)]
+        return (dx, dx0, *gp[:6], g_ve, gp[6] if ve is not None else None) + (None,) * 10
+
+
 class LibraryAttentionFn(torch.autograd.Function):
     """Library attention on the packed buffer (a comparison arm: everything else stays on this package's kernels):
     cuDNN's fused attention through torch SDPA for full-causal layers, flash-attn 2 for sliding windows."""
@@ -592,6 +653,7 @@ class Sm100Backend(OracleBackend):
         K.lib()  # fail loudly when the native library is missing
         self.attn = attn
         self.big_ce_chunk = 16384
+        self.layer_calls = True       # False: one autograd node and one native call per step of a layer
         self._x0_chain = None
 
     def optim_kernels(self):
@@ -609,7 +671,32 @@ class Sm100Backend(OracleBackend):
         # layers are visited in order within one forward pass: index 0 opens a new x0-gradient chain
         if i == 0 or self._x0_chain is None:
             self._x0_chain = _X0GradChain()
-        return ResidScaleNormFn.apply(x.contiguous(), x0.contiguous(), lam_r, lam_0, i, self.eps, self._x0_chain)
+        return self._x0_chain
+
+    def resid_scale_norm(self, x, x0, lam_r, lam_0, i):
+        return ResidScaleNormFn.apply(x.contiguous(), x0.contiguous(), lam_r, lam_0, i, self.eps, self._chain(i))
+
+    def dense_layer(self, x, x0, lam_r, lam_0, i, blk, ids_flat, B, T, cfg, cos, sin, window):
+        """The whole layer through DenseLayerFn, or None where its steps have to run one by one: experts, tensor
+        parallelism, the library attention, parameters that still wait to be copied from their owner by the GEMMs that use
+        them, and operands that are not the dense bf16 tensors the native call takes (the separate steps say what is wrong)."""
+        if not self.layer_calls or blk.router is not None or self._tp() is not None or self.attn != "own" or K.pending_pulls:
+            return None
+        N, D = x.shape
+        M = blk.wfc.shape[0]
+        want = [(x, (N, D)), (x0, (N, D)), (blk.wqkv, (3 * D, D)), (blk.wo, (D, D)), (blk.wfc, (M, D)), (blk.wdn, (D, M)),
+                (lam_r, lam_r.shape), (lam_0, lam_0.shape), (cos, (cos.shape[0], 64)), (sin, (cos.shape[0], 64))]
+        if blk.ve is not None:
+            want += [(blk.ve, (blk.ve.shape[0], D)), (blk.ve_gate, (D // 128, cfg.ve_gate_ch))]
+        dev = x.device
+        for t, shape in want:
+            if t.dtype is not torch.bfloat16 or t.shape != shape or t.device != dev or not t.is_contiguous():
+                return None
+        if (N != B * T or D % 128 or cfg.head_dim != 128 or M % 8 or cos.shape[0] < T or ids_flat.dtype is not torch.int32 or
+                ids_flat.shape != (N,) or ids_flat.device != dev or not ids_flat.is_contiguous() or not x.is_cuda):
+            return None
+        return DenseLayerFn.apply(x, x0, lam_r, lam_0, blk.wqkv, blk.wo, blk.wfc, blk.wdn, blk.ve, blk.ve_gate, ids_flat, cos, sin,
+                                  B, T, window, i, cfg.ve_gate_ch, self.eps, self._chain(i))
 
     def linear_col(self, x, w):
         return LinearFn.apply(x, w)

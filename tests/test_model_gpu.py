@@ -64,3 +64,45 @@ def test_training_step_sm100_loss_decreases():
     losses = [float(tr.train_step()) for _ in range(30)]
     K.check_err_flag()
     assert losses[-1] < losses[0] - 0.3, losses
+
+
+@pytest.mark.parametrize("batch,seq,layers,heads", [(1, 512, 4, 2), (3, 331, 6, 2), (1, 130, 2, 2), (3, 301, 3, 3), (1, 3, 1, 1)])
+def test_whole_layer_calls_give_the_bits_of_the_separate_steps(batch, seq, layers, heads):
+    """One native call per layer and direction against one autograd node per step: the same kernels on the same operands, so
+    losses agree bit for bit and matrix gradients up to the order in which split-K sums meet.  130 rows take the separate
+    rotation kernel (products below the 2-CTA tiles), 993 end inside a tile, 903 x 3 leaves the row statistics at odd offsets."""
+    from autoresearch_b200.config import ModelConfig
+    from autoresearch_b200.ops import kernels as K
+    cfg = ModelConfig(vocab=1024, seq_len=512, d_model=128 * heads, n_head=heads, head_dim=128, mlp_dim=512 * heads,
+                      n_layer=layers)
+    torch.manual_seed(3)
+    mod = _build("sm100", cfg, torch.bfloat16)
+    ids = torch.randint(0, cfg.vocab, (batch, seq), device="cuda", dtype=torch.int32)
+    tgt = torch.randint(0, cfg.vocab, (batch, seq), device="cuda", dtype=torch.int32)
+    got = {}
+    for whole in (True, False):
+        mod.backend.layer_calls = whole
+        for with_main in (False, True):          # gradients handed to autograd, and summed into fp32 main gradients
+            for p in mod.parameters():
+                p.grad = None
+                if with_main:
+                    p.main_grad = torch.zeros(p.shape, dtype=torch.float32, device="cuda")
+                elif hasattr(p, "main_grad"):
+                    del p.main_grad
+            loss, per_tok = mod(ids, tgt, grad_scale=1.0 / ids.numel())
+            loss.backward()
+            got[whole, with_main] = (per_tok.clone(), [(p.main_grad if with_main else p.grad).clone() for p in mod.parameters()])
+        with torch.no_grad():
+            got[whole, "eval"] = mod(ids, tgt)[1].clone()
+    K.check_err_flag()
+    names = [n for n, _ in mod.named_parameters()]
+    assert torch.equal(got[True, "eval"], got[False, "eval"])
+    for with_main in (False, True):
+        a, b = got[True, with_main], got[False, with_main]
+        assert torch.equal(a[0], b[0])
+        for n, x, y in zip(names, a[1], b[1]):
+            if "lambdas" in n or "ve_gate" in n:
+                assert (x - y).float().norm() <= 1e-2 * y.float().norm() + 1e-6, n      # atomics; bf16 gradients: one rounding
+            else:
+                # fp32 split-K sums meet in L2 in any order: a few units in the last place of the largest partial sum
+                assert (x.float() - y.float()).norm() <= (1e-5 if with_main else 4e-3) * y.float().norm(), n
