@@ -667,7 +667,7 @@ class Sm100Backend(OracleBackend):
     def rmsnorm(self, x):
         return RMSNormFn.apply(x.contiguous(), self.eps)
 
-    def resid_scale_norm(self, x, x0, lam_r, lam_0, i):
+    def _chain(self, i):
         # layers are visited in order within one forward pass: index 0 opens a new x0-gradient chain
         if i == 0 or self._x0_chain is None:
             self._x0_chain = _X0GradChain()
