@@ -79,20 +79,37 @@ struct GemmArgs {
   QkvPostArgs qp;
 };
 
-// K blocks of [kb0, kb1) of batch item b that are multiplied
-__device__ __forceinline__ bool kb_live(const GemmArgs& p, int b, int kb) {
-  if (!p.k_valid) return true;
-  const int seg = kb / p.k_seg_kb;
-  return (kb - seg * p.k_seg_kb) * BK < p.k_valid[b * p.k_nseg + seg];
-}
+// The K blocks of [kb0, kb1) of batch item b that are multiplied, in order.  The bound of the current segment is read once
+// per segment: testing every block (a division and a load each, in the producer and in the issuing thread) held the weight
+// gradients of eight experts at 950 TFLOP/s, where the same shapes without k_valid run at 1330 (training pass of the 2.2 B
+// model, 4 x 8192 tokens, together with the router kernel of moe.cu: 170.3 -> 160.3 ms).
+struct LiveK {
+  const GemmArgs& p;
+  int kb, kb1, end, seg, b;       // next block; end of the range; end of the live blocks of segment `seg`
+  __device__ __forceinline__ LiveK(const GemmArgs& args, int item, int kb0, int kb_end) : p(args), kb(kb0), kb1(kb_end), b(item) {
+    seg = 0;
+    end = kb1;
+    if (p.k_valid) { seg = kb / p.k_seg_kb; bound(); }
+  }
+  __device__ __forceinline__ void bound() {
+    const int blocks = min(p.k_seg_kb, (p.k_valid[b * p.k_nseg + seg] + BK - 1) / BK);
+    end = min(kb1, seg * p.k_seg_kb + max(blocks, 0));
+  }
+  __device__ __forceinline__ bool more() {
+    if (kb < end) return true;
+    if (!p.k_valid) return false;
+    while (kb >= end) {
+      ++seg;
+      kb = seg * p.k_seg_kb;
+      if (kb >= kb1) return false;
+      bound();
+    }
+    return true;
+  }
+};
 __device__ __forceinline__ bool item_live(const GemmArgs& p, int b, int m_start, int kb0, int kb1) {
   if (p.m_valid && m_start >= p.m_valid[b]) return false;
-  if (p.k_valid) {
-    for (int kb = kb0; kb < kb1; ++kb)
-      if (kb_live(p, b, kb)) return true;
-    return false;
-  }
-  return true;
+  return !p.k_valid || LiveK(p, b, kb0, kb1).more();
 }
 
 __device__ __forceinline__ uint4 ld_peer16(const uint4* a) {
@@ -277,8 +294,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
         if (!item_live(p, b, mt * BM, kb0, kb1)) continue;
         const int bB = b / p.b_div;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!kb_live(p, b, kb)) continue;
+        for (LiveK k_it(p, b, kb0, kb1); k_it.more(); ++k_it.kb) {
+          const int kb = k_it.kb;
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           ++it;
@@ -329,8 +346,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         bool first = true;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!kb_live(p, b, kb)) continue;
+        for (LiveK k_it(p, b, kb0, kb1); k_it.more(); ++k_it.kb) {
+          const int kb = k_it.kb;
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           ++it;
@@ -537,8 +554,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int n0 = nt * 256 + int(rank) * 128;
         if (!item_live(p, b, mt * 256, kb0, kb1)) continue;
         const int bB = b / p.b_div;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!kb_live(p, b, kb)) continue;
+        for (LiveK k_it(p, b, kb0, kb1); k_it.more(); ++k_it.kb) {
+          const int kb = k_it.kb;
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           ++it;
@@ -584,8 +601,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN2;
         bool first = true;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!kb_live(p, b, kb)) continue;
+        for (LiveK k_it(p, b, kb0, kb1); k_it.more(); ++k_it.kb) {
+          const int kb = k_it.kb;
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           ++it;

@@ -145,3 +145,23 @@ def test_slot_positions_match_token_order_prefix_sum():
         ref = (onehot.cumsum(0) - 1).gather(1, idx.long().view(-1, 1)).squeeze(1)
         assert torch.equal(pos.long(), ref)
         assert torch.equal(counts.long(), onehot.sum(0))
+
+
+@pytest.mark.parametrize("N,D,E,K_", [(1, 128, 4, 2), (9, 1024, 8, 2), (20011, 384, 8, 1), (3000, 264, 5, 4), (700, 4096, 16, 2)])
+def test_router_against_64_bits(N, D, E, K_):
+    """More and fewer tokens than resident warps, expert counts with and without their own kernel, rows of any width and router
+    matrices of any size that fits shared memory: fp32 logits of D products, so 1e-5; the selection is the top of the
+    probabilities the kernel itself wrote, ties to the lower index."""
+    from autoresearch_b200.ops import kernels as K
+    torch.manual_seed(N + D)
+    xn, wr = torch.randn(N, D, device="cuda").bfloat16(), (torch.randn(E, D, device="cuda") * 0.05).bfloat16()
+    probs, gates = torch.empty(N, E, device="cuda"), torch.empty(N, K_, device="cuda")
+    idx = torch.empty(N, K_, device="cuda", dtype=torch.int32)
+    K._check(K.lib().arb_moe_router_fwd(xn.data_ptr(), wr.data_ptr(), probs.data_ptr(), idx.data_ptr(), gates.data_ptr(), N, D, E, K_,
+                                        K._stream()), "moe_router_fwd")
+    want = torch.softmax(xn.double() @ wr.double().t(), -1)
+    assert (probs.double() - want).abs().max().item() < 1e-5
+    order = torch.sort(probs, -1, descending=True, stable=True).indices[:, :K_]
+    assert torch.equal(order.int(), idx)
+    top = probs.gather(1, idx.long())
+    assert (gates - top / top.sum(-1, keepdim=True)).abs().max().item() < 1e-5
