@@ -147,6 +147,10 @@ int arb_embedding_bwd(const int* ids, const void* g, float* dw, long long N, int
 int arb_embedding_bwd_sorted(const long long* perm, const int* item_id, const int* item_start, const int* seg_start,
                              const int* seg_count, const void* g, float* dw, float* partial, int n_items_max, int D, int R,
                              int vocab, cudaStream_t s);
+// The tables of arb_embedding_bwd_sorted for one batch of ids: hist = ceil(N / 1024) * vocab ints of scratch; perm [N],
+// counts / seg_start / item_start [vocab], item_id [n_items_max >= N / R + vocab].  vocab <= 49152.
+int arb_embedding_plan(const int* ids, long long N, int vocab, int R, int n_items_max, int* hist, long long* perm, int* counts,
+                       int* seg_start, int* item_start, int* item_id, cudaStream_t s);
 int arb_add_cols(void* dst, long long ld_dst, const void* src, long long rows, int cols, cudaStream_t s);
 int arb_cast_f32_to_bf16(const float* src, void* dst, long long n, float scale, cudaStream_t s);
 int arb_accum_bf16_into_f32(const void* src, float* dst, long long n, cudaStream_t s);

@@ -34,6 +34,9 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
 }
 
+// Keeps the compiler from carrying the unpacked form of u across this point (it would, at twice the registers)
+__device__ __forceinline__ void stay_packed(uint4& u) { asm volatile("" : "+r"(u.x), "+r"(u.y), "+r"(u.z), "+r"(u.w)); }
+
 constexpr int ROWS_PER_CTA = 8;  // 8 warps, one row each
 
 // ---------------------------------------------------------------------------------------------
@@ -77,16 +80,34 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_k(const __nv_bfloat16* __rest
   const long long row = (long long)blockIdx.x * ROWS_PER_CTA + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int nch = D >> 3;
-  float xv[NV][8], gv[NV][8];
+  // the row stays packed (4 registers per 8 values) between the two passes, and all loads are issued before the reductions.
+  // With fp32 copies the kernel took 81 us at 8192 x 2048 and 70 us at 32768 x 1024, where four passes over memory are 21 and
+  // 41 us at the copy rate.
+  uint4 xq[NV], gq[NV], aq[NV];
   float ss = 0.f, dot = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = lane + 32 * i;
     if (c < nch) {
-      ld8(x + row * D + c * 8, xv[i]);
-      ld8(g + row * D + c * 8, gv[i]);
+      xq[i] = *reinterpret_cast<const uint4*>(x + row * D + c * 8);
+      gq[i] = *reinterpret_cast<const uint4*>(g + row * D + c * 8);
+    }
+  }
+  if (NV <= 8 && add_to) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { ss += xv[i][j] * xv[i][j]; dot += xv[i][j] * gv[i][j]; }
+    for (int i = 0; i < NV; ++i) {
+      const int c = lane + 32 * i;
+      if (c < nch) aq[i] = *reinterpret_cast<const uint4*>(add_to + row * D + c * 8);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = lane + 32 * i;
+    if (c < nch) {
+      float xv[8], gv[8];
+      unpack8(xq[i], xv); unpack8(gq[i], gv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { ss += xv[j] * xv[j]; dot += xv[j] * gv[j]; }
     }
   }
   ss = warp_sum(ss);
@@ -97,11 +118,13 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_k(const __nv_bfloat16* __rest
   for (int i = 0; i < NV; ++i) {
     const int c = lane + 32 * i;
     if (c < nch) {
-      float o[8];
-      if (add_to) ld8(add_to + row * D + c * 8, o);
+      float o[8], xv[8], gv[8];
+      stay_packed(xq[i]); stay_packed(gq[i]);
+      unpack8(xq[i], xv); unpack8(gq[i], gv);
+      if (add_to) { if (NV <= 8) unpack8(aq[i], o); else ld8(add_to + row * D + c * 8, o); }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float t = r * (gv[i][j] - xv[i][j] * coef);
+        const float t = r * (gv[j] - xv[j] * coef);
         o[j] = add_to ? o[j] + t : t;
       }
       st8(gx + row * D + c * 8, o);
@@ -170,7 +193,7 @@ __global__ void __launch_bounds__(256) resid_norm_bwd_k(const __nv_bfloat16* __r
   if (row < rows) {
     // the row is kept as packed bf16 (4 registers per 8 values) between the two passes: with fp32 copies of
     // three arrays the kernel needed 127 registers and ran at a quarter of the possible occupancy
-    uint4 xq[NV], bq[NV], gq[NV];
+    uint4 xq[NV], bq[NV], gq[NV], sq[NV];
     float ss = 0.f, dot = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -179,6 +202,13 @@ __global__ void __launch_bounds__(256) resid_norm_bwd_k(const __nv_bfloat16* __r
         xq[i] = *reinterpret_cast<const uint4*>(x + row * D + c * 8);
         bq[i] = *reinterpret_cast<const uint4*>(x0 + row * D + c * 8);
         gq[i] = *reinterpret_cast<const uint4*>(g_xn + row * D + c * 8);
+        if (NV <= 8) sq[i] = *reinterpret_cast<const uint4*>(g_xs + row * D + c * 8);   // needed behind the reductions only
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = lane + 32 * i;
+      if (c < nch) {
         float xv[8], bv[8], gv[8];
         unpack8(xq[i], xv); unpack8(bq[i], bv); unpack8(gq[i], gv);
 #pragma unroll
@@ -198,8 +228,9 @@ __global__ void __launch_bounds__(256) resid_norm_bwd_k(const __nv_bfloat16* __r
       const int c = lane + 32 * i;
       if (c < nch) {
         float gs[8], o1[8], o2[8], xv[8], bv[8], gv[8], av[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        ld8(g_xs + row * D + c * 8, gs);
+        if (NV <= 8) unpack8(sq[i], gs); else ld8(g_xs + row * D + c * 8, gs);
         if (d_x0_acc) ld8(d_x0_acc + row * D + c * 8, av);
+        stay_packed(xq[i]); stay_packed(bq[i]); stay_packed(gq[i]);
         unpack8(xq[i], xv); unpack8(bq[i], bv); unpack8(gq[i], gv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -319,11 +350,16 @@ __global__ void embedding_bwd_k(const int* __restrict__ ids, const __nv_bfloat16
 // row (it is the only writer), longer ids leave per-item partial sums that embedding_bwd_combine_k adds up in
 // item order.  No atomics: the result does not depend on scheduling (the reference's histogram kernel,
 // brain/kernels/embedding.cu, and the kernel above both rely on the order of atomic adds).
-__global__ void __launch_bounds__(128) embedding_bwd_sorted_k(const long long* __restrict__ perm, const int* __restrict__ item_id,
+// A CTA's 256 threads take D / 8 columns times 256 / (D / 8) row groups (at least one): a group sums every n-th row, four rows
+// in flight, and the groups' sums meet in shared memory in group order.  (One group of D / 8 threads walking all 64 rows of an
+// item took 18 us for 1024 tokens of width 256, whose gradient is 0.5 MB.)
+constexpr int EMB_THREADS = 256;
+__global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_sorted_k(const long long* __restrict__ perm, const int* __restrict__ item_id,
                                                               const int* __restrict__ item_start, const int* __restrict__ seg_start,
                                                               const int* __restrict__ seg_count, const __nv_bfloat16* __restrict__ g,
                                                               float* __restrict__ dw, float* __restrict__ partial, int n_items_max,
                                                               int D, int R, int vocab) {
+  __shared__ __align__(16) float red[EMB_THREADS][8];
   const int item = blockIdx.x;
   const int id = item_id[item];
   if (id < 0 || id >= vocab) return;                 // padding items beyond the real count
@@ -332,14 +368,44 @@ __global__ void __launch_bounds__(128) embedding_bwd_sorted_k(const long long* _
   const int r0 = sub * R, r1 = min(cnt, r0 + R);
   if (r0 >= r1) return;
   const long long base = seg_start[id];
-  for (int c = threadIdx.x; c < (D >> 3); c += blockDim.x) {
+  const int ncol = D >> 3;
+  const int cols = min(ncol, EMB_THREADS), groups = EMB_THREADS / cols;
+  const int grp = threadIdx.x / cols, lc = threadIdx.x - grp * cols;
+  for (int c0 = 0; c0 < ncol; c0 += cols) {
+    const int c = c0 + lc;
+    const bool live = grp < groups && c < ncol;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int j = r0; j < r1; ++j) {
-      float f[8];
-      ld8(g + perm[base + j] * D + c * 8, f);
+    if (live) {
+      int j = r0 + grp;
+      for (; j + 3 * groups < r1; j += 4 * groups) {
+        uint4 u[4];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] += f[k];
+        for (int k = 0; k < 4; ++k) u[k] = *reinterpret_cast<const uint4*>(g + perm[base + j + k * groups] * D + c * 8);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          float f[8];
+          unpack8(u[k], f);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[e] += f[e];
+        }
+      }
+      for (; j < r1; j += groups) {
+        float f[8];
+        ld8(g + perm[base + j] * D + c * 8, f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += f[e];
+      }
     }
+    if (groups > 1) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) red[threadIdx.x][e] = acc[e];
+      __syncthreads();
+      if (grp == 0)
+        for (int q = 1; q < groups; ++q)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[e] += red[q * cols + lc][e];
+    }
+    if (!live || grp != 0) continue;                 // with several groups there is a single pass over the columns
     float* dst = (cnt <= R) ? dw + (long long)id * D + c * 8 : partial + (long long)item * D + c * 8;
     float4 a = make_float4(acc[0], acc[1], acc[2], acc[3]), b = make_float4(acc[4], acc[5], acc[6], acc[7]);
     if (cnt <= R) {
@@ -358,11 +424,105 @@ __global__ void __launch_bounds__(128) embedding_bwd_combine_k(const int* __rest
   const int n_it = (cnt + R - 1) / R, i0 = item_start[id];
   for (int c = threadIdx.x; c < (D >> 2); c += blockDim.x) {
     float4 acc = *reinterpret_cast<float4*>(dw + (long long)id * D + c * 4);
+    const float* src = partial + (long long)i0 * D + c * 4;
+#pragma unroll 8
     for (int i = 0; i < n_it; ++i) {
-      const float4 p = *reinterpret_cast<const float4*>(partial + (long long)(i0 + i) * D + c * 4);
+      const float4 p = *reinterpret_cast<const float4*>(src + (long long)i * D);
       acc.x += p.x; acc.y += p.y; acc.z += p.z; acc.w += p.w;
     }
     *reinterpret_cast<float4*>(dw + (long long)id * D + c * 4) = acc;
+  }
+}
+
+// The plan of the sorted embedding gradient for one batch of ids: a stable counting sort and the work-item tables, in four
+// kernels (twenty library launches took longer on the host than a small model's whole backward pass on the GPU).  Chunks of
+// PLAN_CHUNK tokens: histogram per chunk -> per id the exclusive sum over chunks -> one CTA scans the ids -> every chunk
+// places its tokens.  Ids outside [0, vocab) count as the nearest valid one.  No atomics decide an order.
+constexpr int PLAN_CHUNK = 1024;
+constexpr int PLAN_MAX_VOCAB = 49152;                // one counter per id in shared memory
+__device__ __forceinline__ int plan_id(const int* ids, long long i, int vocab) { return min(max(ids[i], 0), vocab - 1); }
+
+__global__ void __launch_bounds__(256) emb_plan_hist_k(const int* __restrict__ ids, long long N, int vocab, int* __restrict__ hist) {
+  extern __shared__ int plan_cnt[];
+  for (int v = threadIdx.x; v < vocab; v += 256) plan_cnt[v] = 0;
+  __syncthreads();
+  const long long t0 = (long long)blockIdx.x * PLAN_CHUNK, t1 = min(N, t0 + PLAN_CHUNK);
+  for (long long t = t0 + threadIdx.x; t < t1; t += 256) atomicAdd(&plan_cnt[plan_id(ids, t, vocab)], 1);   // integers: any order
+  __syncthreads();
+  for (int v = threadIdx.x; v < vocab; v += 256) hist[(long long)blockIdx.x * vocab + v] = plan_cnt[v];
+}
+__global__ void __launch_bounds__(64) emb_plan_chunks_k(int* __restrict__ hist, int n_chunks, int vocab, int* __restrict__ counts) {
+  const int v = blockIdx.x * 64 + threadIdx.x;
+  if (v >= vocab) return;
+  int sum = 0;
+  int* h = hist + v;
+  int c = 0;
+  for (; c + 8 <= n_chunks; c += 8) {
+    int x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = h[(long long)(c + k) * vocab];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { h[(long long)(c + k) * vocab] = sum; sum += x[k]; }
+  }
+  for (; c < n_chunks; ++c) { const int x = h[(long long)c * vocab]; h[(long long)c * vocab] = sum; sum += x; }
+  counts[v] = sum;
+}
+__global__ void __launch_bounds__(1024) emb_plan_scan_k(const int* __restrict__ counts, int vocab, int R, int n_items_max,
+                                                        int* __restrict__ seg_start, int* __restrict__ item_start,
+                                                        int* __restrict__ item_id) {
+  __shared__ int wsum[2][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int row0 = 0, it0 = 0;                             // rows and items of the ids below this round's
+  for (int v0 = 0; v0 < vocab; v0 += 1024) {
+    const int v = v0 + tid;
+    const int n = v < vocab ? counts[v] : 0, it = (n + R - 1) / R;
+    int a = n, b = it;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
+      if (lane >= o) { a += x; b += y; }
+    }
+    if (lane == 31) { wsum[0][warp] = a; wsum[1][warp] = b; }
+    __syncthreads();
+    int pa = 0, pb = 0, ta = 0, tb = 0;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) { pa += wsum[0][w]; pb += wsum[1][w]; }
+      ta += wsum[0][w]; tb += wsum[1][w];
+    }
+    const int item = it0 + pb + b - it;
+    if (v < vocab) { seg_start[v] = row0 + pa + a - n; item_start[v] = item; }
+    // a lane whose id has many items (a frequent token) fills them together with its warp
+    for (unsigned m = __ballot_sync(0xffffffffu, it > 0); m; m &= m - 1) {
+      const int src = __ffs(int(m)) - 1;
+      const int n_src = __shfl_sync(0xffffffffu, it, src), i_src = __shfl_sync(0xffffffffu, item, src);
+      for (int i = lane; i < n_src; i += 32) item_id[i_src + i] = v0 + warp * 32 + src;
+    }
+    row0 += ta; it0 += tb;
+    __syncthreads();
+  }
+  for (int i = it0 + tid; i < n_items_max; i += 1024) item_id[i] = -1;
+}
+__global__ void __launch_bounds__(256) emb_plan_place_k(const int* __restrict__ ids, long long N, int vocab, const int* __restrict__ hist,
+                                                        const int* __restrict__ seg_start, long long* __restrict__ perm) {
+  extern __shared__ int plan_cnt[];                  // next sorted position of every id
+  for (int v = threadIdx.x; v < vocab; v += 256) plan_cnt[v] = seg_start[v] + hist[(long long)blockIdx.x * vocab + v];
+  __syncthreads();
+  if (threadIdx.x >= 32) return;                     // one warp, 32 tokens at a time: the order of the tokens is kept
+  const int lane = threadIdx.x;
+  const long long t0 = (long long)blockIdx.x * PLAN_CHUNK, t1 = min(N, t0 + PLAN_CHUNK);
+  for (long long b = t0; b < t1; b += 32) {
+    const long long t = b + lane;
+    const int id = t < t1 ? plan_id(ids, t, vocab) : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, id);
+    const int before = __popc(same & ((1u << lane) - 1u));
+    const int at = id >= 0 ? plan_cnt[id] : 0;
+    __syncwarp();
+    if (id >= 0) {
+      if (before == 0) plan_cnt[id] = at + __popc(same);
+      perm[at + before] = t;
+    }
+    __syncwarp();
   }
 }
 
@@ -510,26 +670,49 @@ __global__ void __launch_bounds__(256) qkv_post_bwd_k(__nv_bfloat16* __restrict_
 }
 
 // d_gate_w[h, j] += sum_t dgl[t, h] * xn[t, j] ; d_xn_gate[t, j] = sum_h dgl[t, h] * Wg[h, j]
-// One CTA handles a slab of tokens; thread (h, j) accumulates its column.
+// A CTA handles a slab of tokens, VE_CHUNK (or fewer, as shared memory allows) at a time: both factors are staged in shared
+// memory by all threads, then thread (h, j) walks down its column there.  (With the walk over global memory, 512 dependent
+// steps of two loads on N / 512 CTAs, the kernel took 85 us for 2048 tokens and 119 us for 32768.)
+constexpr int VE_CHUNK = 64;
 __global__ void __launch_bounds__(256) ve_gate_bwd_k(const float* __restrict__ dgl, const __nv_bfloat16* __restrict__ xn,
                                                      const __nv_bfloat16* __restrict__ gate_w, float* __restrict__ d_gate_w,
                                                      __nv_bfloat16* __restrict__ d_xn_gate, long long N, int H, int D_model,
-                                                     int ch, int tok_per_cta) {
+                                                     int ch, int tok_per_cta, int chunk) {
+  extern __shared__ float ve_sm[];
+  float* xs = ve_sm;                  // [chunk][ch]
+  float* ds = ve_sm + chunk * ch;     // [chunk][H]
   const long long t0 = (long long)blockIdx.x * tok_per_cta;
   const long long t1 = min(N, t0 + tok_per_cta);
   const int tid = threadIdx.x;
-  for (int p = tid; p < H * ch; p += blockDim.x) {
-    const int h = p / ch, j = p - h * ch;
-    float acc = 0.f;
-    for (long long t = t0; t < t1; ++t) acc += dgl[t * H + h] * __bfloat162float(xn[t * D_model + j]);
-    atomicAdd(d_gate_w + h * ch + j, acc);
-  }
-  for (long long i = t0 * ch + tid; i < t1 * ch; i += blockDim.x) {
-    const long long t = i / ch;
-    const int j = int(i - t * ch);
-    float acc = 0.f;
-    for (int h = 0; h < H; ++h) acc += dgl[t * H + h] * __bfloat162float(gate_w[h * ch + j]);
-    d_xn_gate[i] = __float2bfloat16(acc);
+  for (int p0 = 0; p0 < H * ch; p0 += 256 * 4) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (long long c0 = t0; c0 < t1; c0 += chunk) {
+      const int n = int(min((long long)chunk, t1 - c0));
+      __syncthreads();
+      for (int i = tid; i < n * ch; i += 256) { const int t = i / ch; xs[i] = __bfloat162float(xn[(c0 + t) * D_model + i - t * ch]); }
+      for (int i = tid; i < n * H; i += 256) ds[i] = dgl[c0 * H + i];
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int p = p0 + u * 256 + tid;
+        if (p >= H * ch) break;
+        const int h = p / ch, j = p - h * ch;
+        float a = 0.f;
+#pragma unroll 8
+        for (int t = 0; t < n; ++t) a += ds[t * H + h] * xs[t * ch + j];
+        acc[u] += a;
+      }
+      if (p0 == 0)
+        for (int i = tid; i < n * ch; i += 256) {
+          const int t = i / ch, j = i - t * ch;
+          float a = 0.f;
+          for (int h = 0; h < H; ++h) a += ds[t * H + h] * __bfloat162float(gate_w[h * ch + j]);
+          d_xn_gate[c0 * ch + i] = __float2bfloat16(a);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (p0 + u * 256 + tid < H * ch) atomicAdd(d_gate_w + p0 + u * 256 + tid, acc[u]);
   }
 }
 
@@ -642,9 +825,15 @@ int arb_qkv_post_bwd(void* d_qkv, const void* qkv, const void* cos_t, const void
                                                       dgl, N, T, H);
   int rc = int(cudaGetLastError());
   if (ve_w) {
-    const int tpc = 512;
-    ve_gate_bwd_k<<<int((N + tpc - 1) / tpc), 256, 0, s>>>(dgl, (const bf16*)xn, (const bf16*)gate_w, d_gate_w, (bf16*)d_xn_gate, N, H,
-                                                            D_model, gate_ch, tpc);
+    // two slabs per SM, at least 16 tokens each (a slab ends with H * gate_ch atomic adds)
+    long long tpc = (N + 295) / 296;
+    if (tpc < 16) tpc = 16;
+    int chunk = int((48 * 1024) / (4ll * (gate_ch + H)));
+    if (chunk > VE_CHUNK) chunk = VE_CHUNK;
+    if (chunk < 1) return -3;
+    if (chunk > tpc) chunk = int(tpc);
+    ve_gate_bwd_k<<<unsigned((N + tpc - 1) / tpc), 256, size_t(chunk) * 4 * (gate_ch + H), s>>>(
+        dgl, (const bf16*)xn, (const bf16*)gate_w, d_gate_w, (bf16*)d_xn_gate, N, H, D_model, gate_ch, int(tpc), chunk);
     if (!rc) rc = int(cudaGetLastError());
   }
   return rc;
@@ -667,11 +856,28 @@ int arb_embedding_bwd_sorted(const long long* perm, const int* item_id, const in
                              const int* seg_count, const void* g, float* dw, float* partial, int n_items_max, int D, int R,
                              int vocab, cudaStream_t s) {
   if (n_items_max <= 0 || (D & 7) || R <= 0 || vocab <= 0 || misaligned(g) || misaligned(dw) || misaligned(partial)) return -3;
-  embedding_bwd_sorted_k<<<n_items_max, 128, 0, s>>>(perm, item_id, item_start, seg_start, seg_count, (const bf16*)g, dw, partial,
+  embedding_bwd_sorted_k<<<n_items_max, EMB_THREADS, 0, s>>>(perm, item_id, item_start, seg_start, seg_count, (const bf16*)g, dw, partial,
                                                      n_items_max, D, R, vocab);
   int rc = int(cudaGetLastError());
   if (rc) return rc;
   embedding_bwd_combine_k<<<vocab, 128, 0, s>>>(item_start, seg_count, partial, dw, D, R);
+  return int(cudaGetLastError());
+}
+int arb_embedding_plan(const int* ids, long long N, int vocab, int R, int n_items_max, int* hist, long long* perm, int* counts,
+                       int* seg_start, int* item_start, int* item_id, cudaStream_t s) {
+  if (N <= 0 || N > 0x7fffffffll || vocab <= 0 || vocab > PLAN_MAX_VOCAB || R <= 0 || n_items_max < N / R + vocab) return -3;
+  const unsigned chunks = unsigned((N + PLAN_CHUNK - 1) / PLAN_CHUNK);
+  const size_t smem = size_t(vocab) * 4;
+  static PerDeviceOnce cfg;
+  if (cfg.first()) {
+    cudaError_t e = cudaFuncSetAttribute(emb_plan_hist_k, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_MAX_VOCAB * 4);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(emb_plan_place_k, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_MAX_VOCAB * 4);
+    if (e != cudaSuccess) return int(e);
+  }
+  emb_plan_hist_k<<<chunks, 256, smem, s>>>(ids, N, vocab, hist);
+  emb_plan_chunks_k<<<(vocab + 63) / 64, 64, 0, s>>>(hist, int(chunks), vocab, counts);
+  emb_plan_scan_k<<<1, 1024, 0, s>>>(counts, vocab, R, n_items_max, seg_start, item_start, item_id);
+  emb_plan_place_k<<<chunks, 256, smem, s>>>(ids, N, vocab, hist, seg_start, perm);
   return int(cudaGetLastError());
 }
 int arb_add_cols(void* dst, long long ld_dst, const void* src, long long rows, int cols, cudaStream_t s) {

@@ -82,6 +82,7 @@ def _signatures() -> dict:
         "arb_embedding_fwd": [vp, vp, vp, i64, i32, i32, vp],
         "arb_embedding_bwd": [vp, vp, vp, i64, i32, i32, vp],
         "arb_embedding_bwd_sorted": [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp],
+        "arb_embedding_plan": [vp, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp],
         "arb_add_cols": [vp, i64, vp, i64, i32, vp],
         "arb_cast_f32_to_bf16": [vp, vp, i64, f32, vp],
         "arb_accum_bf16_into_f32": [vp, vp, i64, vp],
@@ -393,15 +394,33 @@ EMB_BWD_ROWS_PER_ITEM = 64
 _emb_plan = {}
 
 
+EMB_PLAN_MAX_VOCAB = 49152     # one shared-memory counter per id (csrc/elementwise.cu)
+
+
 def _embedding_plan(ids, vocab: int):
-    """Sort order and work-item tables of one batch of token ids; cached, since the word-embedding and every
-    value-embedding gradient of a micro-batch use the same ids.  Fixed-size tensors only (no host sync)."""
-    key = (ids.data_ptr(), ids._version, ids.numel(), vocab)
-    hit = _emb_plan.get(("plan", ids.device.index))
+    """Sort order and work-item tables of one batch of token ids; kept until other ids come, since the word-embedding and
+    every value-embedding gradient of a micro-batch use the same ids.  The entry holds the id tensor itself, so that its
+    address cannot be handed to another one meanwhile, and serves the stream it was made on.  Fixed-size tensors only (no host sync)."""
+    slot = ("plan", ids.device.index)
+    key = (ids.data_ptr(), ids._version, ids.numel(), ids.dtype, vocab, _stream())
+    hit = _emb_plan.get(slot)
     if hit is not None and hit[0] == key:
         return hit[1]
     R = EMB_BWD_ROWS_PER_ITEM
     N = ids.numel()
+    n_max = N // R + vocab + 1                                                     # upper bound of the item count
+    if vocab <= EMB_PLAN_MAX_VOCAB and ids.dtype is torch.int32 and ids.is_contiguous():
+        n_chunks = (N + 1023) // 1024
+        perm = torch.empty(N, dtype=torch.int64, device=ids.device)
+        counts, seg_start, item_start, item_id, hist = torch.empty(
+            3 * vocab + n_max + n_chunks * vocab, dtype=torch.int32, device=ids.device).split(
+            (vocab, vocab, vocab, n_max, n_chunks * vocab))
+        _check(lib().arb_embedding_plan(ids.data_ptr(), N, vocab, R, n_max, hist.data_ptr(), perm.data_ptr(), counts.data_ptr(),
+                                        seg_start.data_ptr(), item_start.data_ptr(), item_id.data_ptr(), _stream()),
+               "embedding_plan")
+        plan = (perm, item_id, item_start, seg_start, counts, n_max)
+        _emb_plan[slot] = (key, plan, ids)
+        return plan
     flat = ids.reshape(-1).long().clamp(0, vocab - 1)
     perm = torch.sort(flat, stable=True).indices.contiguous()                     # int64 [N]
     # (torch.bincount reads the largest id back to the host to size its result: a sync per micro-batch)
@@ -410,12 +429,11 @@ def _embedding_plan(ids, vocab: int):
     n_it = (counts + R - 1) // R
     it_end = torch.cumsum(n_it, 0)
     item_start = (it_end - n_it).to(torch.int32)
-    n_max = N // R + vocab + 1                                                     # upper bound of the item count
     item = torch.arange(n_max, device=ids.device)
     item_id = torch.searchsorted(it_end, item, right=True)
     item_id = torch.where(item < it_end[-1], item_id, torch.full_like(item_id, -1)).to(torch.int32)
     plan = (perm, item_id.contiguous(), item_start.contiguous(), seg_start.contiguous(), counts.to(torch.int32).contiguous(), n_max)
-    _emb_plan[("plan", ids.device.index)] = (key, plan)
+    _emb_plan[slot] = (key, plan, ids)
     return plan
 
 
@@ -427,10 +445,7 @@ def embedding_bwd(ids, g, dw_f32):
                "embedding_bwd")
         return
     perm, item_id, item_start, seg_start, counts, n_max = _embedding_plan(ids, vocab)
-    scratch = _emb_plan.get(("scratch", g.device.index))
-    if scratch is None or scratch.numel() < n_max * D:
-        scratch = torch.empty(n_max * D, dtype=torch.float32, device=g.device)
-        _emb_plan[("scratch", g.device.index)] = scratch
+    scratch = torch.empty(n_max * D, dtype=torch.float32, device=g.device)
     _check(lib().arb_embedding_bwd_sorted(perm.data_ptr(), item_id.data_ptr(), item_start.data_ptr(), seg_start.data_ptr(),
                                           counts.data_ptr(), g.data_ptr(), dw_f32.data_ptr(), scratch.data_ptr(), n_max, D,
                                           EMB_BWD_ROWS_PER_ITEM, vocab, _stream()), "embedding_bwd_sorted")

@@ -230,6 +230,54 @@ def test_embedding_backward_sorted_is_exact_and_deterministic():
     assert (dw2 - outs[0]).abs().max().item() < 2e-3
 
 
+@pytest.mark.parametrize("N,vocab,power", [(1, 8, 1), (31, 1, 1), (1024, 1000, 2), (1025, 5000, 1), (20000, 1000, 6), (3000, 40000, 3)])
+def test_embedding_plan_kernels_give_the_tables_of_a_stable_sort(N, vocab, power):
+    """Whole numbers, so equal: sorted order, counts, segment starts and work items against the library operations (one token,
+    one id, chunk edges, ids with many work items, more ids than tokens, ids outside the vocabulary)."""
+    from autoresearch_b200.ops import kernels as K
+    torch.manual_seed(N)
+    ids = (torch.rand(N, device="cuda") ** power * vocab).int()
+    ids[0] = vocab + 3
+    ids[-1] = -2
+    plans = []
+    for limit in (K.EMB_PLAN_MAX_VOCAB, 0):
+        keep, K.EMB_PLAN_MAX_VOCAB = K.EMB_PLAN_MAX_VOCAB, limit
+        try:
+            K._emb_plan.clear()
+            plans.append(K._embedding_plan(ids, vocab))
+        finally:
+            K.EMB_PLAN_MAX_VOCAB = keep
+    K._emb_plan.clear()
+    for a, b in zip(*plans):
+        assert a == b if isinstance(a, int) else torch.equal(a, b)
+
+
+@pytest.mark.parametrize("N,H,ch", [(1, 1, 32), (17, 3, 32), (700, 8, 32), (5000, 16, 64), (300, 2, 1024)])
+def test_value_gate_gradient(N, H, ch):
+    """Gate gradients against 64-bit sums over slabs of one token, slabs that end inside a chunk, more pairs than threads, and
+    rows too wide for a full chunk; fp32 sums of N products: 1e-5 of the sum of magnitudes."""
+    from autoresearch_b200.ops import kernels as K
+    torch.manual_seed(N)
+    D = max(H * 128, ch)
+    qkv, dqkv = _bf(N, 3 * H * 128), _bf(N, 3 * H * 128)
+    cos, sin = _bf(N, 64), _bf(N, 64)
+    rstd = torch.rand(N, 2 * H, device="cuda") + 0.5
+    xn, ve, gw = _bf(N, D), _bf(50, H * 128), _bf(H, ch)
+    ids = torch.randint(0, 50, (N,), device="cuda", dtype=torch.int32)
+    gate = torch.randn(N, H, device="cuda")
+    d_ve, dxg = torch.empty(N, H * 128, device="cuda", dtype=torch.bfloat16), torch.empty(N, ch, device="cuda", dtype=torch.bfloat16)
+    dgl, dgw = torch.empty(N, H, device="cuda"), torch.zeros(H, ch, device="cuda")
+    dv = dqkv[:, 2 * H * 128:].double().view(N, H, 128)
+    K._check(K.lib().arb_qkv_post_bwd(dqkv.data_ptr(), qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), rstd.data_ptr(), xn.data_ptr(),
+                                      ids.data_ptr(), ve.data_ptr(), gw.data_ptr(), gate.data_ptr(), d_ve.data_ptr(), dgw.data_ptr(),
+                                      dxg.data_ptr(), dgl.data_ptr(), N, N, H, D, ch, K._stream()), "qkv_post_bwd")
+    sg = torch.sigmoid(gate.double())
+    want = 2 * sg * (1 - sg) * (dv * ve[ids.long()].double().view(N, H, 128)).sum(-1)
+    _close(dgl, want.float(), 1e-4, "gate logits")
+    assert (dgw.double() - dgl.double().t() @ xn[:, :ch].double()).abs().max() <= 1e-5 * (dgl.double().abs().t() @ xn[:, :ch].double().abs()).max()
+    _close(dxg, (dgl.double() @ gw.double()).float(), 1e-2, "d_xn_gate")
+
+
 def test_bounded_device_wait_expires_into_the_error_word_and_the_context_stays_usable():
     """A peer barrier whose partner never arrives (a flag that nothing sets): the kernel gives up after its wait
     limit, returns normally and leaves ERR_COMM_TIMEOUT in the status word; the next kernels run as usual."""
