@@ -179,6 +179,10 @@ int arb_adamw_rs(float* master, const void* const* peer_buckets, int world, int 
                  long long bucket_offset, float grad_scale, float* m, float* v, void* shadow_bf16, long long n,
                  float lr, float beta1, float beta2, float eps, float wd, float bc1, float bc2, cudaStream_t s);
 // x = u / (sqrt(sum of partials[mat][0..63])*1.02 + 1e-6)
+// The whole step of n_mat small matrices (short side <= 64, at most 16384 elements): momentum, normalisation, `steps`
+// Newton-Schulz iterations with coefficients abc[3 * steps] (host), NorMuon, cautious update of master and bf16 parameter.
+int arb_muon_small(float* buf, const float* grad, float* second, float* master, void* shadow_bf16, int n_mat, int m, int n, float mu,
+                   float lr, float wd, float beta2, const float* abc, int steps, cudaStream_t s);
 int arb_muon_frob_scale(void* u_bf16, const float* partials, long long per_mat, int n_mat, cudaStream_t s);
 // NorMuon statistics + cautious update, per matrix [m, n]; reduce over columns if m >= n.
 int arb_normuon_stats(const void* x_bf16, float* v_mean, int n_mat, int m, int n, cudaStream_t s);

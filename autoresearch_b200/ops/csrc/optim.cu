@@ -10,9 +10,9 @@
 namespace arb {
 
 __global__ void adamw_k(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                        __nv_bfloat16* __restrict__ shadow, long long n, float lr, float b1, float b2, float eps, float wd,
-                        float bc1, float bc2) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+                        __nv_bfloat16* __restrict__ shadow, long long i0, long long n, float lr, float b1, float b2, float eps,
+                        float wd, float bc1, float bc2) {
+  for (long long i = i0 + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float pi = p[i], gi = g[i], mi = m[i], vi = v[i];
     pi -= lr * wd * pi;
     mi = b1 * mi + (1.f - b1) * gi;
@@ -120,20 +120,56 @@ __global__ void __launch_bounds__(256) muon_frob_scale_k(__nv_bfloat16* __restri
   }
 }
 
-// v_mean[mat, r] = mean_c x[mat, r, c]^2 (ROWS=true, one warp per row) or the column version
-// (ROWS=false: one thread per column, coalesced across threads).
-template <bool ROWS>
+// v_mean[mat, r] = mean_c x[mat, r, c]^2 (ROWS=true, one warp per row) or the column version.  Bounded by reading x once.
+// VEC (rows of a multiple of 8 elements, 16-byte aligned base): 16-byte loads; the column version gives a CTA 256 columns,
+// eight per lane, and every eighth row to a warp, four rows in flight; the warps' sums meet in shared memory in warp order.
+// (The first column version had one thread walk down a whole column with 2-byte loads, 512 or 1024 dependent steps on
+// 2 to 4 CTAs per matrix.)
+template <bool ROWS, bool VEC>
 __global__ void __launch_bounds__(256) normuon_stats_k(const __nv_bfloat16* __restrict__ x, float* __restrict__ v_mean, int m, int n) {
   const int mat = blockIdx.y;
   const __nv_bfloat16* xm = x + (long long)mat * m * n;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (ROWS) {
-    const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int r = blockIdx.x * 8 + warp;
     if (r >= m) return;
+    const __nv_bfloat16* xr = xm + (long long)r * n;
     float acc = 0.f;
-    for (int c = threadIdx.x & 31; c < n; c += 32) { const float f = __bfloat162float(xm[(long long)r * n + c]); acc += f * f; }
+    if (VEC) {
+#pragma unroll 2
+      for (int c = lane * 8; c < n; c += 256) {
+        const uint4 u = *reinterpret_cast<const uint4*>(xr + c);
+        const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), d = unpack_bf16(u.z), e = unpack_bf16(u.w);
+        acc += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + d.x * d.x + d.y * d.y + e.x * e.x + e.y * e.y;
+      }
+    } else {
+      for (int c = lane; c < n; c += 32) { const float f = __bfloat162float(xr[c]); acc += f * f; }
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) v_mean[(long long)mat * m + r] = acc / n;
+    if (lane == 0) v_mean[(long long)mat * m + r] = acc / n;
+  } else if (VEC) {
+    __shared__ float part[8][256];
+    const int c0 = blockIdx.x * 256 + lane * 8;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (c0 < n) {
+#pragma unroll 4
+      for (int r = warp; r < m; r += 8) {
+        const uint4 u = *reinterpret_cast<const uint4*>(xm + (long long)r * n + c0);
+        const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), d = unpack_bf16(u.z), e = unpack_bf16(u.w);
+        acc[0] += a.x * a.x; acc[1] += a.y * a.y; acc[2] += b.x * b.x; acc[3] += b.y * b.y;
+        acc[4] += d.x * d.x; acc[5] += d.y * d.y; acc[6] += e.x * e.x; acc[7] += e.y * e.y;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) part[warp][lane * 8 + j] = acc[j];
+    __syncthreads();
+    const int c = blockIdx.x * 256 + threadIdx.x;
+    if (c >= n) return;
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += part[w][threadIdx.x];
+    v_mean[(long long)mat * n + c] = t / m;
   } else {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n) return;
@@ -220,6 +256,102 @@ __global__ void muon_update_k(float* __restrict__ master, __nv_bfloat16* __restr
       master[mat * per + i] = p;
       shadow[mat * per + i] = __float2bfloat16(p);
     }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The whole Muon step of a small matrix (value-embedding gates: heads x 32) in one CTA, one launch for the group: too small
+// for the GEMM tiles, and as library operations about a hundred launches of 2 us each.  Works on Y = the matrix with its
+// short side as rows (K x L): A = Y Y^T, C = a I + b A + c A^2, Y = C Y.  Every product is summed in fp32 and rounded to
+// bf16, as the tensor operations it stands for store it; the momentum, the statistics and the update are fp32.
+constexpr int SMALL_K = 64, SMALL_ELEMS = 16384, SMALL_STEPS = 8;
+struct NsCoeffs { float abc[SMALL_STEPS][3]; int steps; };
+__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16(x)); }
+__device__ __forceinline__ float cta_sum(float v, float* red) {       // 256 threads; the same sum in every thread
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float t = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) t += red[w];
+  return t;
+}
+__global__ void __launch_bounds__(256) muon_small_k(float* __restrict__ buf, const float* __restrict__ g, float* __restrict__ second,
+                                                    float* __restrict__ master, __nv_bfloat16* __restrict__ shadow, int m, int n,
+                                                    float mu, float lr, float wd, float beta2, const NsCoeffs ns) {
+  extern __shared__ float small_sm[];
+  __shared__ float red[8];
+  const int K = min(m, n), L = max(m, n), ld = L + 1, tid = threadIdx.x;
+  const bool tall = m > n;
+  float* Y = small_sm;                   // [K][ld]
+  float* Y2 = Y + K * ld;
+  float* A = Y2 + K * ld;                // [K][K + 1]
+  float* Cm = A + K * (K + 1);
+  float* stat = Cm + K * (K + 1);        // [max(m, n)]
+  const long long base = (long long)blockIdx.x * m * n;
+  auto at = [&](int i) { const int r = i / n, c = i - r * n; return tall ? c * ld + r : r * ld + c; };
+  float ss = 0.f;
+  for (int i = tid; i < m * n; i += 256) {
+    const float gi = g[base + i], b = mu * buf[base + i] + (1.f - mu) * gi;
+    buf[base + i] = b;
+    const float u = round_bf16((1.f - mu) * gi + mu * b);
+    Y[at(i)] = u;
+    ss += u * u;
+  }
+  const float inv = 1.f / (sqrtf(cta_sum(ss, red)) * 1.02f + 1e-6f);
+  for (int i = tid; i < K * ld; i += 256) if (i % ld < L) Y[i] = round_bf16(Y[i] * inv);
+  __syncthreads();
+  for (int st = 0; st < ns.steps; ++st) {
+    const float ca = ns.abc[st][0], cb = ns.abc[st][1], cc = ns.abc[st][2];
+    for (int i = tid; i < K * K; i += 256) {
+      const int r = i / K, c = i - r * K;
+      float acc = 0.f;
+      for (int l = 0; l < L; ++l) acc += Y[r * ld + l] * Y[c * ld + l];
+      A[r * (K + 1) + c] = round_bf16(acc);
+    }
+    __syncthreads();
+    for (int i = tid; i < K * K; i += 256) {
+      const int r = i / K, c = i - r * K;
+      float acc = 0.f;
+      for (int l = 0; l < K; ++l) acc += A[r * (K + 1) + l] * A[l * (K + 1) + c];
+      Cm[r * (K + 1) + c] = round_bf16((r == c ? ca : 0.f) + cb * A[r * (K + 1) + c] + cc * round_bf16(acc));
+    }
+    __syncthreads();
+    for (int i = tid; i < K * L; i += 256) {
+      const int r = i / L, c = i - r * L;
+      float acc = 0.f;
+      for (int l = 0; l < K; ++l) acc += Cm[r * (K + 1) + l] * Y[l * ld + c];
+      Y2[r * ld + c] = round_bf16(acc);
+    }
+    __syncthreads();
+    float* t = Y; Y = Y2; Y2 = t;
+  }
+  // NorMuon: mean square of each row (m >= n) or column, i.e. over the short side unless the matrix is square
+  const int n_stat = L;
+  float vn = 0.f, vn2 = 0.f;
+  float* sm = second + (long long)blockIdx.x * n_stat;
+  for (int i = tid; i < n_stat; i += 256) {
+    float acc = 0.f;
+    for (int k = 0; k < K; ++k) { const float y = (m == n) ? Y[i * ld + k] : Y[k * ld + i]; acc += y * y; }
+    const float v = acc / K, s2 = beta2 * sm[i] + (1.f - beta2) * v;
+    sm[i] = s2;
+    const float sc = rsqrtf(fmaxf(s2, 1e-10f));
+    stat[i] = sc;
+    vn += v * K;
+    vn2 += v * K * sc * sc;
+  }
+  vn = cta_sum(vn, red);
+  vn2 = cta_sum(vn2, red);
+  const float ratio = sqrtf(vn) / fmaxf(sqrtf(vn2), 1e-10f);
+  for (int i = tid; i < m * n; i += 256) {
+    const int r = i / n, c = i - r * n;
+    const float x = Y[at(i)] * (stat[m >= n ? r : c] * ratio);
+    float p = master[base + i];
+    p -= lr * x + ((x * p >= 0.f) ? lr * wd * p : 0.f);
+    master[base + i] = p;
+    shadow[base + i] = __float2bfloat16(p);
   }
 }
 
@@ -339,6 +471,19 @@ __device__ __forceinline__ void adamw8(float* __restrict__ p, float* __restrict_
   }
 }
 
+// The local form: gradient in fp32, 30 bytes per element, nothing but HBM to wait for.  A thread takes eight consecutive
+// elements, so that eight 16-byte loads are in flight before the first is used.
+__global__ void __launch_bounds__(256) adamw8_k(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
+                                                float* __restrict__ v, __nv_bfloat16* __restrict__ shadow, long long n8, float lr,
+                                                float b1, float b2, float eps, float wd, float bc1, float bc2) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n8; c += stride) {
+    const float4 ga = *reinterpret_cast<const float4*>(g + c * 8), gb = *reinterpret_cast<const float4*>(g + c * 8 + 4);
+    const float gg[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
+    adamw8(p, m, v, shadow, c * 8, gg, lr, b1, b2, eps, wd, bc1, bc2);
+  }
+}
+
 __global__ void __launch_bounds__(256) adamw_rs_k(float* __restrict__ p, GradPeers gp, long long offset, float* __restrict__ m,
                                                   float* __restrict__ v, __nv_bfloat16* __restrict__ shadow, long long n, float lr,
                                                   float b1, float b2, float eps, float wd, float bc1, float bc2) {
@@ -368,6 +513,11 @@ static int fill_peers(GradPeers& gp, const void* const* peers, int world, int ra
   return 0;
 }
 
+static inline bool aligned16(const void* a, const void* b = nullptr, const void* c = nullptr, const void* d = nullptr) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
+           reinterpret_cast<uintptr_t>(d)) & 15) == 0;
+}
+
 static inline int blocks_for(long long n, int threads, int cap) {
   long long b = (n + threads - 1) / threads;
   return int(b < 1 ? 1 : (b > cap ? cap : b));
@@ -382,12 +532,13 @@ extern "C" {
 int arb_adamw(float* master, const float* grad, float* m, float* v, void* shadow_bf16, long long n, float lr, float beta1,
               float beta2, float eps, float wd, float bc1, float bc2, cudaStream_t s) {
   if (n <= 0) return -3;
-  adamw_k<<<blocks_for(n, 256, 148 * 8), 256, 0, s>>>(master, grad, m, v, (__nv_bfloat16*)shadow_bf16, n, lr, beta1, beta2, eps, wd, bc1, bc2);
+  auto* sh = (__nv_bfloat16*)shadow_bf16;
+  // eight elements per thread where all pointers allow it; a tail of at most seven (or everything) element by element
+  const long long n8 = aligned16(master, grad, m, v) && aligned16(shadow_bf16) ? n / 8 : 0;
+  if (n8) adamw8_k<<<blocks_for(n8, 256, 148 * 16), 256, 0, s>>>(master, grad, m, v, sh, n8, lr, beta1, beta2, eps, wd, bc1, bc2);
+  if (n8 * 8 < n)
+    adamw_k<<<blocks_for(n - n8 * 8, 256, 148 * 8), 256, 0, s>>>(master, grad, m, v, sh, n8 * 8, n, lr, beta1, beta2, eps, wd, bc1, bc2);
   return int(cudaGetLastError());
-}
-static inline bool aligned16(const void* a, const void* b = nullptr, const void* c = nullptr, const void* d = nullptr) {
-  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
-           reinterpret_cast<uintptr_t>(d)) & 15) == 0;
 }
 // `partials`: n_mat x 64 floats (per-block partial sums of u^2, consumed by arb_muon_frob_scale)
 int arb_muon_nesterov(float* buf, const float* grad, void* u_bf16, float* partials, long long per_mat, int n_mat, float mu, cudaStream_t s) {
@@ -422,6 +573,26 @@ int arb_adamw_rs(float* master, const void* const* peer_buckets, int world, int 
                                                               beta2, eps, wd, bc1, bc2);
   return int(cudaGetLastError());
 }
+// abc: 3 * steps host floats (the polynomial of every Newton-Schulz step)
+int arb_muon_small(float* buf, const float* grad, float* second, float* master, void* shadow_bf16, int n_mat, int m, int n, float mu,
+                   float lr, float wd, float beta2, const float* abc, int steps, cudaStream_t s) {
+  if (n_mat <= 0 || m <= 0 || n <= 0 || steps < 0 || steps > SMALL_STEPS) return -3;
+  const int K = m < n ? m : n, L = m < n ? n : m;
+  if (K > SMALL_K || (long long)K * L > SMALL_ELEMS) return -3;
+  NsCoeffs ns{};
+  ns.steps = steps;
+  for (int i = 0; i < steps; ++i) for (int j = 0; j < 3; ++j) ns.abc[i][j] = abc[3 * i + j];
+  static PerDeviceOnce cfg;
+  if (cfg.first()) {
+    // K x L <= 16384 twice with padded rows, two K x K, L statistics: at most 197 KB
+    cudaError_t e = cudaFuncSetAttribute(muon_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e != cudaSuccess) return int(e);
+  }
+  const size_t smem = sizeof(float) * (2 * size_t(K) * (L + 1) + 2 * size_t(K) * (K + 1) + size_t(L));
+  if (smem > 200 * 1024) return -3;
+  muon_small_k<<<n_mat, 256, smem, s>>>(buf, grad, second, master, (__nv_bfloat16*)shadow_bf16, m, n, mu, lr, wd, beta2, ns);
+  return int(cudaGetLastError());
+}
 int arb_muon_frob_scale(void* u_bf16, const float* partials, long long per_mat, int n_mat, cudaStream_t s) {
   if (per_mat <= 0 || n_mat <= 0 || n_mat > 65535) return -3;
   if ((per_mat & 7) == 0 && aligned16(u_bf16))
@@ -432,8 +603,13 @@ int arb_muon_frob_scale(void* u_bf16, const float* partials, long long per_mat, 
 }
 int arb_normuon_stats(const void* x_bf16, float* v_mean, int n_mat, int m, int n, cudaStream_t s) {
   if (n_mat <= 0 || m <= 0 || n <= 0 || n_mat > 65535) return -3;
-  if (m >= n) normuon_stats_k<true><<<dim3((m + 7) / 8, n_mat), 256, 0, s>>>((const __nv_bfloat16*)x_bf16, v_mean, m, n);
-  else normuon_stats_k<false><<<dim3((n + 255) / 256, n_mat), 256, 0, s>>>((const __nv_bfloat16*)x_bf16, v_mean, m, n);
+  const auto* x = (const __nv_bfloat16*)x_bf16;
+  const bool vec = (n & 7) == 0 && aligned16(x_bf16);
+  const dim3 rows((m + 7) / 8, n_mat), cols((n + 255) / 256, n_mat);
+  if (m >= n && vec) normuon_stats_k<true, true><<<rows, 256, 0, s>>>(x, v_mean, m, n);
+  else if (m >= n) normuon_stats_k<true, false><<<rows, 256, 0, s>>>(x, v_mean, m, n);
+  else if (vec) normuon_stats_k<false, true><<<cols, 256, 0, s>>>(x, v_mean, m, n);
+  else normuon_stats_k<false, false><<<cols, 256, 0, s>>>(x, v_mean, m, n);
   return int(cudaGetLastError());
 }
 int arb_normuon_scales(const float* v_mean, float* second, float* scale, int n_mat, int n_stat, int red_size, float beta2, cudaStream_t s) {

@@ -17,6 +17,7 @@ Granularity follows what fuses well on a B200 rather than the reference's op lis
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
 from typing import Optional
 
@@ -602,6 +603,13 @@ class OptimKernels:
         if min(m, n) < self.MIN_GEMM_DIM or pv.dtype != torch.bfloat16 or (m % 8) or (n % 8):
             if isinstance(grad, PeerGrad):
                 raise RuntimeError("small Muon groups take the unfused path: reduce them first")
+            if (pv.dtype == torch.bfloat16 and grad.dtype == torch.float32 and min(m, n) <= 64 and m * n <= 16384 and ns_steps <= 5 and
+                    all(t.is_contiguous() for t in (grad, pv, *st.values()))):
+                abc = (C.c_float * 15)(*[c for step in MA.POLAR_EXPRESS for c in step])
+                K._check(K.lib().arb_muon_small(st["momentum"].data_ptr(), grad.data_ptr(), st["second"].data_ptr(),
+                                                st["master"].data_ptr(), pv.data_ptr(), G, m, n, mu, lr, wd, beta2, abc,
+                                                max(0, ns_steps), K._stream()), "muon_small")
+                return
             u = MA.muon_nesterov(st["momentum"], grad.float(), mu, torch.bfloat16)
             x = MA.newton_schulz(MA.frob_normalise(u), ns_steps)
             gfin = MA.normuon(x, st["second"], beta2)

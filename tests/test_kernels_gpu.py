@@ -170,6 +170,29 @@ def test_adamw_and_muon_kernels_match_reference():
         _close(st["second"], rsec, 5e-2, "second moment")
 
 
+@pytest.mark.parametrize("G,m,n", [(4, 8, 32), (3, 32, 8), (1, 1, 40), (2, 60, 60), (2, 100, 64), (1, 16, 1024), (2, 3, 5)])
+def test_muon_step_of_small_matrices(G, m, n):
+    """One CTA per matrix against the tensor operations it replaces, which round to bf16 in the same places: what differs is
+    the order of the fp32 sums, i.e. single last places of bf16 values (2^-8), damped by the five steps."""
+    from autoresearch_b200.ops.sm100 import OptimKernels
+    from autoresearch_b200.optim import muon_adamw as MA
+    torch.manual_seed(G * m + n)
+    ok = OptimKernels()
+    master, sshape = torch.randn(G, m, n, device="cuda") * 0.05, (G, m, 1) if m >= n else (G, 1, n)
+    st = dict(master=master.clone(), momentum=torch.zeros_like(master), second=torch.zeros(sshape, device="cuda"))
+    pv = master.to(torch.bfloat16)
+    rmaster, rmom, rsec = master.clone(), torch.zeros_like(master), torch.zeros(sshape, device="cuda")
+    for _ in range(3):
+        grad = torch.randn(G, m, n, device="cuda") * 0.01
+        ok.muon_group(st, grad, pv, 0.9, 0.02, 0.1, 0.95, 5)
+        u = MA.muon_nesterov(rmom, grad, 0.9, torch.bfloat16)
+        MA.cautious_update(rmaster, MA.normuon(MA.newton_schulz(MA.frob_normalise(u), 5), rsec, 0.95), 0.02, 0.1)
+    assert (st["master"] - rmaster).norm() <= 1e-2 * (rmaster - master).norm()
+    _close(st["momentum"], rmom, 1e-6, "momentum")
+    _close(st["second"], rsec, 2e-2, "second moment")
+    assert torch.equal(pv, st["master"].to(torch.bfloat16))
+
+
 def test_muon_step_is_bitwise_reproducible_and_handles_ragged_shapes():
     """The Frobenius norm is summed in a fixed order (no atomics), so two runs of a Muon step from the same state
     give the same bits; a matrix whose column count is not a multiple of 8 takes the scalar kernels."""
