@@ -21,7 +21,34 @@ struct AttnArgs {
   // dkv
   void* dk; void* dv; long long lddk, lddv;
   int* err;
+  int group;                         // heads x sequences whose tiles are interleaved (attn_tile)
 };
+
+// Which tile of which head a CTA of the flat grid takes.  The (sequence, head) pairs go in groups of p.group; inside a group the
+// pair changes fastest and the tile rank (0 = most work) slowest, so the long tiles of a whole group start first and its last
+// wave is made of short ones.  One pair after the other instead leaves the last pair's long tiles for the end: full causal,
+// B=1 H=16 T=8192: 328 us, grouped 277; B=1 H=16 T=4096: 120, 82.  All pairs in one group lose their K and V between a tile and
+// the next once they outgrow L2: B=64 H=4 T=2048: 403 us, one after the other 361.
+struct AttnTile { int rank, h, b; };
+__device__ __forceinline__ AttnTile attn_tile(const AttnArgs& p, int n_tiles) {
+  const int per = p.group * n_tiles, g = int(blockIdx.x) / per, i = int(blockIdx.x) - g * per;
+  const int n = min(p.group, p.B * p.H - g * p.group);
+  const int bh = g * p.group + i % n, b = bh / p.H;
+  return {i / n, bh - b * p.H, b};
+}
+// K and V of a group within 48 MB (of 126 MB L2), at least eight pairs: that leaves 37 tiles of each in flight on 148 SMs.
+// Up to 148 tiles of 128 rows all start at once and keep the order of memory.
+inline int attn_group(int B, int H, int T) {
+  if ((long long)((T + 127) / 128) * H * B <= 148) return 1;
+  const long long fit = (48ll << 20) / (512ll * T), bh = (long long)B * H;
+  const long long g = fit < 8 ? 8 : fit;
+  return int(g < bh ? g : bh);
+}
+// grid of the flat form, or 0 where it would not fit
+inline unsigned attn_grid(int B, int H, int T, int rows) {
+  const long long n = (long long)((T + rows - 1) / rows) * H * B;
+  return n <= 0x7fffffffll ? unsigned(n) : 0u;
+}
 
 // Optional per-role cycle accounting (compile with -DARB_ATTN_PROF): each role of the CTA with
 // blockIdx == (0,0,0) sums clock64() deltas between PROF_TOC marks and stores eight counters at
@@ -114,6 +141,49 @@ __device__ __forceinline__ void exp64_store(const uint32_t (&s0)[32], const uint
   tmem_st32(tm_dst, pk);
 }
 
+// packed fp32 pairs in one 64-bit register
+__device__ __forceinline__ unsigned long long pk2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpk2(unsigned long long v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// row maximum of 32 scores, columns [col0, col0 + 32) of a tile whose visible columns are [mlo, mlo + span]
+template <bool MASK>
+__device__ __forceinline__ float max32(const uint32_t (&s)[32], int col0, int mlo, unsigned span, float m) {
+  float a = m, b = m;
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) {
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      v[u] = __uint_as_float(s[j + u]);
+      if constexpr (MASK) v[u] = (unsigned(col0 + j + u - mlo) <= span) ? v[u] : -INFINITY;
+    }
+    a = fmaxf(a, fmaxf(v[0], v[1]));      // three-input maximum: one instruction each
+    b = fmaxf(b, fmaxf(v[2], v[3]));
+  }
+  return fmaxf(a, b);
+}
+
 __device__ __forceinline__ void named_bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
@@ -145,8 +215,12 @@ int attn_fwd2_launch(const void* q, const void* k, const void* v, long long ldq,
                      cudaStream_t stream);
 
 
+// attn_fwd4_sm100.cu
+int attn_fwd4_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, cudaStream_t stream);
+
+
 // attn_fwd3_sm100.cu
-int attn_fwd3_launch(const void* q, const void* k, const void* v, long long ldq, long long ldk, long long ldv, AttnArgs a,
+int attn_fwd3_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, bool poly,
                      cudaStream_t stream);
 
 }  // namespace arb

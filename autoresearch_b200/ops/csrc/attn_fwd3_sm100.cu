@@ -26,31 +26,6 @@ constexpr int ATT_FWD3_THREADS = 384;   // softmax group 0 (warps 0-3), softmax 
 __device__ __forceinline__ void reg_alloc_224() { asm volatile("setmaxnreg.inc.sync.aligned.u32 224;"); }
 __device__ __forceinline__ void reg_dealloc_56() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;"); }
 
-// packed fp32 pairs in one 64-bit register
-__device__ __forceinline__ unsigned long long pk2(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpk2(unsigned long long v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // 2^x for a pair, x <= ~1, on the FMA pipe (see poly_exp2 in attn_common.cuh for the scalar form)
 __device__ __forceinline__ void poly_exp2_pair(unsigned long long x, float& e0, float& e1) {
   float x0, x1;
@@ -71,14 +46,14 @@ __device__ __forceinline__ void poly_exp2_pair(unsigned long long x, float& e0, 
 
 // Exponentials of 32 scores (one tcgen05.ld chunk) of a row: e = 2^(s*c - mc); bf16 pairs into pk[16]; row sum into
 // the packed accumulator.  Pairs 3, 7, 11, 15 of the chunk (one in four) take the polynomial.
-template <bool MASK>
+template <bool MASK, bool POLY>
 __device__ __forceinline__ void exp32(const uint32_t (&s)[32], uint32_t* pk, unsigned long long c2, unsigned long long nmc2,
                                       int col0, int mlo, unsigned span, unsigned long long& rs2) {
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
     const unsigned long long x = fma2(pk2(__uint_as_float(s[2 * j]), __uint_as_float(s[2 * j + 1])), c2, nmc2);
     float e0, e1;
-    if ((j & 3) == 3) {
+    if (POLY && (j & 3) == 3) {
       poly_exp2_pair(x, e0, e1);
     } else {
       float x0, x1;
@@ -95,23 +70,6 @@ __device__ __forceinline__ void exp32(const uint32_t (&s)[32], uint32_t* pk, uns
   }
 }
 
-template <bool MASK>
-__device__ __forceinline__ float max32(const uint32_t (&s)[32], int col0, int mlo, unsigned span, float m) {
-  float a = m, b = m;
-#pragma unroll
-  for (int j = 0; j < 32; j += 4) {
-    float v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      v[u] = __uint_as_float(s[j + u]);
-      if constexpr (MASK) v[u] = (unsigned(col0 + j + u - mlo) <= span) ? v[u] : -INFINITY;
-    }
-    a = fmaxf(a, fmaxf(v[0], v[1]));      // three-input maximum: one instruction each
-    b = fmaxf(b, fmaxf(v[2], v[3]));
-  }
-  return fmaxf(a, b);
-}
-
 struct Fwd3Smem {
   static constexpr int Q = 0;                       // 2 x 32 KB
   static constexpr int K0 = 65536;                  // 3 x 32 KB
@@ -121,6 +79,7 @@ struct Fwd3Smem {
 };
 static_assert(Fwd3Smem::TOTAL <= 232448, "exceeds the 227 KB shared memory of one CTA");
 
+template <bool POLY>
 __global__ void __launch_bounds__(ATT_FWD3_THREADS, 1)
 attn_fwd3_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
             const __grid_constant__ CUtensorMap tmV, const AttnArgs p) {
@@ -143,8 +102,8 @@ attn_fwd3_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_pair = (p.T + 255) / 256;
-  const int mp = n_pair - 1 - int(blockIdx.x);     // later queries see more keys: schedule them first
-  const int h = blockIdx.y, b = blockIdx.z;
+  const AttnTile tile = attn_tile(p, n_pair);
+  const int mp = n_pair - 1 - tile.rank, h = tile.h, b = tile.b;     // later queries see more keys
   const int m0 = mp * 256;
   // key-tile range of each query tile; tile 1 is empty when the sequence ends inside tile 0
   int lo_i[2], hi_i[2];
@@ -343,15 +302,15 @@ attn_fwd3_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
       unsigned long long rs2 = pk2(0.f, 0.f);
       uint32_t p0[32], p1[32];
       if (need_mask) {
-        exp32<true>(sa, p0, c2, nmc2, 0, mlo, span, rs2);
-        exp32<true>(sb, p0 + 16, c2, nmc2, 32, mlo, span, rs2);
-        exp32<true>(sc, p1, c2, nmc2, 64, mlo, span, rs2);
-        exp32<true>(sd, p1 + 16, c2, nmc2, 96, mlo, span, rs2);
+        exp32<true, POLY>(sa, p0, c2, nmc2, 0, mlo, span, rs2);
+        exp32<true, POLY>(sb, p0 + 16, c2, nmc2, 32, mlo, span, rs2);
+        exp32<true, POLY>(sc, p1, c2, nmc2, 64, mlo, span, rs2);
+        exp32<true, POLY>(sd, p1 + 16, c2, nmc2, 96, mlo, span, rs2);
       } else {
-        exp32<false>(sa, p0, c2, nmc2, 0, mlo, span, rs2);
-        exp32<false>(sb, p0 + 16, c2, nmc2, 32, mlo, span, rs2);
-        exp32<false>(sc, p1, c2, nmc2, 64, mlo, span, rs2);
-        exp32<false>(sd, p1 + 16, c2, nmc2, 96, mlo, span, rs2);
+        exp32<false, POLY>(sa, p0, c2, nmc2, 0, mlo, span, rs2);
+        exp32<false, POLY>(sb, p0 + 16, c2, nmc2, 32, mlo, span, rs2);
+        exp32<false, POLY>(sc, p1, c2, nmc2, 64, mlo, span, rs2);
+        exp32<false, POLY>(sd, p1 + 16, c2, nmc2, 96, mlo, span, rs2);
       }
       tmem_st32(TM_S + lane_addr, p0);
       tmem_st32(TM_S + lane_addr + 32u, p1);
@@ -398,17 +357,18 @@ attn_fwd3_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
   if (warp == 9) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-int attn_fwd3_launch(const void* q, const void* k, const void* v, long long ldq, long long ldk, long long ldv, AttnArgs a,
+// poly: one exponential in four on the FMA pipe (relative error 7.5e-5), else all on the ex2 unit
+int attn_fwd3_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, bool poly,
                      cudaStream_t stream) {
   static PerDeviceOnce cfg;
   int r;
-  if (cfg.first()) { if ((r = set_smem(attn_fwd3_k, Fwd3Smem::TOTAL))) return r; }
-  CUtensorMap tq, tk, tv;
-  if ((r = make_qkv_tmap(&tq, q, a.B, a.T, a.H, ldq, 128))) return 1000 + r;
-  if ((r = make_qkv_tmap(&tk, k, a.B, a.T, a.H, ldk, 128))) return 1000 + r;
-  if ((r = make_qkv_tmap(&tv, v, a.B, a.T, a.H, ldv, 128))) return 1000 + r;
-  dim3 grid((a.T + 255) / 256, a.H, a.B);
-  attn_fwd3_k<<<grid, ATT_FWD3_THREADS, Fwd3Smem::TOTAL, stream>>>(tq, tk, tv, a);
+  if (cfg.first()) {
+    if ((r = set_smem(attn_fwd3_k<true>, Fwd3Smem::TOTAL))) return r;
+    if ((r = set_smem(attn_fwd3_k<false>, Fwd3Smem::TOTAL))) return r;
+  }
+  const unsigned grid = attn_grid(a.B, a.H, a.T, 256);
+  if (!grid) return -3;
+  (poly ? attn_fwd3_k<true> : attn_fwd3_k<false>)<<<grid, ATT_FWD3_THREADS, Fwd3Smem::TOTAL, stream>>>(tq, tk, tv, a);
   return int(cudaGetLastError());
 }
 
@@ -421,8 +381,13 @@ extern "C" int arb_attn_prof_fwd3(const void* q, const void* k, const void* v, v
                                   long long ld, long long ldo, int window, float scale, int* err, long long* prof) {
   cudaMemcpyToSymbol(arb::arb_attn_prof_buffer, &prof, sizeof(prof));
   arb::AttnArgs a{};
-  a.B = B; a.T = T; a.H = H; a.window = window > T ? T : window; a.scale = scale;
+  a.B = B; a.T = T; a.H = H; a.window = window > T ? T : window; a.scale = scale; a.group = arb::attn_group(B, H, T);
   a.o = o; a.ldo = ldo; a.lse = lse; a.err = err;
-  return arb::attn_fwd3_launch(q, k, v, ld, ld, ld, a, 0);
+  CUtensorMap tq, tk, tv;
+  int r;
+  if ((r = arb::make_qkv_tmap(&tq, q, B, T, H, ld, 128)) || (r = arb::make_qkv_tmap(&tk, k, B, T, H, ld, 128)) ||
+      (r = arb::make_qkv_tmap(&tv, v, B, T, H, ld, 128)))
+    return 1000 + r;
+  return arb::attn_fwd3_launch(tq, tk, tv, a, true, 0);
 }
 #endif

@@ -815,12 +815,13 @@ __global__ void __launch_bounds__(256) attn_delta_k(const __nv_bfloat16* __restr
 
 using namespace arb;
 
+// 6: as 4 without the polynomial; 5: as 2 with two CTAs per SM in the forward (attn_fwd4_sm100.cu) for every shape;
 // 4: as 2 with the register-split forward (attn_fwd3_sm100.cu) for every shape; 3: as 2 with the two-query-tile forward
 // for every shape; 2 (default): wide backward, forward chosen by shape (see arb_attn_fwd); 1: 64-wide sub-tiles with TMEM
 // operands; 0: with shared-memory operands
 static int g_attn_mode = 2;
 static int g_attn_ts = 1;
-extern "C" void arb_attn_set_mode(int mode) { g_attn_mode = mode < 0 ? 0 : (mode > 4 ? 4 : mode); g_attn_ts = g_attn_mode ? 1 : 0; }
+extern "C" void arb_attn_set_mode(int mode) { g_attn_mode = mode < 0 ? 0 : (mode > 6 ? 6 : mode); g_attn_ts = g_attn_mode ? 1 : 0; }
 
 template <bool TS>
 static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, dim3 grid,
@@ -863,15 +864,23 @@ extern "C" int arb_attn_fwd(const void* q, const void* k, const void* v, void* o
   if ((r = make_qkv_tmap(&tv, v, B, T, H, ldv, 128))) return 1000 + r;
   AttnArgs a{};
   a.B = B; a.T = T; a.H = H; a.window = window > T ? T : window; a.scale = scale;
-  a.o = o; a.ldo = ldo; a.lse = lse; a.err = err_flag;
-  // Two query tiles per CTA pay on grids of several waves (B=4, H=8, T=32768, ms one tile / two tiles: full causal
-  // 9.79 / 9.42, window 4096 2.61 / 2.50, window 256 0.51 / 0.47) and lose on small grids, where halving the CTA count
-  // costs more than the shared K / V loads save, and on short sequences.  Of the two-tile kernels the register-split
-  // one (attn_fwd3) is the default: 4-5 % faster than attn_fwd2 on the same shapes (full causal 8.95 -> 8.54 ms,
-  // window 4096 2.13 -> 2.04, window 256 0.471 -> 0.458; B=8, H=16, T=8192 full 2.38 -> 2.27).
-  const long long pair_ctas = (long long)((T + 255) / 256) * H * B;
-  if (g_attn_mode == 4 || (g_attn_mode == 2 && pair_ctas >= 2048 && T >= 4096))
-    return attn_fwd3_launch(q, k, v, ldq, ldk, ldv, a, stream);
+  a.o = o; a.ldo = ldo; a.lse = lse; a.err = err_flag; a.group = attn_group(B, H, T);
+  // Which forward, measured (us): one tile per CTA with an SM to itself and double-buffered scores (attn_fwd_k) / two tiles in one
+  // CTA with the register split (attn_fwd3, all exponentials on the ex2 unit) / two CTAs per SM (attn_fwd4):
+  //   B=1 H=8 T=32768   window 256: 135 / 121 / 100    2048: 349 / 305 / 292    4096: 576 / 510 / 509
+  //   B=4 H=8 T=8192    window 256: 144 / 135 / 109    full: 644 / 534 / 554
+  //   B=1 H=16 T=4096   full (256 pairs): 109 / 80 / 91
+  //   B=64 H=4 T=2048   window 256: 246 / 216 / 183    full: 412 / 353 / 342
+  //   B=5 H=3 T=1531 (180 query tiles)  window 256: 24.6 / 23.6 / 20.7   full: 32.9 / 36.9 / 33.0
+  //   B=1 H=4 T=2048 (64 query tiles)   window 256: 15.4 / 21.5 / 17.4   full: 29.7 / 44.0 / 40.0
+  // Up to 148 query tiles every tile has an SM to itself anyway and the first is faster.  Beyond, two CTAs per SM, except where
+  // tiles see many keys and there are pairs enough: there the fixed order of the two-tile kernel wins.  On grids of several waves
+  // of pairs that kernel evaluates one exponential in four as a cubic (B=4 H=8 T=32768 full: 8650 us, without 8838).
+  const long long ctas = (long long)((T + 127) / 128) * H * B, pair_ctas = (long long)((T + 255) / 256) * H * B;
+  const bool long_keys = T >= 4096 && window > 2048;
+  if (g_attn_mode == 4 || (g_attn_mode == 2 && long_keys && pair_ctas >= 2048)) return attn_fwd3_launch(tq, tk, tv, a, true, stream);
+  if (g_attn_mode == 6 || (g_attn_mode == 2 && long_keys && pair_ctas >= 256)) return attn_fwd3_launch(tq, tk, tv, a, false, stream);
+  if (g_attn_mode == 5 || (g_attn_mode == 2 && ctas > 148)) return attn_fwd4_launch(tq, tk, tv, a, stream);
   if (g_attn_mode == 3) return attn_fwd2_launch(q, k, v, ldq, ldk, ldv, a, stream);
   dim3 grid((T + 127) / 128, H, B);
   return g_attn_ts ? launch_fwd<true>(tq, tk, tv, a, grid, stream) : launch_fwd<false>(tq, tk, tv, a, grid, stream);

@@ -120,8 +120,8 @@ attn_bwd_dq_wide_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_mt = (p.T + 127) / 128;
-  const int mt = n_mt - 1 - int(blockIdx.x);   // later query tiles see more keys: schedule them first
-  const int h = blockIdx.y, b = blockIdx.z;
+  const AttnTile tile = attn_tile(p, n_mt);
+  const int mt = n_mt - 1 - tile.rank, h = tile.h, b = tile.b;       // later query tiles see more keys
   const int m0 = mt * 128;
   const int j_lo = (p.window >= p.T) ? 0 : max(0, (m0 - p.window) / 128);
   const int j_hi = min((p.T - 1) / 128, (m0 + 127) / 128);
@@ -343,8 +343,9 @@ attn_bwd_dkv_wide_k(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   float* stat_dl = stat_lse + 256;                                      // [2][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int n0 = int(blockIdx.x) * 128;      // earlier key tiles are seen by more queries and come first
+  const AttnTile tile = attn_tile(p, (p.T + 127) / 128);
+  const int h = tile.h, b = tile.b;
+  const int n0 = tile.rank * 128;            // earlier key tiles are seen by more queries
   const int i_lo = n0 / 128;
   const long long last_q = (p.window >= p.T) ? (long long)(p.T - 1) : min((long long)(p.T - 1), (long long)n0 + 127 + p.window);
   const int i_hi = int(last_q / 128);
@@ -574,7 +575,9 @@ int attn_wide_bwd_launch(const void* q, const void* k, const void* v, const void
   if ((r = make_qkv_tmap(&tk, k, a.B, a.T, a.H, ldk, 128))) return 1000 + r;
   if ((r = make_qkv_tmap(&tv, v, a.B, a.T, a.H, ldv, 128))) return 1000 + r;
   if ((r = make_qkv_tmap(&tdo, d_o, a.B, a.T, a.H, lddo, 128))) return 1000 + r;
-  dim3 grid((a.T + 127) / 128, a.H, a.B);
+  const unsigned grid = attn_grid(a.B, a.H, a.T, 128);
+  if (!grid) return -3;
+  a.group = attn_group(a.B, a.H, a.T);
   a.o = dq; a.ldo = lddq;
   attn_bwd_dq_wide_k<<<grid, ATT_WIDE_THREADS, WideSmem::TOTAL, stream>>>(tq, tk, tv, tdo, a);
   if ((r = int(cudaGetLastError()))) return r;

@@ -314,7 +314,8 @@ def layer_call(entry: str, pointers, sizes, eps: float, scale: float) -> None:
 
 
 def attn_set_mode(mode: int) -> None:
-    """4 = as 2, with the register-split two-query-tile forward (attn_fwd3) for every shape;
+    """6 = as 4 with every exponential on the ex2 unit; 5 = as 2, with the forward of two CTAs per SM (attn_fwd4) for every
+    shape; 4 = as 2, with the register-split two-query-tile forward (attn_fwd3) for every shape;
     3 = as 2, with the forward on two query tiles per CTA in ping-pong; 2 = backward on 128 x 128 tiles with
     the two-phase softmax; 1 = 64-wide sub-tiles with P / dS operands in TMEM; 0 = 64-wide sub-tiles with P / dS
     in shared memory (forward too)."""

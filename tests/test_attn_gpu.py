@@ -74,6 +74,22 @@ def test_attention_register_split_forward(B, T, H, window):
     _run(B, T, H, window, mode=4)
 
 
+@pytest.mark.parametrize("B,T,H,window", [(1, 5, 1, 5), (1, 128, 1, 128), (2, 256, 2, 256), (1, 384, 1, 384), (1, 512, 2, 256),
+                                         (1, 1024, 1, 256), (1, 640, 1, 64), (2, 320, 3, 100), (3, 129, 2, 129), (1, 1536, 2, 1536),
+                                         (1, 2000, 1, 700), (1, 4096, 1, 4096), (1, 300, 2, 1)])
+def test_attention_two_ctas_per_sm_forward(B, T, H, window):
+    """Forward with half an SM per CTA: a few rows, tiles that end inside, windows that start mid-tile, several heads and
+    sequences in the flat grid."""
+    _run(B, T, H, window, mode=5)
+
+
+@pytest.mark.parametrize("B,T,H,window", [(10, 1100, 9, 1100), (9, 700, 17, 200), (600, 130, 1, 130), (2, 4100, 8, 4100)])
+def test_attention_many_heads_in_groups(B, T, H, window):
+    """More tiles than SMs, so heads are interleaved: group sizes that do and do not divide the number of heads, several groups;
+    the last case is the two-tile kernel without the polynomial."""
+    _run(B, T, H, window)
+
+
 def test_attention_long_sequence():
     """Enough tiles for every ring slot and barrier phase to wrap several times."""
     _run(1, 4096, 1, 4096)

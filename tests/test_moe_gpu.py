@@ -161,7 +161,7 @@ def test_router_against_64_bits(N, D, E, K_):
                                         K._stream()), "moe_router_fwd")
     want = torch.softmax(xn.double() @ wr.double().t(), -1)
     assert (probs.double() - want).abs().max().item() < 1e-5
-    order = torch.sort(probs, -1, descending=True, stable=True).indices[:, :K_]
+    order = torch.sort(probs, dim=-1, descending=True, stable=True).indices[:, :K_]
     assert torch.equal(order.int(), idx)
     top = probs.gather(1, idx.long())
     assert (gates - top / top.sum(-1, keepdim=True)).abs().max().item() < 1e-5
