@@ -85,6 +85,7 @@ attn_fwd3_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
             const __grid_constant__ CUtensorMap tmV, const AttnArgs p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {
+    grid_wait();
     if (threadIdx.x == 0 && p.err) atomicExch(p.err, ERR_SMEM_ALIGN);
     return;
   }
@@ -132,6 +133,7 @@ attn_fwd3_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_enter();                 // global memory is not touched above
   // The data-movement warp group hands registers to the two softmax groups; each setmaxnreg is the first
   // instruction of its group's branch (executed by all four warps of the group) and dominates the group's code.
   if (warp >= 8) {
@@ -368,8 +370,7 @@ int attn_fwd3_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
   }
   const unsigned grid = attn_grid(a.B, a.H, a.T, 256);
   if (!grid) return -3;
-  (poly ? attn_fwd3_k<true> : attn_fwd3_k<false>)<<<grid, ATT_FWD3_THREADS, Fwd3Smem::TOTAL, stream>>>(tq, tk, tv, a);
-  return int(cudaGetLastError());
+  return launch_dependent(true, poly ? attn_fwd3_k<true> : attn_fwd3_k<false>, grid, ATT_FWD3_THREADS, Fwd3Smem::TOTAL, stream, tq, tk, tv, a);
 }
 
 }  // namespace arb

@@ -79,6 +79,7 @@ attn_fwd4_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_enter();                 // global memory is not touched above
   const uint32_t TM_S = tmem, TM_P = tmem + 64, TM_O = tmem + 128;
 
   if (warp == 0) {
@@ -263,8 +264,7 @@ int attn_fwd4_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
   if (cfg.first()) { if (int r = set_smem(attn_fwd4_k, Fwd4Smem::TOTAL)) return r; }
   const unsigned grid = attn_grid(a.B, a.H, a.T, 128);
   if (!grid) return -3;
-  attn_fwd4_k<<<grid, ATT_THREADS, Fwd4Smem::TOTAL, stream>>>(tq, tk, tv, a);
-  return int(cudaGetLastError());
+  return launch_dependent(true, attn_fwd4_k, grid, ATT_THREADS, Fwd4Smem::TOTAL, stream, tq, tk, tv, a);
 }
 
 }  // namespace arb

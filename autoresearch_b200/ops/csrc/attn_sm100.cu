@@ -93,6 +93,7 @@ attn_fwd_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_enter();                 // global memory is not touched above
   const uint32_t TM_S = tmem, TM_O = tmem + 256, TM_P = tmem + 384;   // S[2] x 128, O 128, P[2] x 64 (TS)
 
   if (warp == 0) {
@@ -786,6 +787,7 @@ attn_bwd_dkv_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 // per iteration), the token arithmetic done once per warp
 __global__ void __launch_bounds__(256) attn_delta_k(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                                                     float* __restrict__ delta, int B, int T, int H, long long ldo, long long lddo) {
+  grid_enter();
   const long long bt = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (bt >= (long long)B * T) return;
@@ -829,8 +831,7 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   static PerDeviceOnce cfg;
   int r;
   if (cfg.first()) { if ((r = set_smem(attn_fwd_k<TS>, FwdSmemT<TS>::TOTAL))) return r; }
-  attn_fwd_k<TS><<<grid, ATT_THREADS, FwdSmemT<TS>::TOTAL, stream>>>(tq, tk, tv, a);
-  return int(cudaGetLastError());
+  return launch_dependent(true, attn_fwd_k<TS>, grid, ATT_THREADS, FwdSmemT<TS>::TOTAL, stream, tq, tk, tv, a);
 }
 template <bool TS>
 static int launch_dq(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
@@ -895,8 +896,9 @@ extern "C" int arb_attn_bwd(const void* q, const void* k, const void* v, const v
   if (bad_ptr(q) || bad_ptr(k) || bad_ptr(v) || bad_ptr(o) || bad_ptr(d_o) || bad_ptr(dq) || bad_ptr(dk) || bad_ptr(dv)) return -4;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (ldo % 8) || (lddo % 8) || (lddq % 8) || (lddk % 8) || (lddv % 8)) return -4;
   int r;
-  attn_delta_k<<<unsigned(((long long)B * T + 7) / 8), 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, B, T, H, ldo, lddo);
-  if ((r = int(cudaGetLastError()))) return r;
+  if ((r = launch_dependent((long long)B * T * H * 256 <= EARLY_BYTES, attn_delta_k, unsigned(((long long)B * T + 7) / 8), 256, 0, stream, (const __nv_bfloat16*)o,
+                            (const __nv_bfloat16*)d_o, delta, B, T, H, ldo, lddo)))
+    return r;
   AttnArgs a{};
   a.B = B; a.T = T; a.H = H; a.window = window > T ? T : window; a.scale = scale;
   a.lse = const_cast<float*>(lse); a.delta = delta; a.err = err_flag;

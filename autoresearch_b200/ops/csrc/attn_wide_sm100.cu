@@ -102,6 +102,7 @@ attn_bwd_dq_wide_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, const AttnArgs p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {   // the swizzled tiles need 1 KB alignment; nothing has been allocated yet
+    grid_wait();
     if (threadIdx.x == 0 && p.err) atomicExch(p.err, ERR_SMEM_ALIGN);
     return;
   }
@@ -142,6 +143,7 @@ attn_bwd_dq_wide_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_enter();                 // global memory is not touched above
   const uint32_t TM_S = tmem, TM_DP = tmem + 128, TM_DQ = tmem + 256, TM_DS = tmem + 384;
 
   if (warp == 0) {
@@ -323,6 +325,7 @@ attn_bwd_dkv_wide_k(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, const AttnArgs p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {
+    grid_wait();
     if (threadIdx.x == 0 && p.err) atomicExch(p.err, ERR_SMEM_ALIGN);
     return;
   }
@@ -364,6 +367,7 @@ attn_bwd_dkv_wide_k(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_enter();                 // global memory is not touched above
   const uint32_t TM_S = tmem, TM_DP = tmem + 128, TM_DV = tmem + 256, TM_DK = tmem + 384;
 
   if (warp == 0) {
@@ -579,11 +583,9 @@ int attn_wide_bwd_launch(const void* q, const void* k, const void* v, const void
   if (!grid) return -3;
   a.group = attn_group(a.B, a.H, a.T);
   a.o = dq; a.ldo = lddq;
-  attn_bwd_dq_wide_k<<<grid, ATT_WIDE_THREADS, WideSmem::TOTAL, stream>>>(tq, tk, tv, tdo, a);
-  if ((r = int(cudaGetLastError()))) return r;
+  if ((r = launch_dependent(true, attn_bwd_dq_wide_k, grid, ATT_WIDE_THREADS, WideSmem::TOTAL, stream, tq, tk, tv, tdo, a))) return r;
   a.dk = dk; a.dv = dv; a.lddk = lddk; a.lddv = lddv;
-  attn_bwd_dkv_wide_k<<<grid, ATT_WIDE_THREADS, WideSmem::TOTAL, stream>>>(tq, tk, tv, tdo, a);
-  return int(cudaGetLastError());
+  return launch_dependent(true, attn_bwd_dkv_wide_k, grid, ATT_WIDE_THREADS, WideSmem::TOTAL, stream, tq, tk, tv, tdo, a);
 }
 
 }  // namespace arb

@@ -17,6 +17,7 @@ template <int VPT>  // 8-element vectors per thread
 __global__ void __launch_bounds__(CE_THREADS) softcap_ce_k(__nv_bfloat16* __restrict__ logits, long long ld,
                                                            const int* __restrict__ targets, float* __restrict__ loss,
                                                            int V, float cap, float gscale) {
+  grid_enter();
   __shared__ float red[CE_THREADS / 32];
   const long long row = blockIdx.x;
   __nv_bfloat16* p = logits + row * ld;
@@ -90,11 +91,12 @@ extern "C" int arb_softcap_ce(void* logits, long long ld, const int* targets, fl
   const int nch = V / 8;
   const int vpt = (nch + CE_THREADS - 1) / CE_THREADS;
   __nv_bfloat16* p = reinterpret_cast<__nv_bfloat16*>(logits);
-  if (vpt <= 1) softcap_ce_k<1><<<unsigned(rows), CE_THREADS, 0, s>>>(p, ld, targets, loss, V, softcap, dlogits_scale);
-  else if (vpt <= 2) softcap_ce_k<2><<<unsigned(rows), CE_THREADS, 0, s>>>(p, ld, targets, loss, V, softcap, dlogits_scale);
-  else if (vpt <= 4) softcap_ce_k<4><<<unsigned(rows), CE_THREADS, 0, s>>>(p, ld, targets, loss, V, softcap, dlogits_scale);
-  else if (vpt <= 8) softcap_ce_k<8><<<unsigned(rows), CE_THREADS, 0, s>>>(p, ld, targets, loss, V, softcap, dlogits_scale);
-  else if (vpt <= 16) softcap_ce_k<16><<<unsigned(rows), CE_THREADS, 0, s>>>(p, ld, targets, loss, V, softcap, dlogits_scale);
+  const bool early = rows * V * 2 <= EARLY_BYTES;
+  if (vpt <= 1) launch_dependent(early, softcap_ce_k<1>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
+  else if (vpt <= 2) launch_dependent(early, softcap_ce_k<2>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
+  else if (vpt <= 4) launch_dependent(early, softcap_ce_k<4>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
+  else if (vpt <= 8) launch_dependent(early, softcap_ce_k<8>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
+  else if (vpt <= 16) launch_dependent(early, softcap_ce_k<16>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
   else return -3;  // vocabularies above 32768 are not supported by this kernel
   return int(cudaGetLastError());
 }

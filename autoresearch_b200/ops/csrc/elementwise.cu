@@ -43,6 +43,7 @@ constexpr int ROWS_PER_CTA = 8;  // 8 warps, one row each
 template <int NV>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_k(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                                      long long rows, int D, float eps) {
+  grid_enter();
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * ROWS_PER_CTA + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -76,6 +77,7 @@ template <int NV>
 __global__ void __launch_bounds__(256) rmsnorm_bwd_k(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
                                                      const __nv_bfloat16* __restrict__ add_to, __nv_bfloat16* __restrict__ gx,
                                                      long long rows, int D, float eps) {
+  grid_enter();
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * ROWS_PER_CTA + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -138,6 +140,7 @@ __global__ void __launch_bounds__(256) resid_norm_fwd_k(const __nv_bfloat16* __r
                                                         const __nv_bfloat16* __restrict__ lam_r, const __nv_bfloat16* __restrict__ lam_0,
                                                         int idx, __nv_bfloat16* __restrict__ xo, __nv_bfloat16* __restrict__ xn,
                                                         long long rows, int D, float eps) {
+  grid_enter();
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * ROWS_PER_CTA + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -182,6 +185,7 @@ __global__ void __launch_bounds__(256) resid_norm_bwd_k(const __nv_bfloat16* __r
                                                         const __nv_bfloat16* d_x0_acc,
                                                         float* __restrict__ dlam_r, float* __restrict__ dlam_0,
                                                         long long rows, int D, float eps) {
+  grid_enter();
   // d_x0_acc (may equal d_x0): the x0 gradient of the layers above, added here instead of by a separate pass
   __shared__ float red[2][ROWS_PER_CTA];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -260,6 +264,7 @@ __global__ void __launch_bounds__(256) resid_norm_bwd_k(const __nv_bfloat16* __r
 
 // ---------------------------------------------------------------------------------------------
 __global__ void residual_add_k(const uint4* __restrict__ a, const uint4* __restrict__ b, uint4* __restrict__ o, long long n8) {
+  grid_enter();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
     float x[8], y[8];
     ld8(reinterpret_cast<const __nv_bfloat16*>(a + i), x);
@@ -305,6 +310,7 @@ __global__ void accum_bf16_f32_k(const uint2* __restrict__ s, float4* __restrict
 }
 // dst[r, 0:cols] += src[r, 0:cols]  (dst row stride ld_dst, src dense)
 __global__ void add_cols_k(__nv_bfloat16* dst, long long ld_dst, const __nv_bfloat16* src, long long rows, int cols) {
+  grid_enter();
   const long long n = rows * cols;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / cols;
@@ -318,6 +324,7 @@ __global__ void add_cols_k(__nv_bfloat16* dst, long long ld_dst, const __nv_bflo
 // embedding
 __global__ void embedding_fwd_k(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                 long long N, int D, int vocab) {
+  grid_enter();
   const int nch = D >> 3;
   const long long total = N * nch;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -359,6 +366,7 @@ __global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_sorted_k(const long
                                                               const int* __restrict__ seg_count, const __nv_bfloat16* __restrict__ g,
                                                               float* __restrict__ dw, float* __restrict__ partial, int n_items_max,
                                                               int D, int R, int vocab) {
+  grid_enter();
   __shared__ __align__(16) float red[EMB_THREADS][8];
   const int item = blockIdx.x;
   const int id = item_id[item];
@@ -418,6 +426,7 @@ __global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_sorted_k(const long
 }
 __global__ void __launch_bounds__(128) embedding_bwd_combine_k(const int* __restrict__ item_start, const int* __restrict__ seg_count,
                                                                const float* __restrict__ partial, float* __restrict__ dw, int D, int R) {
+  grid_enter();
   const int id = blockIdx.x;
   const int cnt = seg_count[id];
   if (cnt <= R) return;
@@ -443,6 +452,7 @@ constexpr int PLAN_MAX_VOCAB = 49152;                // one counter per id in sh
 __device__ __forceinline__ int plan_id(const int* ids, long long i, int vocab) { return min(max(ids[i], 0), vocab - 1); }
 
 __global__ void __launch_bounds__(256) emb_plan_hist_k(const int* __restrict__ ids, long long N, int vocab, int* __restrict__ hist) {
+  grid_enter();
   extern __shared__ int plan_cnt[];
   for (int v = threadIdx.x; v < vocab; v += 256) plan_cnt[v] = 0;
   __syncthreads();
@@ -452,6 +462,7 @@ __global__ void __launch_bounds__(256) emb_plan_hist_k(const int* __restrict__ i
   for (int v = threadIdx.x; v < vocab; v += 256) hist[(long long)blockIdx.x * vocab + v] = plan_cnt[v];
 }
 __global__ void __launch_bounds__(64) emb_plan_chunks_k(int* __restrict__ hist, int n_chunks, int vocab, int* __restrict__ counts) {
+  grid_enter();
   const int v = blockIdx.x * 64 + threadIdx.x;
   if (v >= vocab) return;
   int sum = 0;
@@ -470,6 +481,7 @@ __global__ void __launch_bounds__(64) emb_plan_chunks_k(int* __restrict__ hist, 
 __global__ void __launch_bounds__(1024) emb_plan_scan_k(const int* __restrict__ counts, int vocab, int R, int n_items_max,
                                                         int* __restrict__ seg_start, int* __restrict__ item_start,
                                                         int* __restrict__ item_id) {
+  grid_enter();
   __shared__ int wsum[2][32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int row0 = 0, it0 = 0;                             // rows and items of the ids below this round's
@@ -505,6 +517,7 @@ __global__ void __launch_bounds__(1024) emb_plan_scan_k(const int* __restrict__ 
 }
 __global__ void __launch_bounds__(256) emb_plan_place_k(const int* __restrict__ ids, long long N, int vocab, const int* __restrict__ hist,
                                                         const int* __restrict__ seg_start, long long* __restrict__ perm) {
+  grid_enter();
   extern __shared__ int plan_cnt[];                  // next sorted position of every id
   for (int v = threadIdx.x; v < vocab; v += 256) plan_cnt[v] = seg_start[v] + hist[(long long)blockIdx.x * vocab + v];
   __syncthreads();
@@ -548,6 +561,7 @@ __global__ void __launch_bounds__(256) qkv_post_fwd_k(__nv_bfloat16* __restrict_
                                                       const __nv_bfloat16* __restrict__ ve_w, const __nv_bfloat16* __restrict__ gate_w,
                                                       float* __restrict__ gate_out, long long N, int T, int H, int D_model,
                                                       int gate_ch, float eps) {
+  grid_enter();
   const int lane = threadIdx.x & 31;
   const long long tok = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (tok >= N) return;
@@ -612,6 +626,7 @@ __global__ void __launch_bounds__(256) qkv_post_bwd_k(__nv_bfloat16* __restrict_
                                                       const __nv_bfloat16* __restrict__ gate_w, const float* __restrict__ gate,
                                                       __nv_bfloat16* __restrict__ d_ve, float* __restrict__ d_gate_logit,
                                                       long long N, int T, int H) {
+  grid_enter();
   const int lane = threadIdx.x & 31;
   const long long tok = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (tok >= N) return;
@@ -678,6 +693,7 @@ __global__ void __launch_bounds__(256) ve_gate_bwd_k(const float* __restrict__ d
                                                      const __nv_bfloat16* __restrict__ gate_w, float* __restrict__ d_gate_w,
                                                      __nv_bfloat16* __restrict__ d_xn_gate, long long N, int H, int D_model,
                                                      int ch, int tok_per_cta, int chunk) {
+  grid_enter();
   extern __shared__ float ve_sm[];
   float* xs = ve_sm;                  // [chunk][ch]
   float* ds = ve_sm + chunk * ch;     // [chunk][H]
@@ -726,11 +742,11 @@ static inline int grid_for(long long n, int threads, int cap = 148 * 16) {
 #define ROW_DISPATCH(KERNEL, ...)                                                        \
   do {                                                                                     \
     const int blocks = int((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA);                      \
-    if (D <= 256) KERNEL<1><<<blocks, 256, 0, s>>>(__VA_ARGS__);                           \
-    else if (D <= 512) KERNEL<2><<<blocks, 256, 0, s>>>(__VA_ARGS__);                      \
-    else if (D <= 1024) KERNEL<4><<<blocks, 256, 0, s>>>(__VA_ARGS__);                     \
-    else if (D <= 2048) KERNEL<8><<<blocks, 256, 0, s>>>(__VA_ARGS__);                     \
-    else KERNEL<16><<<blocks, 256, 0, s>>>(__VA_ARGS__);                                   \
+    if (D <= 256) launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<1>, blocks, 256, 0, s, __VA_ARGS__);                           \
+    else if (D <= 512) launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<2>, blocks, 256, 0, s, __VA_ARGS__);                      \
+    else if (D <= 1024) launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<4>, blocks, 256, 0, s, __VA_ARGS__);                     \
+    else if (D <= 2048) launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<8>, blocks, 256, 0, s, __VA_ARGS__);                     \
+    else launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<16>, blocks, 256, 0, s, __VA_ARGS__);                                   \
   } while (0)
 
 static inline int check_row_args(long long rows, int D) {
@@ -761,11 +777,11 @@ int arb_resid_scale_norm_fwd(const void* x, const void* x0, const void* lam_r, c
   if (check_row_args(rows, D) || misaligned(x) || misaligned(x0) || misaligned(x_out) || misaligned(xn_out)) return -3;
 #define RSN(NV) resid_norm_fwd_k<NV, true>
   const int blocks = int((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA);
-  if (D <= 256) RSN(1)<<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 512) RSN(2)<<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 1024) RSN(4)<<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 2048) RSN(8)<<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else RSN(16)<<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  if (D <= 256) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(1), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 512) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(2), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 1024) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(4), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 2048) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(8), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(16), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
 #undef RSN
   return int(cudaGetLastError());
 }
@@ -773,11 +789,11 @@ int arb_add_norm_fwd(const void* x, const void* proj, void* x_out, void* xn_out,
   if (check_row_args(rows, D) || misaligned(x) || misaligned(proj) || misaligned(x_out) || misaligned(xn_out)) return -3;
 #define RSN(NV) resid_norm_fwd_k<NV, false>
   const int blocks = int((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA);
-  if (D <= 256) RSN(1)<<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 512) RSN(2)<<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 1024) RSN(4)<<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 2048) RSN(8)<<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else RSN(16)<<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  if (D <= 256) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(1), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 512) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(2), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 1024) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(4), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 2048) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(8), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(16), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
 #undef RSN
   return int(cudaGetLastError());
 }
@@ -793,7 +809,7 @@ int arb_resid_scale_norm_bwd(const void* x, const void* x0, const void* lam_r, c
 }
 int arb_residual_add(const void* a, const void* b, void* out, long long n, cudaStream_t s) {
   if (n <= 0 || (n & 7) || misaligned(a) || misaligned(b) || misaligned(out)) return -3;
-  residual_add_k<<<grid_for(n / 8, 256), 256, 0, s>>>((const uint4*)a, (const uint4*)b, (uint4*)out, n / 8);
+  launch_dependent(n * 2 <= EARLY_BYTES, residual_add_k, grid_for(n / 8, 256), 256, 0, s, (const uint4*)a, (const uint4*)b, (uint4*)out, n / 8);
   return int(cudaGetLastError());
 }
 int arb_relu_sq_fwd(const void* x, void* y, long long n, cudaStream_t s) {
@@ -811,7 +827,7 @@ int arb_qkv_post_fwd(void* qkv, const void* cos_t, const void* sin_t, float* rst
                      int gate_ch, float eps, cudaStream_t s) {
   if (N <= 0 || T <= 0 || H <= 0 || misaligned(qkv) || (reinterpret_cast<uintptr_t>(cos_t) & 7) || (reinterpret_cast<uintptr_t>(sin_t) & 7)) return -3;
   if (ve_w && (!gate_w || !gate_out || !xn || !ids || misaligned(ve_w))) return -3;
-  qkv_post_fwd_k<<<int((N + 7) / 8), 256, 0, s>>>((bf16*)qkv, (const bf16*)cos_t, (const bf16*)sin_t, rstd_qk, (const bf16*)xn, ids,
+  launch_dependent(N * H * 768 <= EARLY_BYTES, qkv_post_fwd_k, int((N + 7) / 8), 256, 0, s, (bf16*)qkv, (const bf16*)cos_t, (const bf16*)sin_t, rstd_qk, (const bf16*)xn, ids,
                                                       (const bf16*)ve_w, (const bf16*)gate_w, gate_out, N, T, H, D_model, gate_ch, eps);
   return int(cudaGetLastError());
 }
@@ -820,7 +836,7 @@ int arb_qkv_post_bwd(void* d_qkv, const void* qkv, const void* cos_t, const void
                      void* d_xn_gate, float* dgl, long long N, int T, int H, int D_model, int gate_ch, cudaStream_t s) {
   if (N <= 0 || T <= 0 || H <= 0 || misaligned(d_qkv) || misaligned(qkv)) return -3;
   if (ve_w && (!gate_w || !gate || !xn || !ids || !d_ve || !d_gate_w || !d_xn_gate || !dgl)) return -3;
-  qkv_post_bwd_k<<<int((N + 7) / 8), 256, 0, s>>>((bf16*)d_qkv, (const bf16*)qkv, (const bf16*)cos_t, (const bf16*)sin_t, rstd_qk,
+  launch_dependent(N * H * 768 <= EARLY_BYTES, qkv_post_bwd_k, int((N + 7) / 8), 256, 0, s, (bf16*)d_qkv, (const bf16*)qkv, (const bf16*)cos_t, (const bf16*)sin_t, rstd_qk,
                                                       (const bf16*)xn, ids, (const bf16*)ve_w, (const bf16*)gate_w, gate, (bf16*)d_ve,
                                                       dgl, N, T, H);
   int rc = int(cudaGetLastError());
@@ -832,15 +848,14 @@ int arb_qkv_post_bwd(void* d_qkv, const void* qkv, const void* cos_t, const void
     if (chunk > VE_CHUNK) chunk = VE_CHUNK;
     if (chunk < 1) return -3;
     if (chunk > tpc) chunk = int(tpc);
-    ve_gate_bwd_k<<<unsigned((N + tpc - 1) / tpc), 256, size_t(chunk) * 4 * (gate_ch + H), s>>>(
-        dgl, (const bf16*)xn, (const bf16*)gate_w, d_gate_w, (bf16*)d_xn_gate, N, H, D_model, gate_ch, int(tpc), chunk);
+    launch_dependent(N * gate_ch * 2 <= EARLY_BYTES, ve_gate_bwd_k, unsigned((N + tpc - 1) / tpc), 256, size_t(chunk) * 4 * (gate_ch + H), s, dgl, (const bf16*)xn, (const bf16*)gate_w, d_gate_w, (bf16*)d_xn_gate, N, H, D_model, gate_ch, int(tpc), chunk);
     if (!rc) rc = int(cudaGetLastError());
   }
   return rc;
 }
 int arb_embedding_fwd(const int* ids, const void* w, void* out, long long N, int D, int vocab, cudaStream_t s) {
   if (N <= 0 || (D & 7) || misaligned(w) || misaligned(out)) return -3;
-  embedding_fwd_k<<<grid_for(N * (D / 8), 256), 256, 0, s>>>(ids, (const bf16*)w, (bf16*)out, N, D, vocab);
+  launch_dependent(N * D * 2 <= EARLY_BYTES, embedding_fwd_k, grid_for(N * (D / 8), 256), 256, 0, s, ids, (const bf16*)w, (bf16*)out, N, D, vocab);
   return int(cudaGetLastError());
 }
 int arb_embedding_bwd(const int* ids, const void* g, float* dw, long long N, int D, int vocab, cudaStream_t s) {
@@ -856,11 +871,11 @@ int arb_embedding_bwd_sorted(const long long* perm, const int* item_id, const in
                              const int* seg_count, const void* g, float* dw, float* partial, int n_items_max, int D, int R,
                              int vocab, cudaStream_t s) {
   if (n_items_max <= 0 || (D & 7) || R <= 0 || vocab <= 0 || misaligned(g) || misaligned(dw) || misaligned(partial)) return -3;
-  embedding_bwd_sorted_k<<<n_items_max, EMB_THREADS, 0, s>>>(perm, item_id, item_start, seg_start, seg_count, (const bf16*)g, dw, partial,
+  launch_dependent((long long)(n_items_max - vocab) * R * D * 2 <= EARLY_BYTES, embedding_bwd_sorted_k, n_items_max, EMB_THREADS, 0, s, perm, item_id, item_start, seg_start, seg_count, (const bf16*)g, dw, partial,
                                                      n_items_max, D, R, vocab);
   int rc = int(cudaGetLastError());
   if (rc) return rc;
-  embedding_bwd_combine_k<<<vocab, 128, 0, s>>>(item_start, seg_count, partial, dw, D, R);
+  launch_dependent((long long)(n_items_max - vocab) * D * 4 <= EARLY_BYTES, embedding_bwd_combine_k, vocab, 128, 0, s, item_start, seg_count, partial, dw, D, R);
   return int(cudaGetLastError());
 }
 int arb_embedding_plan(const int* ids, long long N, int vocab, int R, int n_items_max, int* hist, long long* perm, int* counts,
@@ -874,15 +889,15 @@ int arb_embedding_plan(const int* ids, long long N, int vocab, int R, int n_item
     if (e == cudaSuccess) e = cudaFuncSetAttribute(emb_plan_place_k, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_MAX_VOCAB * 4);
     if (e != cudaSuccess) return int(e);
   }
-  emb_plan_hist_k<<<chunks, 256, smem, s>>>(ids, N, vocab, hist);
-  emb_plan_chunks_k<<<(vocab + 63) / 64, 64, 0, s>>>(hist, int(chunks), vocab, counts);
-  emb_plan_scan_k<<<1, 1024, 0, s>>>(counts, vocab, R, n_items_max, seg_start, item_start, item_id);
-  emb_plan_place_k<<<chunks, 256, smem, s>>>(ids, N, vocab, hist, seg_start, perm);
+  launch_dependent(true, emb_plan_hist_k, chunks, 256, smem, s, ids, N, vocab, hist);
+  launch_dependent(true, emb_plan_chunks_k, (vocab + 63) / 64, 64, 0, s, hist, int(chunks), vocab, counts);
+  launch_dependent(true, emb_plan_scan_k, 1, 1024, 0, s, counts, vocab, R, n_items_max, seg_start, item_start, item_id);
+  launch_dependent(true, emb_plan_place_k, chunks, 256, smem, s, ids, N, vocab, hist, seg_start, perm);
   return int(cudaGetLastError());
 }
 int arb_add_cols(void* dst, long long ld_dst, const void* src, long long rows, int cols, cudaStream_t s) {
   if (rows <= 0 || cols <= 0) return -3;
-  add_cols_k<<<grid_for(rows * cols, 256), 256, 0, s>>>((bf16*)dst, ld_dst, (const bf16*)src, rows, cols);
+  launch_dependent(rows * cols * 2 <= EARLY_BYTES, add_cols_k, grid_for(rows * cols, 256), 256, 0, s, (bf16*)dst, ld_dst, (const bf16*)src, rows, cols);
   return int(cudaGetLastError());
 }
 int arb_cast_f32_to_bf16(const float* src, void* dst, long long n, float scale, cudaStream_t s) {

@@ -263,7 +263,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int items = p.batch * p.m_tiles * p.n_tiles * p.splitk;
-  pull_prologue(p);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -276,6 +275,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_enter();                 // global memory is not touched above
+  pull_prologue(p);
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -522,7 +523,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int cluster_id = blockIdx.x >> 1;
   const int n_clusters = gridDim.x >> 1;
   const int items = p.batch * p.m_tiles * p.n_tiles * p.splitk;   // m_tiles counted in 256-row tiles
-  pull_prologue(p);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -535,6 +535,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_enter();                 // global memory is not touched above
+  pull_prologue(p);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -877,8 +879,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
   const int grid = items < g_num_sms ? items : g_num_sms;
   GemmArgs args = a;
   if (int r = arm_pull(args, grid)) return r;
-  kern<<<grid, GEMM_THREADS, L::TOTAL, st>>>(ta, tb, args);
-  return int(cudaGetLastError());
+  return launch_dependent(true, kern, grid, GEMM_THREADS, L::TOTAL, st, ta, tb, args);
 }
 
 template <bool A_MN, bool B_MN, int EPI>
@@ -913,13 +914,15 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
   cfg.blockDim = dim3(GEMM_THREADS);
   cfg.dynamicSmemBytes = Smem2<EPI>::TOTAL;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // as launch_dependent()
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   GemmArgs args = a;
   if (int r = arm_pull(args, clusters * 2)) return r;
   return int(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tx, args));
