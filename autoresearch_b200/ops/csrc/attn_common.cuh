@@ -30,8 +30,8 @@ struct AttnArgs {
 // B=1 H=16 T=8192: 328 us, grouped 277; B=1 H=16 T=4096: 120, 82.  All pairs in one group lose their K and V between a tile and
 // the next once they outgrow L2: B=64 H=4 T=2048: 403 us, one after the other 361.
 struct AttnTile { int rank, h, b; };
-__device__ __forceinline__ AttnTile attn_tile(const AttnArgs& p, int n_tiles) {
-  const int per = p.group * n_tiles, g = int(blockIdx.x) / per, i = int(blockIdx.x) - g * per;
+__device__ __forceinline__ AttnTile attn_tile(const AttnArgs& p, int n_tiles, int block = int(blockIdx.x)) {
+  const int per = p.group * n_tiles, g = block / per, i = block - g * per;
   const int n = min(p.group, p.B * p.H - g * p.group);
   const int bh = g * p.group + i % n, b = bh / p.H;
   return {i / n, bh - b * p.H, b};
@@ -55,13 +55,14 @@ inline unsigned attn_grid(int B, int H, int T, int rows) {
 // arb_attn_prof_buffer[role * 8 ..]; counter 0 is the role's total.  Compiled out by default.
 #ifdef ARB_ATTN_PROF
 __device__ long long* arb_attn_prof_buffer;
+#define PROF_CTA0 (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
 #define PROF_DECL() long long prof_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}; long long prof_t0 = clock64(); const long long prof_begin = prof_t0
 #define PROF_TIC() prof_t0 = clock64()
 #define PROF_TOC(i) do { const long long prof_t1 = clock64(); prof_acc[i] += prof_t1 - prof_t0; prof_t0 = prof_t1; } while (0)
 #define PROF_DUMP(role)                                                                                   \
   do {                                                                                                    \
     prof_acc[0] = clock64() - prof_begin;                                                                 \
-    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && arb_attn_prof_buffer)                    \
+    if (PROF_CTA0 && arb_attn_prof_buffer)                                                                \
       for (int prof_i = 0; prof_i < 8; ++prof_i) arb_attn_prof_buffer[(role) * 8 + prof_i] = prof_acc[prof_i]; \
   } while (0)
 #else
