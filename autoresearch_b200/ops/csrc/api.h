@@ -17,6 +17,8 @@ enum ArbEpilogue {
   EPI_ADD_AUX = 6,      // C = aux + acc                (bf16)
   EPI_QKV_POST = 7,     // packed q|k|v projection: RoPE + RMS norm on q and k heads, value embedding on v heads (bf16);
                         // 2-CTA tiles, NT layout; parameters from arb_gemm_qkv_post_args
+  EPI_SYM_STORE = 8,    // as EPI_STORE_BF16 / EPI_NS_COMBINE of a product that is symmetric (M = N, op(B) = op(A)^T, or A = A^T = B):
+  EPI_SYM_NS_COMBINE = 9,  // above 768 a side the 2-CTA tiles below the diagonal are written as transposes
 };
 
 enum ArbError {

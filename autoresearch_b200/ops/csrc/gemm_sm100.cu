@@ -481,7 +481,37 @@ __device__ __forceinline__ void qkv_post_head(float (&f)[128], const QkvPostArgs
 // each CTA runs the epilogue for its 128 rows.  Loads carry no cluster multicast.
 // ------------------------------------------------------------------------------------------
 __host__ __device__ constexpr bool epi_is_bf16(int epi) { return epi != EPI_ATOMIC_F32 && epi != EPI_STORE_F32; }
-__host__ __device__ constexpr bool epi_has_aux(int epi) { return epi == EPI_NS_COMBINE || epi == EPI_RELU2_BWD || epi == EPI_ADD_AUX; }
+__host__ __device__ constexpr bool epi_has_aux(int epi) {
+  return epi == EPI_NS_COMBINE || epi == EPI_RELU2_BWD || epi == EPI_ADD_AUX || epi == EPI_SYM_NS_COMBINE;
+}
+__host__ __device__ constexpr bool epi_is_sym(int epi) { return epi == EPI_SYM_STORE || epi == EPI_SYM_NS_COMBINE; }
+
+// Work item -> output tile.  A symmetric product (Gram matrix, its square) computes the tiles on and above the diagonal only and
+// its epilogue also writes the transpose: 10 of 16 tiles at 1024, 36 of 64 at 2048.
+struct TileXY { int mt, nt, ks, b; };
+template <bool SYM>
+__host__ __device__ __forceinline__ TileXY tile_of(const GemmArgs& p, int w) {
+  TileXY t;
+  if (SYM) {
+    const int per = p.n_tiles * (p.n_tiles + 1) / 2;
+    t.b = w / per;
+    int i = w - t.b * per;
+    t.mt = 0;
+    while (i >= p.n_tiles - t.mt) { i -= p.n_tiles - t.mt; ++t.mt; }
+    t.nt = t.mt + i;
+    t.ks = 0;
+  } else {
+    t.nt = w % p.n_tiles; w /= p.n_tiles;
+    t.mt = w % p.m_tiles; w /= p.m_tiles;
+    t.ks = w % p.splitk;
+    t.b = w / p.splitk;
+  }
+  return t;
+}
+template <bool SYM>
+__host__ __device__ __forceinline__ int tile_count(const GemmArgs& p) {
+  return SYM ? p.batch * (p.n_tiles * (p.n_tiles + 1) / 2) : p.batch * p.m_tiles * p.n_tiles * p.splitk;
+}
 
 // bf16 outputs leave through a swizzled smem staging slab (128 rows x 64 columns, double buffered)
 // and TMA stores, so every request to L2 is a full line; aux operands arrive the same way.
@@ -522,7 +552,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const bool leader = rank == 0;
   const int cluster_id = blockIdx.x >> 1;
   const int n_clusters = gridDim.x >> 1;
-  const int items = p.batch * p.m_tiles * p.n_tiles * p.splitk;   // m_tiles counted in 256-row tiles
+  constexpr bool SYM = epi_is_sym(EPI);
+  const int items = tile_count<SYM>(p);                            // m_tiles counted in 256-row tiles
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -545,11 +576,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t it = 0;
       bool ok = true;
       for (int w = cluster_id; w < items && ok; w += n_clusters) {
-        int t = w;
-        const int nt = t % p.n_tiles; t /= p.n_tiles;
-        const int mt = t % p.m_tiles; t /= p.m_tiles;
-        const int ks = t % p.splitk;
-        const int b = t / p.splitk;
+        const TileXY tile = tile_of<SYM>(p, w);
+        const int nt = tile.nt, mt = tile.mt, ks = tile.ks, b = tile.b;
         const int kb0 = ks * p.kb_per_split;
         const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
         const int m0 = mt * 256 + int(rank) * 128;
@@ -589,10 +617,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t it = 0, tile_it = 0;
       bool ok = true;
       for (int w = cluster_id; w < items && ok; w += n_clusters) {
-        int t = w / p.n_tiles;
-        const int mt = t % p.m_tiles; t /= p.m_tiles;
-        const int ks = t % p.splitk;
-        const int b = t / p.splitk;
+        const TileXY tile = tile_of<SYM>(p, w);
+        const int mt = tile.mt, ks = tile.ks, b = tile.b;
         const int kb0 = ks * p.kb_per_split;
         const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
         if (!item_live(p, b, mt * 256, kb0, kb1)) continue;
@@ -637,11 +663,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint32_t tile_it = 0, slab_it = 0;
     bool ok = true;
     for (int w = cluster_id; w < items; w += n_clusters) {
-      int t = w;
-      const int nt = t % p.n_tiles; t /= p.n_tiles;
-      const int mt = t % p.m_tiles; t /= p.m_tiles;
-      const int ks = t % p.splitk;
-      const int b = t / p.splitk;
+      const TileXY tile = tile_of<SYM>(p, w);
+      const int nt = tile.nt, mt = tile.mt, ks = tile.ks, b = tile.b;
       {
         const int kb0 = ks * p.kb_per_split;
         if (!item_live(p, b, mt * 256, kb0, min(p.kb_total, kb0 + p.kb_per_split))) continue;
@@ -755,18 +778,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               if (nsl == 4) {                              // the next item of this cluster that is not skipped
                 nsl = 0;
                 for (nw = w + n_clusters; nw < items; nw += n_clusters) {
-                  int tt = nw / p.n_tiles;
-                  const int nmt = tt % p.m_tiles; tt /= p.m_tiles;
-                  const int nks = tt % p.splitk;
-                  const int nkb0 = nks * p.kb_per_split;
-                  if (item_live(p, tt / p.splitk, nmt * 256, nkb0, min(p.kb_total, nkb0 + p.kb_per_split))) break;
+                  const TileXY nx = tile_of<SYM>(p, nw);
+                  const int nkb0 = nx.ks * p.kb_per_split;
+                  if (item_live(p, nx.b, nx.mt * 256, nkb0, min(p.kb_total, nkb0 + p.kb_per_split))) break;
                 }
               }
               if (nw < items) {
-                int tt = nw;
-                const int nnt = tt % p.n_tiles; tt /= p.n_tiles;
-                const int nmt = tt % p.m_tiles; tt /= p.m_tiles;
-                const int nb = tt / p.splitk;
+                const TileXY nx = tile_of<SYM>(p, nw);
+                const int nnt = nx.nt, nmt = nx.mt, nb = nx.b;
                 mbar_expect_tx(&xfull_bar[buf ^ 1], 16384);
                 tma_load_3d(smem + L::X_STAGE + (buf ^ 1) * 16384, &tmX, &xfull_bar[buf ^ 1], nnt * BN2 + nsl * 64,
                             nmt * 256 + int(rank) * 128, nb);
@@ -797,7 +816,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                   float& x = f[j + e];
-                  if (EPI == EPI_NS_COMBINE) x = p.beta * ax[e] + p.gamma * x + ((row == col_s + hc * 32 + j + e) ? p.alpha : 0.f);
+                  if (EPI == EPI_NS_COMBINE || EPI == EPI_SYM_NS_COMBINE) x = p.beta * ax[e] + p.gamma * x + ((row == col_s + hc * 32 + j + e) ? p.alpha : 0.f);
                   else if (EPI == EPI_RELU2_BWD) x = x * 2.f * sqrtf(fmaxf(ax[e], 0.f));
                   else x = x + ax[e];
                 }
@@ -809,6 +828,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               u.x = pack_bf16(f[j], f[j + 1]); u.y = pack_bf16(f[j + 2], f[j + 3]);
               u.z = pack_bf16(f[j + 4], f[j + 5]); u.w = pack_bf16(f[j + 6], f[j + 7]);
               st_sw128(cbase, 128, r_local, hc * 32 + j, u);
+            }
+            if (SYM && nt > mt) {
+              // the transpose: two neighbouring rows (lanes) exchange halves of a column pair, so that an even lane holds two
+              // rows of column j and an odd one two rows of column j + 1, i.e. four adjacent bytes of the mirrored row
+              const bool odd = lane & 1;
+#pragma unroll
+              for (int j = 0; j < 32; j += 2) {
+                const float got = __shfl_xor_sync(0xffffffffu, odd ? f[j] : f[j + 1], 1);
+                const int col = col_s + hc * 32 + j + (odd ? 1 : 0);
+                const uint32_t v2 = odd ? pack_bf16(got, f[j + 1]) : pack_bf16(f[j], got);
+                if (row_ok && col < p.N)
+                  *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.C) + (long long)b * p.stride_c +
+                                               (long long)col * p.ldc + (row & ~1)) = v2;
+              }
             }
           }
           fence_proxy_async_smem();
@@ -906,7 +939,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem2<EPI>::TOTAL);
     if (e != cudaSuccess) return int(e);
   }
-  const int items = a.batch * a.m_tiles * a.n_tiles * a.splitk;
+  const int items = tile_count<epi_is_sym(EPI)>(a);
   int clusters = g_num_sms / 2;
   if (items < clusters) clusters = items;
   cudaLaunchConfig_t cfg = {};
@@ -940,6 +973,12 @@ static int dispatch_pair(int epi, const CUtensorMap& ta, const CUtensorMap& tb, 
     case EPI_ADD_AUX: return launch_pair<A_MN, B_MN, EPI_ADD_AUX>(ta, tb, a, st);
     case EPI_QKV_POST:
       if constexpr (!A_MN && !B_MN) return launch_pair<false, false, EPI_QKV_POST>(ta, tb, a, st);
+      else return -3;
+    case EPI_SYM_STORE:
+      if constexpr (A_MN == B_MN) return launch_pair<A_MN, B_MN, EPI_SYM_STORE>(ta, tb, a, st);
+      else return -3;
+    case EPI_SYM_NS_COMBINE:
+      if constexpr (!A_MN && !B_MN) return launch_pair<false, false, EPI_SYM_NS_COMBINE>(ta, tb, a, st);
       else return -3;
   }
   return -2;
@@ -1029,7 +1068,8 @@ extern "C" int arb_gemm_bf16_ragged(const void* A, const void* B, void* C, const
   const bool c_f32 = (epi == EPI_ATOMIC_F32 || epi == EPI_STORE_F32);
   if (ldc % (c_f32 ? 4 : 8)) return -4;
   if (aux && (reinterpret_cast<uintptr_t>(aux) & 15)) return -4;
-  if ((epi == EPI_NS_COMBINE || epi == EPI_RELU2_BWD || epi == EPI_ADD_AUX) && !aux) return -5;
+  if (epi_has_aux(epi) && !aux) return -5;
+  const bool sym = epi_is_sym(epi);
   if (g_num_sms == 0) {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1038,6 +1078,13 @@ extern "C" int arb_gemm_bf16_ragged(const void* A, const void* B, void* C, const
   const int BN = (N > 128) ? 256 : 128;
   // 2-CTA tiles (256 x 256) for problems that are large in both output dimensions
   const bool pair = (g_gemm_mode != 1) && (g_gemm_mode == 2 || (M >= 512 && N >= 256));
+  if (sym) {
+    // The caller vouches for a symmetric result.  Mirrored from four tiles a side: 428 M model (1024 a side), optimizer update
+    // 11.12 -> 10.40 ms; at two a side (3 of 4 tiles left, main loops of 8 K blocks) the transposed stores cost more than the
+    // skipped tile: 119.5 M model 2.25 -> 2.39 ms.
+    if (M != N || m_valid || k_valid || (a_mn_major != b_mn_major)) return -3;
+    if (!pair || M <= 768 || (epi == EPI_SYM_NS_COMBINE && a_mn_major)) epi = epi == EPI_SYM_STORE ? EPI_STORE_BF16 : EPI_NS_COMBINE;
+  }
   const int bm_eff = pair ? 256 : BM;
   GemmArgs a;
   a.M = M; a.N = N; a.K = K; a.batch = batch;

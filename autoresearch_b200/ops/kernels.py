@@ -18,7 +18,7 @@ _lib = None
 _gemm_mode = 0       # as set by gemm_set_mode: 0 automatic, 1 always 1-CTA tiles, 2 always 2-CTA tiles
 _err_flag = {}
 
-EPI_STORE_BF16, EPI_RELU2, EPI_ATOMIC_F32, EPI_NS_COMBINE, EPI_RELU2_BWD, EPI_STORE_F32, EPI_ADD_AUX, EPI_QKV_POST = range(8)
+EPI_STORE_BF16, EPI_RELU2, EPI_ATOMIC_F32, EPI_NS_COMBINE, EPI_RELU2_BWD, EPI_STORE_F32, EPI_ADD_AUX, EPI_QKV_POST, EPI_SYM_STORE, EPI_SYM_NS_COMBINE = range(10)
 ERR_NAMES = {1: "GEMM barrier wait timed out", 2: "attention barrier wait timed out",
              3: "peer barrier wait timed out", 4: "MoE dispatch wait timed out",
              5: "dynamic shared memory base is not 1 KB aligned"}
@@ -180,6 +180,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     tiles beyond are neither computed nor written); ``b_div``: ``b`` holds G / b_div matrices, item g uses matrix
     g // b_div; ``k_valid`` int32 [G, K // k_seg] with ``k_seg`` rows per segment: for EPI_ATOMIC_F32 products over
     rows, only the 64-row blocks below ``k_valid`` of each segment are multiplied.
+
+    ``epi=EPI_SYM_STORE`` / ``EPI_SYM_NS_COMBINE``: the caller vouches that the product is symmetric (X X^T, or the square of a
+    symmetric matrix); tiles below the diagonal are then mirrored instead of computed.
 
     ``epi=EPI_QKV_POST`` with ``post`` = the arguments of :func:`qkv_post_args`: the packed q|k|v projection with
     RoPE + RMS norm of the q / k heads and the value embedding of the v heads done in the epilogue.

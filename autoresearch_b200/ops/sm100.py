@@ -632,10 +632,10 @@ class OptimKernels:
         tall = m > n
         for a, b, c in MA.POLAR_EXPRESS[:ns_steps]:
             if tall:
-                K.gemm(x, x, trans_a=True, trans_b=False, out=A)          # X^T X
+                K.gemm(x, x, trans_a=True, trans_b=False, out=A, epi=K.EPI_SYM_STORE)     # X^T X
             else:
-                K.gemm(x, x, out=A)                                        # X X^T
-            K.gemm(A, A, out=Cm, epi=K.EPI_NS_COMBINE, aux=A, alpha=a, beta=b, gamma=c)
+                K.gemm(x, x, out=A, epi=K.EPI_SYM_STORE)                                   # X X^T
+            K.gemm(A, A, out=Cm, epi=K.EPI_SYM_NS_COMBINE, aux=A, alpha=a, beta=b, gamma=c)
             if tall:
                 K.gemm(x, Cm, out=x2)                                      # X C  (C symmetric)
             else:

@@ -233,3 +233,23 @@ def test_ragged_batches_skip_rows_beyond_the_valid_count(mode):
             assert ((dw[e] - ref).norm() / ref.norm()).item() < 1e-2
     finally:
         K.gemm_set_mode(0)
+
+
+@pytest.mark.parametrize("G,d,k", [(1, 512, 512), (3, 520, 264), (2, 776, 1024), (5, 1024, 128), (1, 2048, 256), (2, 256, 512), (1, 1288, 72)])
+def test_symmetric_products_mirror_their_upper_tiles(G, d, k):
+    """Gram matrices in both layouts and the Newton-Schulz combination, against the same products with every tile computed: each
+    element is the same sum in the same order, so the bits are equal (sizes with one tile, ragged last tiles, many tiles)."""
+    from autoresearch_b200.ops import kernels as K
+    torch.manual_seed(d + k)
+    x = (torch.randn(G, d, k, device="cuda") * 0.1).to(torch.bfloat16)
+    xt = x.transpose(1, 2).contiguous()
+    for a, kw in ((x, {}), (xt, dict(trans_a=True, trans_b=False))):
+        full = K.gemm(a, a, **kw)
+        buf = torch.full((G, d + 2, d), 3.0, device="cuda", dtype=torch.bfloat16)
+        half = buf[:, 1:-1]
+        K.gemm(a, a, out=half, epi=K.EPI_SYM_STORE, **kw)
+        assert torch.equal(full, full.transpose(1, 2)) and torch.equal(half, full)
+        assert (buf[:, 0] == 3.0).all() and (buf[:, -1] == 3.0).all()
+    args = dict(aux=full, alpha=3.4, beta=-4.7, gamma=2.0)
+    assert torch.equal(K.gemm(full, full, epi=K.EPI_NS_COMBINE, **args), K.gemm(full, full, epi=K.EPI_SYM_NS_COMBINE, **args))
+    K.check_err_flag()
