@@ -1075,9 +1075,14 @@ extern "C" int arb_gemm_bf16_ragged(const void* A, const void* B, void* C, const
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  const int BN = (N > 128) ? 256 : 128;
-  // 2-CTA tiles (256 x 256) for problems that are large in both output dimensions
-  const bool pair = (g_gemm_mode != 1) && (g_gemm_mode == 2 || (M >= 512 && N >= 256));
+  // 2-CTA tiles (256 x 256) for problems that are large in both output dimensions, unless so few of them come out that tiles of
+  // 128 x 128 all run at once: a tile's main loop is then a third shorter and up to four times as many SMs work (us, 2-CTA tiles ->
+  // 128 x 128, operands from HBM: 2048 x 512 x 2048 22.5 -> 18.4, 2048 x 512 x 1536 19.3 -> 17.3, 1024 x 1024 x 4096 32.8 -> 28.7,
+  // 1024 x 256 x 256 15.2 -> 13.2; with 256 tiles of 128 x 128, i.e. two waves, 2048 x 2048 x 512 gains nothing).
+  const long long tiles128 = (long long)batch * ((M + 127) / 128) * ((N + 127) / 128);
+  const bool few = g_gemm_mode == 0 && tiles128 <= 148 && epi != EPI_ATOMIC_F32 && epi != EPI_QKV_POST;
+  const int BN = (N > 128 && !few) ? 256 : 128;
+  const bool pair = (g_gemm_mode != 1) && (g_gemm_mode == 2 || (M >= 512 && N >= 256 && !few));
   if (sym) {
     // The caller vouches for a symmetric result.  Mirrored from four tiles a side: 428 M model (1024 a side), optimizer update
     // 11.12 -> 10.40 ms; at two a side (3 of 4 tiles left, main loops of 8 K blocks) the transposed stores cost more than the

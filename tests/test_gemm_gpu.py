@@ -253,3 +253,21 @@ def test_symmetric_products_mirror_their_upper_tiles(G, d, k):
     args = dict(aux=full, alpha=3.4, beta=-4.7, gamma=2.0)
     assert torch.equal(K.gemm(full, full, epi=K.EPI_NS_COMBINE, **args), K.gemm(full, full, epi=K.EPI_SYM_NS_COMBINE, **args))
     K.check_err_flag()
+
+
+@pytest.mark.parametrize("M,N,Kd", [(512, 256, 64), (2048, 512, 1536), (1544, 1416, 200), (512, 4736, 128), (640, 3840, 72)])
+def test_few_tiles_and_just_too_many(M, N, Kd):
+    """Products around the 148 tiles of 128 x 128 where the tile choice changes (148 and 150 tiles in the last two), with every
+    bf16 epilogue that both kernels have: bf16 outputs of K products, 1e-2."""
+    from autoresearch_b200.ops import kernels as K
+    torch.manual_seed(M + N)
+    a, w = torch.randn(M, Kd, device="cuda").bfloat16(), (torch.randn(N, Kd, device="cuda") / Kd ** 0.5).bfloat16()
+    x = torch.rand(M, N, device="cuda").bfloat16()
+    acc = a.float() @ w.float().t()
+    for epi, ref in ((K.EPI_STORE_BF16, acc), (K.EPI_RELU2, acc.clamp_min(0) ** 2), (K.EPI_ADD_AUX, acc + x.float()),
+                     (K.EPI_RELU2_BWD, acc * 2 * x.float().sqrt())):
+        out = K.gemm(a, w, epi=epi, aux=x if epi in (K.EPI_ADD_AUX, K.EPI_RELU2_BWD) else None)
+        assert ((out.float() - ref).norm() / ref.norm()).item() < 1e-2
+    out = K.gemm(a, w.t().contiguous(), trans_b=False)
+    assert ((out.float() - acc).norm() / acc.norm()).item() < 1e-2
+    K.check_err_flag()
