@@ -69,6 +69,9 @@ int arb_gemm_bf16_ragged(const void* A, const void* B, void* C, const void* aux,
                          float gamma, int* err_flag, cudaStream_t stream, const void* pull_src, long long pull_bytes,
                          const void* ahead_src, void* ahead_dst, long long ahead_bytes, const int* m_valid, int b_div,
                          const int* k_valid, int k_seg_rows);
+// n <= 4 weight gradients c[g] (fp32 [M, N], dense) += dy[g]^T x[g] with dy[g] [K, M] and x[g] [K, N] bf16 dense, one launch.
+int arb_gemm_dw_group(const void* const* dy, const void* const* x, float* const* c, const int* M, const int* N, int n, int K,
+                      int* err_flag, cudaStream_t stream);
 // Parameters of the next EPI_QKV_POST product on this host thread (consumed by it).  The product is
 // [rows, D] x [3 * H * 128, D]^T; column blocks of 128 are heads: H query heads, H key heads, H value heads.
 // Query and key heads are rotated (cos / sin: bf16 [T, 64], position = row % T; lo' = lo c + hi s, hi' = hi c - lo s)
@@ -257,7 +260,7 @@ typedef struct {
   void *work, *d_x, *d_x0;
   const void* d_x0_acc;
   void *g_lam_r, *g_lam_0, *g_wqkv, *g_wo, *g_wfc, *g_wdn, *g_gate;
-  long long B, T, H, M, window, idx, gate_ch, fuse_post;
+  long long B, T, H, M, window, idx, gate_ch, fuse_post, group_dw;
   double eps, scale;
 } ArbLayer;
 int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s);

@@ -872,6 +872,166 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------
+// Several weight gradients C_g += A_g^T B_g (fp32, all over the same K rows) in one launch of 2-CTA tiles.  The four of a small
+// layer have 1 to 16 tiles each and K loops of a few us: one after the other they leave most SMs idle and pay four starts (training
+// pass of the 119.5 M model on 1 x 2048 tokens 6.24 -> 5.51 ms in one launch).  Work items are (problem, K split, tile); the roles are those of gemm_pair_kernel without ragged batches and copies.
+constexpr int DW_MAX = 4;
+struct DwMaps { CUtensorMap a[DW_MAX], b[DW_MAX], c[DW_MAX]; };
+struct DwArgs {
+  int n, first[DW_MAX + 1];                    // items [first[g], first[g + 1]) belong to problem g
+  int M[DW_MAX], N[DW_MAX], m_tiles[DW_MAX], n_tiles[DW_MAX];
+  int kb_total, kb_per_split, splitk;
+  int* err;
+};
+struct DwItem { int g, mt, nt, kb0, kb1; };
+__device__ __forceinline__ DwItem dw_item(const DwArgs& p, int w) {
+  DwItem t;
+  t.g = 0;
+  while (t.g + 1 < p.n && w >= p.first[t.g + 1]) ++t.g;
+  w -= p.first[t.g];
+  t.nt = w % p.n_tiles[t.g]; w /= p.n_tiles[t.g];
+  t.mt = w % p.m_tiles[t.g]; w /= p.m_tiles[t.g];
+  t.kb0 = w * p.kb_per_split;
+  t.kb1 = min(p.kb_total, t.kb0 + p.kb_per_split);
+  return t;
+}
+
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_dw_group_kernel(const __grid_constant__ DwMaps maps, const __grid_constant__ DwArgs p) {
+  using L = Smem2<EPI_ATOMIC_F32>;
+  constexpr int STAGES = L::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);   // used in the leader only (count 1)
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* tfull_bar = empty_bar + STAGES;
+  uint64_t* tempty_bar = tfull_bar + 2;                                      // used in the leader only (count 8)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const bool leader = rank == 0;
+  const int cluster_id = blockIdx.x >> 1;
+  const int n_clusters = gridDim.x >> 1;
+  const int items = p.first[p.n];
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 8); }
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
+  tc_fence_before();
+  cluster_sync_all();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_enter();                 // global memory is not touched above
+
+  if (warp == 0) {
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int w = cluster_id; w < items && ok; w += n_clusters) {
+        const DwItem t = dw_item(p, w);
+        const int m0 = t.mt * 256 + int(rank) * 128, n0 = t.nt * 256 + int(rank) * 128;
+        for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          uint8_t* sa = smem + s * L::STAGE_BYTES;
+          uint8_t* sb = sa + L::A_BYTES;
+          const uint32_t lead_bar = mapa_u32(smem_u32(&full_bar[s]), 0);
+          if (leader) mbar_expect_tx(&full_bar[s], 2 * L::STAGE_BYTES);       // both CTAs' bytes, as in gemm_pair_kernel
+#pragma unroll
+          for (int c = 0; c < 2; ++c) tma_load_3d_pair(sa + c * 8192, &maps.a[t.g], lead_bar, m0 + c * 64, kb * BK, 0);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) tma_load_3d_pair(sb + c * 8192, &maps.b[t.g], lead_bar, n0 + c * 64, kb * BK, 0);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && leader) {
+      constexpr uint32_t idesc = make_idesc_bf16(256, 256, true, true);
+      uint32_t it = 0, tile_it = 0;
+      bool ok = true;
+      for (int w = cluster_id; w < items && ok; w += n_clusters, ++tile_it) {
+        const DwItem t = dw_item(p, w);
+        const int acc = tile_it & 1;
+        if (!mbar_wait(&tempty_bar[acc], ((tile_it >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * 256;
+        for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait(&full_bar[s], (it / STAGES) & 1, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
+          const uint32_t sb = sa + L::A_BYTES;
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            tc_mma_ss_pair(d_tmem, make_smem_desc(sa + k * 2048, 8192, 1024), make_smem_desc(sb + k * 2048, 8192, 1024), idesc,
+                           (kb > t.kb0 || k > 0) ? 1u : 0u);
+          const uint32_t eb = smem_u32(&empty_bar[s]);
+          tc_commit_pair(eb);
+          tc_commit_pair(mapa_u32(eb, 1));
+        }
+        if (ok) {
+          const uint32_t tb = smem_u32(&tfull_bar[acc]);
+          tc_commit_pair(tb);
+          tc_commit_pair(mapa_u32(tb, 1));
+        }
+      }
+    }
+  } else if (warp < 6) {
+    const int q = warp & 3;
+    const bool t0 = (threadIdx.x == 64);
+    const int r_local = q * 32 + lane;
+    uint32_t tile_it = 0, slab_it = 0;
+    bool ok = true;
+    for (int w = cluster_id; w < items; w += n_clusters, ++tile_it) {
+      const DwItem t = dw_item(p, w);
+      const int acc = tile_it & 1;
+      // after a time-out keep walking the loop (named barriers below need all four warps) but skip waits
+      if (ok && !mbar_wait(&tfull_bar[acc], (tile_it >> 1) & 1, abort_flag)) ok = false;
+      tc_fence_after();
+      const int row0 = t.mt * 256 + int(rank) * 128;
+#pragma unroll 1
+      for (int sl = 0; sl < 8; ++sl, ++slab_it) {          // eight slabs of 128 rows x 32 columns, as TMA reduce-adds
+        const int col_s = t.nt * 256 + sl * 32;
+        uint8_t* buf = smem + L::C_STAGE + (slab_it & 1) * 16384;
+        if (t0) tma_store_wait_read_1();
+        named_barrier(2, 128);
+        uint32_t v[32];
+        tmem_ld32(tmem_base + (uint32_t(q * 32) << 16) + uint32_t(acc * 256 + sl * 32), v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          st_sw128(smem_u32(buf), 128, r_local, j * 2, make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+        fence_proxy_async_smem();
+        named_barrier(3, 128);
+        if (t0) {
+          if (ok && col_s < p.N[t.g] && row0 < p.M[t.g]) tma_reduce_add_3d(&maps.c[t.g], buf, col_s, row0, 0);
+          tma_store_commit();
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (leader) mbar_arrive(&tempty_bar[acc]);
+        else mbar_arrive_remote(mapa_u32(smem_u32(&tempty_bar[acc]), 0));
+      }
+    }
+    if (t0) tma_store_wait_all();
+  }
+
+  tc_fence_before();
+  cluster_sync_all();
+  if (threadIdx.x == 0 && *abort_flag && p.err) atomicExch(p.err, ERR_GEMM_TIMEOUT);
+  if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc_pair(tmem_base, 512); }
+}
+
+// ------------------------------------------------------------------------------------------
 static int g_num_sms = 0;
 // Counters of the prologue pull: a ring per device, one slot per pulling launch (round-robin), each slot with a
 // running target, so that pulling GEMMs in flight on different streams never share a counter.
@@ -899,6 +1059,21 @@ static int arm_pull(GemmArgs& a, int grid_ctas) {
 }
 static int g_gemm_mode = 0;   // 0 = automatic, 1 = always 1-CTA tiles, 2 = always 2-CTA tiles
 
+// The split of the K loop that fills the last wave of `units` CTAs (or pairs) best, with at least 8 K blocks per split
+static int pick_split(int tiles, int kb_total, int units) {
+  int max_split = kb_total / 8 > 0 ? kb_total / 8 : 1;
+  if (max_split > 32) max_split = 32;
+  int split = 1;
+  double best = 0.0;
+  for (int sp = 1; sp <= max_split; ++sp) {
+    const long long it = (long long)tiles * sp;
+    const long long waves = (it + units - 1) / units;
+    const double eff = double(it) / double(waves * units);
+    if (eff > best + 0.02) { best = eff; split = sp; }
+  }
+  return split;
+}
+
 template <bool A_MN, bool B_MN, int EPI, int BN>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& a, cudaStream_t st) {
   using L = SmemLayout<BN>;
@@ -913,6 +1088,21 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
   GemmArgs args = a;
   if (int r = arm_pull(args, grid)) return r;
   return launch_dependent(true, kern, grid, GEMM_THREADS, L::TOTAL, st, ta, tb, args);
+}
+
+static void pair_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int clusters, int smem, cudaStream_t st) {
+  cfg.gridDim = dim3(unsigned(clusters * 2));
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = size_t(smem);
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // as launch_dependent()
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
 }
 
 template <bool A_MN, bool B_MN, int EPI>
@@ -943,19 +1133,8 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
   int clusters = g_num_sms / 2;
   if (items < clusters) clusters = items;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned(clusters * 2));
-  cfg.blockDim = dim3(GEMM_THREADS);
-  cfg.dynamicSmemBytes = Smem2<EPI>::TOTAL;
-  cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // as launch_dependent()
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  pair_launch_config(cfg, attr, clusters, Smem2<EPI>::TOTAL, st);
   GemmArgs args = a;
   if (int r = arm_pull(args, clusters * 2)) return r;
   return int(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tx, args));
@@ -1021,6 +1200,54 @@ extern "C" int arb_gemm_qkv_post_args(const void* cos_t, const void* sin_t, floa
   q.gate_w = (const __nv_bfloat16*)gate_w; q.gate = gate_out; q.gate_ch = gate_ch; q.eps = eps;
   g_qkv_post_set = true;
   return 0;
+}
+
+extern "C" int arb_gemm_dw_group(const void* const* dy, const void* const* x, float* const* c, const int* M, const int* N, int n, int K,
+                                 int* err_flag, cudaStream_t stream) {
+  if (n < 1 || n > DW_MAX || K <= 0) return -3;
+  if (g_num_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  static PerDeviceOnce configured;
+  DwMaps maps;
+  DwArgs a;
+  std::memset(&maps, 0, sizeof maps);
+  std::memset(&a, 0, sizeof a);
+  int tiles = 0;
+  for (int g = 0; g < n; ++g) {
+    if (M[g] <= 0 || N[g] <= 0 || (M[g] % 8) || (N[g] % 8)) return -4;
+    if ((reinterpret_cast<uintptr_t>(dy[g]) | reinterpret_cast<uintptr_t>(x[g]) | reinterpret_cast<uintptr_t>(c[g])) & 15) return -4;
+    a.M[g] = M[g]; a.N[g] = N[g];
+    a.m_tiles[g] = (M[g] + 255) / 256; a.n_tiles[g] = (N[g] + 255) / 256;
+    tiles += a.m_tiles[g] * a.n_tiles[g];
+    const uint32_t in_box[3] = {64, BK, 1}, out_box[3] = {32, 128, 1};
+    uint64_t da[3] = {uint64_t(M[g]), uint64_t(K), 1}, db[3] = {uint64_t(N[g]), uint64_t(K), 1}, dc[3] = {uint64_t(N[g]), uint64_t(M[g]), 1};
+    uint64_t sa[2] = {uint64_t(M[g]) * 2, uint64_t(M[g]) * 2 * K}, sb[2] = {uint64_t(N[g]) * 2, uint64_t(N[g]) * 2 * K};
+    uint64_t sc[2] = {uint64_t(N[g]) * 4, uint64_t(N[g]) * 4 * M[g]};
+    int r = make_tmap_bf16(&maps.a[g], dy[g], 3, da, sa, in_box);
+    if (r) return 1000 + r;
+    if ((r = make_tmap_bf16(&maps.b[g], x[g], 3, db, sb, in_box))) return 2000 + r;
+    if ((r = make_tmap_typed(&maps.c[g], c[g], 3, dc, sc, out_box, CU_TENSOR_MAP_DATA_TYPE_FLOAT32))) return 3000 + r;
+  }
+  a.n = n;
+  a.err = err_flag;
+  a.kb_total = (K + BK - 1) / BK;
+  const int split = pick_split(tiles, a.kb_total, g_num_sms / 2);
+  a.kb_per_split = (a.kb_total + split - 1) / split;
+  a.splitk = (a.kb_total + a.kb_per_split - 1) / a.kb_per_split;
+  for (int g = 0; g < n; ++g) a.first[g + 1] = a.first[g] + a.m_tiles[g] * a.n_tiles[g] * a.splitk;
+  constexpr int SMEM = Smem2<EPI_ATOMIC_F32>::TOTAL;
+  if (configured.first()) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_dw_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return int(e);
+  }
+  const int clusters = a.first[n] < g_num_sms / 2 ? a.first[n] : g_num_sms / 2;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  pair_launch_config(cfg, attr, clusters, SMEM, stream);
+  return int(cudaLaunchKernelEx(&cfg, gemm_dw_group_kernel, maps, a));
 }
 
 extern "C" int arb_gemm_set_mode(int mode) {
@@ -1097,21 +1324,8 @@ extern "C" int arb_gemm_bf16_ragged(const void* A, const void* B, void* C, const
   a.n_tiles = pair ? (N + 255) / 256 : (N + BN - 1) / BN;
   a.kb_total = (K + BK - 1) / BK;
   if (epi != EPI_ATOMIC_F32) splitk = 1;
-  if (splitk <= 0) {  // automatic: fill the SMs when there are few output tiles
-    const int tiles = batch * a.m_tiles * a.n_tiles;
-    const int units = pair ? g_num_sms / 2 : g_num_sms;     // CTAs, or CTA pairs, that can run at once
-    int max_split = a.kb_total / 8 > 0 ? a.kb_total / 8 : 1;        // at least 8 K blocks per split
-    if (max_split > 32) max_split = 32;
-    // pick the split that fills the last wave best: efficiency = items / (waves * units)
-    splitk = 1;
-    double best = 0.0;
-    for (int sp = 1; sp <= max_split; ++sp) {
-      const long long it = (long long)tiles * sp;
-      const long long waves = (it + units - 1) / units;
-      const double eff = double(it) / double(waves * units);
-      if (eff > best + 0.02) { best = eff; splitk = sp; }
-    }
-  }
+  if (splitk <= 0)  // automatic: fill the SMs when there are few output tiles
+    splitk = pick_split(batch * a.m_tiles * a.n_tiles, a.kb_total, pair ? g_num_sms / 2 : g_num_sms);
   if (splitk > a.kb_total) splitk = a.kb_total;
   a.kb_per_split = (a.kb_total + splitk - 1) / splitk;
   a.splitk = (a.kb_total + a.kb_per_split - 1) / a.kb_per_split;

@@ -81,7 +81,8 @@ extern "C" int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s
   return 0;
 }
 
-// a.work: bf16 [N, max(M, 4 D) + 2 D], then d_xn_gate [N, gate_ch], then (16-byte aligned, as is dgl) fp32 delta and dgl
+// a.group_dw: the four weight gradients leave in one launch at the end; d_h then has a place of its own.
+// a.work: bf16 [N, max(M, 4 D) + 2 D] (with group_dw [N, M + 4 D + 2 D], the value rows' gradients behind M + 3 D), then d_xn_gate [N, gate_ch], then (16-byte aligned, as is dgl) fp32 delta and dgl
 // [N, H] each.
 // On return the value embedding's row gradients [N, D] lie behind the first 3 N D elements.
 extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s) {
@@ -94,31 +95,40 @@ extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s
   const int* ids = static_cast<const int*>(a.ids);
   const int H = int(a.H), T = int(a.T), ch = int(a.gate_ch);
   auto* w = static_cast<char*>(a.work);
-  const long long wide = a.M > 4 * D ? a.M : 4 * D;
-  char *dh = w, *dqkv = w, *dve = w + N * 3 * D * 2;          // d_h is dead when the attention backward writes d_qkv
+  const long long wide = a.group_dw ? a.M + 4 * D : a.M > 4 * D ? a.M : 4 * D;
+  char *dh = w, *dqkv = w + (a.group_dw ? N * a.M * 2 : 0);   // else d_h is dead when the attention backward writes d_qkv
+  char* dve = dqkv + N * 3 * D * 2;
   char *t1 = w + N * wide * 2, *g2 = t1 + N * D * 2;          // t1: d_xn2, then d_att, then d_xn
   char* dxg = g2 + N * D * 2;
   float *delta = reinterpret_cast<float*>(dxg + (N * ch * 2 + 15) / 16 * 16), *dgl = delta + (N * H + 3) / 4 * 4;
   int n = 0;
   // MLP: out = xs2 + relu(xn2 wfc^T)^2 wdn^T
   ARB_TRY(g.nn(a.g, a.wdn, dh, k.act, N, a.M, D, EPI_RELU2_BWD));
-  ARB_TRY(g.dw(a.g, k.act, a.g_wdn, D, a.M, N));
-  ARB_TRY(g.dw(dh, k.xn2, a.g_wfc, a.M, D, N));
+  if (!a.group_dw) {
+    ARB_TRY(g.dw(a.g, k.act, a.g_wdn, D, a.M, N));
+    ARB_TRY(g.dw(dh, k.xn2, a.g_wfc, a.M, D, N));
+  }
   ARB_TRY(g.nn(dh, a.wfc, t1, nullptr, N, D, a.M, EPI_STORE_BF16));
   ARB_TRY(arb_rmsnorm_bwd(k.xs2, t1, a.g, g2, N, int(D), eps, s));
   // attention: xs2 = xs + att wo^T
   ARB_TRY(g.nn(g2, a.wo, t1, nullptr, N, D, D, EPI_STORE_BF16));
-  ARB_TRY(g.dw(g2, k.att, a.g_wo, D, D, N));
+  if (!a.group_dw) ARB_TRY(g.dw(g2, k.att, a.g_wo, D, D, N));
   ARB_TRY(arb_attn_bwd(k.qkv, k.qkv + 2 * D, k.qkv + 4 * D, k.att, t1, k.lse, dqkv, dqkv + 2 * D, dqkv + 4 * D, delta, nullptr, int(a.B),
                        T, H, 3 * D, 3 * D, 3 * D, D, D, 3 * D, 3 * D, 3 * D, int(a.window), float(a.scale), g.err, s));
   ARB_TRY(arb_qkv_post_bwd(dqkv, k.qkv, a.cos_t, a.sin_t, k.rstd, k.xn, ids, a.ve, a.ve ? a.gate_w : nullptr, a.ve ? k.gate : nullptr,
                            a.ve ? dve : nullptr, a.ve ? static_cast<float*>(a.g_gate) : nullptr, a.ve ? dxg : nullptr,
                            a.ve ? dgl : nullptr, N, T, H, int(D), ch, s));
-  ARB_TRY(g.dw(dqkv, k.xn, a.g_wqkv, 3 * D, D, N));
+  if (!a.group_dw) ARB_TRY(g.dw(dqkv, k.xn, a.g_wqkv, 3 * D, D, N));
   ARB_TRY(g.nn(dqkv, a.wqkv, t1, nullptr, N, D, 3 * D, EPI_STORE_BF16));
   if (a.ve) ARB_TRY(arb_add_cols(t1, D, dxg, N, ch, s));
   ARB_TRY(arb_resid_scale_norm_bwd(a.x, a.x0, a.lam_r, a.lam_0, int(a.idx), g2, t1, a.d_x, a.d_x0, a.d_x0_acc,
                                    static_cast<float*>(a.g_lam_r), static_cast<float*>(a.g_lam_0), N, int(D), eps, s));
+  if (a.group_dw) {
+    const void *dy[4] = {dqkv, dh, a.g, g2}, *x[4] = {k.xn, k.xn2, k.act, k.att};
+    float* c[4] = {static_cast<float*>(a.g_wqkv), static_cast<float*>(a.g_wfc), static_cast<float*>(a.g_wdn), static_cast<float*>(a.g_wo)};
+    const int d = int(D), f = int(a.M), rows[4] = {3 * d, f, d, d}, cols[4] = {d, d, f, d};
+    ARB_TRY(arb_gemm_dw_group(dy, x, c, rows, cols, 4, int(N), g.err, s));
+  }
   *launches = n;
   return 0;
 }

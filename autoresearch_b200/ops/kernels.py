@@ -110,6 +110,7 @@ def _signatures() -> dict:
         "arb_moe_finish_dispatch": [vp, vp, vp, i32, i32, i32, i32, i32, vp],
         "arb_moe_combine_fwd": [vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, vp],
         "arb_moe_combine_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, vp],
+        "arb_gemm_dw_group": [vp, vp, vp, vp, vp, i32, i32, vp, vp],
         "arb_layer_fwd": [vp, vp, vp],
         "arb_layer_bwd": [vp, vp, vp],
     }
@@ -304,7 +305,7 @@ def flush_pending_pulls() -> None:
     _check(lib().arb_pull_ranges(src, dst, nb, n, _stream()), "pull_ranges")
 
 
-_LAYER = struct.Struct("=36q2d")        # ArbLayer of csrc/api.h: 28 pointers, 8 sizes, eps and scale
+_LAYER = struct.Struct("=37q2d")        # ArbLayer of csrc/api.h: 28 pointers, 9 sizes, eps and scale
 
 
 def layer_call(entry: str, pointers, sizes, eps: float, scale: float) -> None:

@@ -400,6 +400,11 @@ class AttentionFn(torch.autograd.Function):
         return d_qkv, None, None, None, None
 
 
+# Layers whose four weight gradients together are at most this many operations (46 us at 1.3 PFLOP/s) compute them in one launch at
+# the end of the backward call; above, each of them fills the GPU by itself and d_h need not be kept for it.
+GROUP_DW_FLOPS = 6e10
+
+
 class DenseLayerFn(torch.autograd.Function):
     """A whole dense layer, launched by one native call per direction (csrc/layer.cu): the kernels, their order and their
     arguments are those of ResidScaleNormFn, AttnPreFn, AttentionFn, LinearAddNormFn and MLPFn in a row.  What the layer
@@ -412,7 +417,8 @@ class DenseLayerFn(torch.autograd.Function):
         stat = (N * H + 3) // 4 * 8                            # fp32 [N, H] in bf16 elements; lse, rstd of q and k, gate
         kept = torch.empty(N * (8 * D + M) + 4 * stat, dtype=torch.bfloat16, device=x.device)
         out = torch.empty_like(x)
-        sizes = (B, T, H, M, window, idx, gate_ch, int(K.qkv_post_fusable(N, 3 * D)))
+        group = int(2 * N * D * (4 * D + 2 * M) <= GROUP_DW_FLOPS)
+        sizes = (B, T, H, M, window, idx, gate_ch, int(K.qkv_post_fusable(N, 3 * D)), group)
         ptrs = [t.data_ptr() for t in (x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn)]
         ptrs += (ve.data_ptr(), gate_w.data_ptr()) if ve is not None else (0, 0)
         ptrs += (ids.data_ptr(), cos.data_ptr(), sin.data_ptr(), kept.data_ptr(), out.data_ptr(), K.err_flag(x.device).data_ptr())
@@ -424,7 +430,7 @@ class DenseLayerFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept = ctx.saved_tensors
-        B, T, H, M, _, idx, gate_ch, _ = ctx.sizes
+        B, T, H, M, _, idx, gate_ch, _, group = ctx.sizes
         chain = ctx.chain
         N, D = x.shape
         dev = x.device
@@ -434,7 +440,7 @@ class DenseLayerFn(torch.autograd.Function):
         params = (lam_r, lam_0, wqkv, wo, wfc, wdn) + ((gate_w,) if ve is not None else ())
         mains = [_main_grad(p) for p in params]
         accs = [m if m is not None else torch.zeros(p.shape, dtype=torch.float32, device=dev) for m, p in zip(mains, params)]
-        wide = max(M, 4 * D)
+        wide = M + 4 * D if group else max(M, 4 * D)
         work = torch.empty(N * (wide + 2 * D + gate_ch) + 8 + 2 * ((N * H + 3) // 4 * 8), dtype=torch.bfloat16, device=dev)
         dx = torch.empty_like(x)
         acc0 = chain.buf
@@ -447,7 +453,8 @@ class DenseLayerFn(torch.autograd.Function):
         K.layer_call("arb_layer_bwd", ptrs, ctx.sizes, ctx.eps, 1.0 / math.sqrt(128.0))
         g_ve = None
         if ve is not None:
-            d_ve = work[3 * N * D:4 * N * D].view(N, D)
+            lo = N * (3 * D + (M if group else 0))
+            d_ve = work[lo:lo + N * D].view(N, D)
             mgv = _main_grad(ve)
             acc = mgv if mgv is not None else torch.zeros(ve.shape, dtype=torch.float32, device=dev)
             K.embedding_bwd(ids, d_ve, acc)

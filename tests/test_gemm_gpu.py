@@ -271,3 +271,28 @@ def test_few_tiles_and_just_too_many(M, N, Kd):
     out = K.gemm(a, w.t().contiguous(), trans_b=False)
     assert ((out.float() - acc).norm() / acc.norm()).item() < 1e-2
     K.check_err_flag()
+
+
+@pytest.mark.parametrize("Kd,shapes", [(1, [(8, 8)]), (130, [(256, 256), (264, 512)]), (2048, [(1536, 512), (2048, 512), (512, 2048), (512, 512)]),
+                                       (993, [(1152, 384), (1536, 384), (384, 1536), (384, 384)]), (8000, [(128, 128), (384, 128), (512, 128)])])
+def test_grouped_weight_gradients(Kd, shapes):
+    """One launch against 64 bits: one row, ragged tiles and K, splits that do and do not divide the K blocks; fp32 sums of Kd
+    products of bf16 values, and rows around the outputs that stay untouched."""
+    import ctypes as C
+    from autoresearch_b200.ops import kernels as K
+    torch.manual_seed(Kd)
+    dy = [torch.randn(Kd, m, device="cuda").bfloat16() for m, _ in shapes]
+    x = [torch.randn(Kd, n, device="cuda").bfloat16() for _, n in shapes]
+    buf = [torch.full((m + 2, n), 0.25, device="cuda") for m, n in shapes]
+    out = [b[1:-1] for b in buf]
+    n = len(shapes)
+    vec = lambda ts: (C.c_void_p * n)(*[t.data_ptr() for t in ts])
+    ints = lambda v: (C.c_int * n)(*v)
+    K._check(K.lib().arb_gemm_dw_group(vec(dy), vec(x), vec(out), ints([m for m, _ in shapes]), ints([c for _, c in shapes]), n, Kd,
+                                       K.err_flag().data_ptr(), K._stream()), "gemm_dw_group")
+    torch.cuda.synchronize()
+    K.check_err_flag()
+    for a, b, c, full in zip(dy, x, out, buf):
+        ref = 0.25 + a.double().t() @ b.double()
+        assert (c.double() - ref).abs().max() <= 2e-6 * (a.double().abs().t() @ b.double().abs()).max() + 1e-6
+        assert (full[0] == 0.25).all() and (full[-1] == 0.25).all()
