@@ -410,13 +410,14 @@ def _embedding_plan(ids, vocab: int):
     slot = ("plan", ids.device.index)
     key = (ids.data_ptr(), ids._version, ids.numel(), ids.dtype, vocab, _stream())
     hit = _emb_plan.get(slot)
-    if hit is not None and hit[0] == key:
+    # a graph that is being captured holds its own plan kernels: the ids are other ones when it is replayed
+    if hit is not None and hit[0] == key and not torch.cuda.is_current_stream_capturing():
         return hit[1]
     R = EMB_BWD_ROWS_PER_ITEM
     N = ids.numel()
     n_max = N // R + vocab + 1                                                     # upper bound of the item count
-    if vocab <= EMB_PLAN_MAX_VOCAB and ids.dtype is torch.int32 and ids.is_contiguous():
-        n_chunks = (N + 1023) // 1024
+    n_chunks = (N + 1023) // 1024
+    if vocab <= EMB_PLAN_MAX_VOCAB and n_chunks * vocab <= 1 << 25 and ids.dtype is torch.int32 and ids.is_contiguous():
         perm = torch.empty(N, dtype=torch.int64, device=ids.device)
         counts, seg_start, item_start, item_id, hist = torch.empty(
             3 * vocab + n_max + n_chunks * vocab, dtype=torch.int32, device=ids.device).split(

@@ -106,3 +106,43 @@ def test_whole_layer_calls_give_the_bits_of_the_separate_steps(batch, seq, layer
             else:
                 # fp32 split-K sums meet in L2 in any order: a few units in the last place of the largest partial sum
                 assert (x.float() - y.float()).norm() <= (1e-5 if with_main else 4e-3) * y.float().norm(), n
+
+
+def test_captured_pass_follows_its_inputs():
+    """A training pass (forward, backward into main gradients) captured in a CUDA graph, with its early-started kernels, and
+    replayed on other tokens, against the same pass run directly: losses bit for bit, gradients up to the order of split-K sums."""
+    from autoresearch_b200.config import model_preset
+    from autoresearch_b200.ops import kernels as K
+    cfg = model_preset("small")
+    torch.manual_seed(5)
+    mod = _build("sm100", cfg, torch.bfloat16)
+    for p in mod.parameters():
+        p.main_grad = torch.zeros(p.shape, dtype=torch.float32, device="cuda")
+    batches = [torch.randint(0, cfg.vocab, (2, 2, 200), device="cuda", dtype=torch.int32) for _ in range(3)]
+    ids, tgt = batches[0][0].clone(), batches[0][1].clone()
+
+    def step():
+        for p in mod.parameters():
+            p.main_grad.zero_()
+        loss, per_tok = mod(ids, tgt, grad_scale=1.0 / ids.numel())
+        loss.backward()
+        return per_tok
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(2):
+            step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step()
+    for b in batches[1:]:
+        ids.copy_(b[0]); tgt.copy_(b[1])
+        graph.replay()
+        got = out.clone(), [p.main_grad.clone() for p in mod.parameters()]
+        want = step()
+        assert torch.equal(got[0], want)
+        for p, g in zip(mod.parameters(), got[1]):
+            assert (p.main_grad - g).norm() <= 1e-3 * p.main_grad.norm() + 1e-9
+    K.check_err_flag()
