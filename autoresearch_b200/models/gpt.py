@@ -108,23 +108,27 @@ class GPT(nn.Module):
         cfg, be = self.cfg, self.backend
         ids_flat = ids.reshape(-1)
         aux_total = None
-        whole_layer = getattr(be, "dense_layer", None)
+        whole_layer, first_half = getattr(be, "dense_layer", None), getattr(be, "attention_half", None)
         for bi, blk in enumerate(self.blocks):
             l = blk.layer
             if self.grad_bucket_cb is not None and l in self.grad_bucket_boundaries and x.requires_grad:
                 cb, b = self.grad_bucket_cb, self.grad_bucket_boundaries[l]
                 x.register_hook(lambda g, cb=cb, b=b: cb(b))
             with nvtx_range(f"layer {l}"):
-                if whole_layer is not None:
-                    y = whole_layer(x, x0, self.resid_lambdas, self.x0_lambdas, bi, blk, ids_flat, B, T, cfg, self.rope_cos,
-                                    self.rope_sin, cfg.window(l))
-                    if y is not None:
+                one_call = whole_layer if blk.router is None else first_half
+                if one_call is not None:
+                    y = one_call(x, x0, self.resid_lambdas, self.x0_lambdas, bi, blk, ids_flat, B, T, cfg, self.rope_cos,
+                                 self.rope_sin, cfg.window(l))
+                    if y is not None and blk.router is None:
                         x = y
                         continue
-                x, xn = be.resid_scale_norm(x, x0, self.resid_lambdas, self.x0_lambdas, bi)
-                a = be.attention_block(xn, blk, ids_flat, B, T, cfg, self.rope_cos, self.rope_sin,
-                                       cfg.window(l))
-                x, xn = be.proj_add_norm(a, blk.wo, x)
+                if one_call is not None and y is not None:
+                    x, xn = y
+                else:
+                    x, xn = be.resid_scale_norm(x, x0, self.resid_lambdas, self.x0_lambdas, bi)
+                    a = be.attention_block(xn, blk, ids_flat, B, T, cfg, self.rope_cos, self.rope_sin,
+                                           cfg.window(l))
+                    x, xn = be.proj_add_norm(a, blk.wo, x)
                 if blk.router is not None:
                     x, aux = be.moe_mlp_add(xn, x, blk, cfg.moe)
                     aux_total = aux if aux_total is None else aux_total + aux

@@ -254,15 +254,17 @@ typedef struct {
   // forward: inputs, parameters, the buffer for what the layer keeps (bf16 [N, 8 D + M] then four times
   // fp32 [N, H], each rounded up to 4 floats), output [N, D]
   const void *x, *x0, *lam_r, *lam_0, *wqkv, *wo, *wfc, *wdn, *ve, *gate_w, *ids, *cos_t, *sin_t;
-  void *kept, *out, *err;
+  void *kept, *out, *out2, *err;
   // backward: incoming gradient [N, D], scratch, input gradients (d_x0_acc as in arb_resid_scale_norm_bwd), fp32 gradients
-  const void* g;
+  const void *g, *g_xn;
   void *work, *d_x, *d_x0;
   const void* d_x0_acc;
   void *g_lam_r, *g_lam_0, *g_wqkv, *g_wo, *g_wfc, *g_wdn, *g_gate;
-  long long B, T, H, M, window, idx, gate_ch, fuse_post, group_dw;
+  long long B, T, H, M, window, idx, gate_ch, fuse_post, group_dw, half;
   double eps, scale;
 } ArbLayer;
+// half: the layer up to its second norm (what comes before the experts of an expert layer): out = the residual stream, out2 = its
+// norm, M = 0, kept without their copies; backward: out as input, g and g_xn their gradients (either may be null, not both).
 int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s);
 int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s);
 

@@ -18,10 +18,11 @@ namespace {
 struct Kept {
   char *xs, *xn, *qkv, *att, *xs2, *xn2, *act;
   float *lse, *rstd, *gate;
-  Kept(void* base, long long N, long long D, long long M, long long H) {
+  Kept(void* base, long long N, long long D, long long M, long long H, bool half) {
     char* p = static_cast<char*>(base);
     auto take = [&](long long cols) { char* q = p; p += N * cols * 2; return q; };
-    xs = take(D); xn = take(D); qkv = take(3 * D); att = take(D); xs2 = take(D); xn2 = take(D); act = take(M);
+    xs = take(D); xn = take(D); qkv = take(3 * D); att = take(D);
+    xs2 = take(half ? 0 : D); xn2 = take(half ? 0 : D); act = take(half ? 0 : M);
     const long long nh = (N * H + 3) / 4 * 4;
     lse = reinterpret_cast<float*>(p); rstd = lse + nh; gate = rstd + 2 * nh;
   }
@@ -44,7 +45,7 @@ struct Gemm {
 };
 
 bool bad_sizes(const ArbLayer& a) {
-  return a.B <= 0 || a.T <= 0 || a.H <= 0 || a.M <= 0 || (a.M & 7) || a.B * a.T > 0x7fffffffll || a.H > 65535 || a.M > 0x7fffffffll;
+  return a.B <= 0 || a.T <= 0 || a.H <= 0 || (a.half ? a.M != 0 : a.M <= 0) || (a.M & 7) || a.B * a.T > 0x7fffffffll || a.H > 65535 || a.M > 0x7fffffffll;
 }
 
 }  // namespace
@@ -53,9 +54,9 @@ bool bad_sizes(const ArbLayer& a) {
 
 extern "C" int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s) {
   const ArbLayer& a = *args;
-  if (bad_sizes(a) || !a.kept || !a.out) return -3;
+  if (bad_sizes(a) || !a.kept || !a.out || (a.half && !a.out2)) return -3;
   const long long N = a.B * a.T, D = a.H * 128;
-  const Kept k(a.kept, N, D, a.M, a.H);
+  const Kept k(a.kept, N, D, a.M, a.H, a.half);
   const Gemm g{static_cast<int*>(a.err), s};
   const float eps = float(a.eps);
   const int* ids = static_cast<const int*>(a.ids);
@@ -73,10 +74,13 @@ extern "C" int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s
   }
   ARB_TRY(arb_attn_fwd(k.qkv, k.qkv + 2 * D, k.qkv + 4 * D, k.att, k.lse, int(a.B), T, H, 3 * D, 3 * D, 3 * D, D, int(a.window),
                        float(a.scale), g.err, s));
-  ARB_TRY(g.nt(k.att, a.wo, k.xs2, k.xs, N, D, D, EPI_ADD_AUX));
-  ARB_TRY(arb_rmsnorm_fwd(k.xs2, k.xn2, N, int(D), eps, s));
-  ARB_TRY(g.nt(k.xn2, a.wfc, k.act, nullptr, N, a.M, D, EPI_RELU2));
-  ARB_TRY(g.nt(k.act, a.wdn, a.out, k.xs2, N, D, a.M, EPI_ADD_AUX));
+  void *xs2 = a.half ? a.out : k.xs2, *xn2 = a.half ? a.out2 : k.xn2;
+  ARB_TRY(g.nt(k.att, a.wo, xs2, k.xs, N, D, D, EPI_ADD_AUX));
+  ARB_TRY(arb_rmsnorm_fwd(xs2, xn2, N, int(D), eps, s));
+  if (!a.half) {
+    ARB_TRY(g.nt(xn2, a.wfc, k.act, nullptr, N, a.M, D, EPI_RELU2));
+    ARB_TRY(g.nt(k.act, a.wdn, a.out, xs2, N, D, a.M, EPI_ADD_AUX));
+  }
   *launches = n;
   return 0;
 }
@@ -87,9 +91,9 @@ extern "C" int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s
 // On return the value embedding's row gradients [N, D] lie behind the first 3 N D elements.
 extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s) {
   const ArbLayer& a = *args;
-  if (bad_sizes(a) || !a.kept || !a.work || !a.g || !a.d_x || !a.d_x0) return -3;
+  if (bad_sizes(a) || !a.kept || !a.work || !a.d_x || !a.d_x0 || (a.half ? !a.out || (!a.g && !a.g_xn) : !a.g)) return -3;
   const long long N = a.B * a.T, D = a.H * 128;
-  const Kept k(a.kept, N, D, a.M, a.H);
+  const Kept k(a.kept, N, D, a.M, a.H, a.half);
   const Gemm g{static_cast<int*>(a.err), s};
   const float eps = float(a.eps);
   const int* ids = static_cast<const int*>(a.ids);
@@ -102,17 +106,23 @@ extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s
   char* dxg = g2 + N * D * 2;
   float *delta = reinterpret_cast<float*>(dxg + (N * ch * 2 + 15) / 16 * 16), *dgl = delta + (N * H + 3) / 4 * 4;
   int n = 0;
-  // MLP: out = xs2 + relu(xn2 wfc^T)^2 wdn^T
-  ARB_TRY(g.nn(a.g, a.wdn, dh, k.act, N, a.M, D, EPI_RELU2_BWD));
-  if (!a.group_dw) {
-    ARB_TRY(g.dw(a.g, k.act, a.g_wdn, D, a.M, N));
-    ARB_TRY(g.dw(dh, k.xn2, a.g_wfc, a.M, D, N));
+  const void* gs = g2;                                        // gradient of xs2
+  if (a.half) {
+    if (a.g_xn) ARB_TRY(arb_rmsnorm_bwd(a.out, a.g_xn, a.g, g2, N, int(D), eps, s));
+    else gs = a.g;
+  } else {
+    // MLP: out = xs2 + relu(xn2 wfc^T)^2 wdn^T
+    ARB_TRY(g.nn(a.g, a.wdn, dh, k.act, N, a.M, D, EPI_RELU2_BWD));
+    if (!a.group_dw) {
+      ARB_TRY(g.dw(a.g, k.act, a.g_wdn, D, a.M, N));
+      ARB_TRY(g.dw(dh, k.xn2, a.g_wfc, a.M, D, N));
+    }
+    ARB_TRY(g.nn(dh, a.wfc, t1, nullptr, N, D, a.M, EPI_STORE_BF16));
+    ARB_TRY(arb_rmsnorm_bwd(k.xs2, t1, a.g, g2, N, int(D), eps, s));
   }
-  ARB_TRY(g.nn(dh, a.wfc, t1, nullptr, N, D, a.M, EPI_STORE_BF16));
-  ARB_TRY(arb_rmsnorm_bwd(k.xs2, t1, a.g, g2, N, int(D), eps, s));
   // attention: xs2 = xs + att wo^T
-  ARB_TRY(g.nn(g2, a.wo, t1, nullptr, N, D, D, EPI_STORE_BF16));
-  if (!a.group_dw) ARB_TRY(g.dw(g2, k.att, a.g_wo, D, D, N));
+  ARB_TRY(g.nn(gs, a.wo, t1, nullptr, N, D, D, EPI_STORE_BF16));
+  if (!a.group_dw) ARB_TRY(g.dw(gs, k.att, a.g_wo, D, D, N));
   ARB_TRY(arb_attn_bwd(k.qkv, k.qkv + 2 * D, k.qkv + 4 * D, k.att, t1, k.lse, dqkv, dqkv + 2 * D, dqkv + 4 * D, delta, nullptr, int(a.B),
                        T, H, 3 * D, 3 * D, 3 * D, D, D, 3 * D, 3 * D, 3 * D, int(a.window), float(a.scale), g.err, s));
   ARB_TRY(arb_qkv_post_bwd(dqkv, k.qkv, a.cos_t, a.sin_t, k.rstd, k.xn, ids, a.ve, a.ve ? a.gate_w : nullptr, a.ve ? k.gate : nullptr,
@@ -121,13 +131,13 @@ extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s
   if (!a.group_dw) ARB_TRY(g.dw(dqkv, k.xn, a.g_wqkv, 3 * D, D, N));
   ARB_TRY(g.nn(dqkv, a.wqkv, t1, nullptr, N, D, 3 * D, EPI_STORE_BF16));
   if (a.ve) ARB_TRY(arb_add_cols(t1, D, dxg, N, ch, s));
-  ARB_TRY(arb_resid_scale_norm_bwd(a.x, a.x0, a.lam_r, a.lam_0, int(a.idx), g2, t1, a.d_x, a.d_x0, a.d_x0_acc,
+  ARB_TRY(arb_resid_scale_norm_bwd(a.x, a.x0, a.lam_r, a.lam_0, int(a.idx), gs, t1, a.d_x, a.d_x0, a.d_x0_acc,
                                    static_cast<float*>(a.g_lam_r), static_cast<float*>(a.g_lam_0), N, int(D), eps, s));
   if (a.group_dw) {
-    const void *dy[4] = {dqkv, dh, a.g, g2}, *x[4] = {k.xn, k.xn2, k.act, k.att};
-    float* c[4] = {static_cast<float*>(a.g_wqkv), static_cast<float*>(a.g_wfc), static_cast<float*>(a.g_wdn), static_cast<float*>(a.g_wo)};
-    const int d = int(D), f = int(a.M), rows[4] = {3 * d, f, d, d}, cols[4] = {d, d, f, d};
-    ARB_TRY(arb_gemm_dw_group(dy, x, c, rows, cols, 4, int(N), g.err, s));
+    const void *dy[4] = {dqkv, gs, a.g, dh}, *x[4] = {k.xn, k.att, k.act, k.xn2};
+    float* c[4] = {static_cast<float*>(a.g_wqkv), static_cast<float*>(a.g_wo), static_cast<float*>(a.g_wdn), static_cast<float*>(a.g_wfc)};
+    const int d = int(D), f = int(a.M), rows[4] = {3 * d, d, d, f}, cols[4] = {d, d, f, d};
+    ARB_TRY(arb_gemm_dw_group(dy, x, c, rows, cols, a.half ? 2 : 4, int(N), g.err, s));
   }
   *launches = n;
   return 0;

@@ -405,67 +405,89 @@ class AttentionFn(torch.autograd.Function):
 GROUP_DW_FLOPS = 6e10
 
 
+def _layer_forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, B, T, window, idx, gate_ch, eps, chain, out2):
+    """Forward launches of a layer, or with ``out2`` (and no MLP matrices) of its half up to the second norm."""
+    N, D = x.shape
+    half = out2 is not None
+    M, H = 0 if half else wfc.shape[0], D // 128
+    stat = (N * H + 3) // 4 * 8                            # fp32 [N, H] in bf16 elements; lse, rstd of q and k, gate
+    kept = torch.empty(N * ((6 if half else 8) * D + M) + 4 * stat, dtype=torch.bfloat16, device=x.device)
+    out = torch.empty_like(x)
+    group = int(2 * N * D * (4 * D + 2 * M) <= GROUP_DW_FLOPS)
+    sizes = (B, T, H, M, window, idx, gate_ch, int(K.qkv_post_fusable(N, 3 * D)), group, int(half))
+    ptrs = [t.data_ptr() if t is not None else 0 for t in (x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin)]
+    ptrs += (kept.data_ptr(), out.data_ptr(), out2.data_ptr() if half else 0, K.err_flag(x.device).data_ptr())
+    K.layer_call("arb_layer_fwd", ptrs + [0] * 13, sizes, eps, 1.0 / math.sqrt(128.0))
+    ctx.save_for_backward(x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept, out if half else None)
+    ctx.sizes, ctx.eps, ctx.chain = sizes, eps, chain
+    return out
+
+
+def _layer_backward(ctx, g, g_xn):
+    x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept, out = ctx.saved_tensors
+    B, T, H, M, _, idx, gate_ch, _, group, half = ctx.sizes
+    chain = ctx.chain
+    N, D = x.shape
+    dev = x.device
+    if K.pending_pulls:
+        K.flush_pending_pulls()
+    g, g_xn = (t.contiguous() if t is not None else None for t in (g, g_xn))
+    params = (lam_r, lam_0, wqkv, wo, wfc, wdn, gate_w)
+    mains = [_main_grad(p) if p is not None else None for p in params]
+    accs = [m if m is not None or p is None else torch.zeros(p.shape, dtype=torch.float32, device=dev) for m, p in zip(mains, params)]
+    wide = M + 4 * D if group else max(M, 4 * D)
+    work = torch.empty(N * (wide + 2 * D + gate_ch) + 8 + 2 * ((N * H + 3) // 4 * 8), dtype=torch.bfloat16, device=dev)
+    dx = torch.empty_like(x)
+    acc0 = chain.buf
+    dx0 = acc0 if acc0 is not None else torch.empty_like(x)
+    ptrs = [t.data_ptr() if t is not None else 0 for t in
+            (x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept, out, None, K.err_flag(dev), g, g_xn, work, dx, dx0,
+             acc0, *accs)]
+    K.layer_call("arb_layer_bwd", ptrs, ctx.sizes, ctx.eps, 1.0 / math.sqrt(128.0))
+    g_ve = None
+    if ve is not None:
+        lo = N * (3 * D + (M if group else 0))
+        d_ve = work[lo:lo + N * D].view(N, D)
+        mgv = _main_grad(ve)
+        acc = mgv if mgv is not None else torch.zeros(ve.shape, dtype=torch.float32, device=dev)
+        K.embedding_bwd(ids, d_ve, acc)
+        g_ve = None if mgv is not None else acc.to(ve.dtype)
+    chain.buf = dx0
+    if idx != 0:
+        dx0 = None              # still being summed; layer 0 of the stage returns it
+    else:
+        chain.buf = None
+    gp = [None if m is not None or p is None else a.to(p.dtype) for m, a, p in zip(mains, accs, params)]
+    return dx, dx0, gp[:6], g_ve, gp[6]
+
+
 class DenseLayerFn(torch.autograd.Function):
     """A whole dense layer, launched by one native call per direction (csrc/layer.cu): the kernels, their order and their
     arguments are those of ResidScaleNormFn, AttnPreFn, AttentionFn, LinearAddNormFn and MLPFn in a row.  What the layer
     keeps for its backward pass is one buffer."""
 
     @staticmethod
-    def forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, B, T, window, idx, gate_ch, eps, chain):
-        N, D = x.shape
-        M, H = wfc.shape[0], D // 128
-        stat = (N * H + 3) // 4 * 8                            # fp32 [N, H] in bf16 elements; lse, rstd of q and k, gate
-        kept = torch.empty(N * (8 * D + M) + 4 * stat, dtype=torch.bfloat16, device=x.device)
-        out = torch.empty_like(x)
-        group = int(2 * N * D * (4 * D + 2 * M) <= GROUP_DW_FLOPS)
-        sizes = (B, T, H, M, window, idx, gate_ch, int(K.qkv_post_fusable(N, 3 * D)), group)
-        ptrs = [t.data_ptr() for t in (x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn)]
-        ptrs += (ve.data_ptr(), gate_w.data_ptr()) if ve is not None else (0, 0)
-        ptrs += (ids.data_ptr(), cos.data_ptr(), sin.data_ptr(), kept.data_ptr(), out.data_ptr(), K.err_flag(x.device).data_ptr())
-        K.layer_call("arb_layer_fwd", ptrs + [0] * 12, sizes, eps, 1.0 / math.sqrt(128.0))
-        ctx.save_for_backward(x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept)
-        ctx.sizes, ctx.eps, ctx.chain = sizes, eps, chain
-        return out
+    def forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, *rest):
+        return _layer_forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, *rest, None)
 
     @staticmethod
     def backward(ctx, g):
-        x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept = ctx.saved_tensors
-        B, T, H, M, _, idx, gate_ch, _, group = ctx.sizes
-        chain = ctx.chain
-        N, D = x.shape
-        dev = x.device
-        if K.pending_pulls:
-            K.flush_pending_pulls()
-        g = g.contiguous()
-        params = (lam_r, lam_0, wqkv, wo, wfc, wdn) + ((gate_w,) if ve is not None else ())
-        mains = [_main_grad(p) for p in params]
-        accs = [m if m is not None else torch.zeros(p.shape, dtype=torch.float32, device=dev) for m, p in zip(mains, params)]
-        wide = M + 4 * D if group else max(M, 4 * D)
-        work = torch.empty(N * (wide + 2 * D + gate_ch) + 8 + 2 * ((N * H + 3) // 4 * 8), dtype=torch.bfloat16, device=dev)
-        dx = torch.empty_like(x)
-        acc0 = chain.buf
-        dx0 = acc0 if acc0 is not None else torch.empty_like(x)
-        ptrs = [t.data_ptr() for t in (x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn)]
-        ptrs += (ve.data_ptr(), gate_w.data_ptr()) if ve is not None else (0, 0)
-        ptrs += (ids.data_ptr(), cos.data_ptr(), sin.data_ptr(), kept.data_ptr(), 0, K.err_flag(dev).data_ptr(),
-                 g.data_ptr(), work.data_ptr(), dx.data_ptr(), dx0.data_ptr(), dx0.data_ptr() if acc0 is not None else 0)
-        ptrs += [t.data_ptr() for t in accs] + ([0] if ve is None else [])
-        K.layer_call("arb_layer_bwd", ptrs, ctx.sizes, ctx.eps, 1.0 / math.sqrt(128.0))
-        g_ve = None
-        if ve is not None:
-            lo = N * (3 * D + (M if group else 0))
-            d_ve = work[lo:lo + N * D].view(N, D)
-            mgv = _main_grad(ve)
-            acc = mgv if mgv is not None else torch.zeros(ve.shape, dtype=torch.float32, device=dev)
-            K.embedding_bwd(ids, d_ve, acc)
-            g_ve = None if mgv is not None else acc.to(ve.dtype)
-        chain.buf = dx0
-        if idx != 0:
-            dx0 = None              # still being summed; layer 0 of the stage returns it
-        else:
-            chain.buf = None
-        gp = [None if m is not None else a.to(p.dtype) for m, a, p in zip(mains, accs, params)]
-        return (dx, dx0, *gp[:6], g_ve, gp[6] if ve is not None else None) + (None,) * 10
+        dx, dx0, gp, g_ve, g_gate = _layer_backward(ctx, g, None)
+        return (dx, dx0, *gp, g_ve, g_gate) + (None,) * 10
+
+
+class AttentionHalfFn(torch.autograd.Function):
+    """The same calls for what precedes the experts of an expert layer: (residual stream, its norm)."""
+
+    @staticmethod
+    def forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, ve, gate_w, *rest):
+        xn2 = torch.empty_like(x)
+        return _layer_forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, None, None, ve, gate_w, *rest, xn2), xn2
+
+    @staticmethod
+    def backward(ctx, g_xs, g_xn):
+        dx, dx0, gp, g_ve, g_gate = _layer_backward(ctx, g_xs, g_xn)
+        return (dx, dx0, *gp[:4], g_ve, g_gate) + (None,) * 10
 
 
 class LibraryAttentionFn(torch.autograd.Function):
@@ -691,27 +713,42 @@ class Sm100Backend(OracleBackend):
     def resid_scale_norm(self, x, x0, lam_r, lam_0, i):
         return ResidScaleNormFn.apply(x.contiguous(), x0.contiguous(), lam_r, lam_0, i, self.eps, self._chain(i))
 
-    def dense_layer(self, x, x0, lam_r, lam_0, i, blk, ids_flat, B, T, cfg, cos, sin, window):
-        """The whole layer through DenseLayerFn, or None where its steps have to run one by one: experts, tensor
-        parallelism, the library attention, parameters that still wait to be copied from their owner by the GEMMs that use
-        them, and operands that are not the dense bf16 tensors the native call takes (the separate steps say what is wrong)."""
-        if not self.layer_calls or blk.router is not None or self._tp() is not None or self.attn != "own" or K.pending_pulls:
-            return None
+    def _one_call(self, x, x0, lam_r, lam_0, blk, ids_flat, B, T, cfg, cos, sin):
+        """Whether a layer can go through one native call: not under tensor parallelism, with the library attention or while
+        parameters still wait to be copied from their owner by the GEMMs that use them, and only with the dense bf16 operands the
+        call takes (the separate steps say what is wrong with others)."""
+        if not self.layer_calls or self._tp() is not None or self.attn != "own" or K.pending_pulls or x.dim() != 2:
+            return False
         N, D = x.shape
-        M = blk.wfc.shape[0]
-        want = [(x, (N, D)), (x0, (N, D)), (blk.wqkv, (3 * D, D)), (blk.wo, (D, D)), (blk.wfc, (M, D)), (blk.wdn, (D, M)),
-                (lam_r, lam_r.shape), (lam_0, lam_0.shape), (cos, (cos.shape[0], 64)), (sin, (cos.shape[0], 64))]
+        want = [(x, (N, D)), (x0, (N, D)), (blk.wqkv, (3 * D, D)), (blk.wo, (D, D)), (lam_r, lam_r.shape), (lam_0, lam_0.shape),
+                (cos, (cos.shape[0], 64)), (sin, (cos.shape[0], 64))]
+        if blk.router is None:
+            M = blk.wfc.shape[0]
+            if M % 8:
+                return False
+            want += [(blk.wfc, (M, D)), (blk.wdn, (D, M))]
         if blk.ve is not None:
             want += [(blk.ve, (blk.ve.shape[0], D)), (blk.ve_gate, (D // 128, cfg.ve_gate_ch))]
         dev = x.device
         for t, shape in want:
             if t.dtype is not torch.bfloat16 or t.shape != shape or t.device != dev or not t.is_contiguous():
-                return None
-        if (N != B * T or D % 128 or cfg.head_dim != 128 or M % 8 or cos.shape[0] < T or ids_flat.dtype is not torch.int32 or
-                ids_flat.shape != (N,) or ids_flat.device != dev or not ids_flat.is_contiguous() or not x.is_cuda):
+                return False
+        return (N == B * T and D % 128 == 0 and cfg.head_dim == 128 and cos.shape[0] >= T and ids_flat.dtype is torch.int32 and
+                ids_flat.shape == (N,) and ids_flat.device == dev and ids_flat.is_contiguous() and x.is_cuda)
+
+    def dense_layer(self, x, x0, lam_r, lam_0, i, blk, ids_flat, B, T, cfg, cos, sin, window):
+        """A dense layer through DenseLayerFn: its output, or None where its steps have to run one by one."""
+        if blk.router is not None or not self._one_call(x, x0, lam_r, lam_0, blk, ids_flat, B, T, cfg, cos, sin):
             return None
         return DenseLayerFn.apply(x, x0, lam_r, lam_0, blk.wqkv, blk.wo, blk.wfc, blk.wdn, blk.ve, blk.ve_gate, ids_flat, cos, sin,
                                   B, T, window, i, cfg.ve_gate_ch, self.eps, self._chain(i))
+
+    def attention_half(self, x, x0, lam_r, lam_0, i, blk, ids_flat, B, T, cfg, cos, sin, window):
+        """An expert layer up to the input of its experts: (residual stream, its norm), or None as in dense_layer."""
+        if blk.router is None or not self._one_call(x, x0, lam_r, lam_0, blk, ids_flat, B, T, cfg, cos, sin):
+            return None
+        return AttentionHalfFn.apply(x, x0, lam_r, lam_0, blk.wqkv, blk.wo, blk.ve, blk.ve_gate, ids_flat, cos, sin,
+                                     B, T, window, i, cfg.ve_gate_ch, self.eps, self._chain(i))
 
     def linear_col(self, x, w):
         return LinearFn.apply(x, w)

@@ -66,15 +66,17 @@ def test_training_step_sm100_loss_decreases():
     assert losses[-1] < losses[0] - 0.3, losses
 
 
-@pytest.mark.parametrize("batch,seq,layers,heads", [(1, 512, 4, 2), (3, 331, 6, 2), (1, 130, 2, 2), (3, 301, 3, 3), (1, 3, 1, 1)])
-def test_whole_layer_calls_give_the_bits_of_the_separate_steps(batch, seq, layers, heads):
+@pytest.mark.parametrize("batch,seq,layers,heads,experts", [(1, 512, 4, 2, 0), (3, 331, 6, 2, 0), (1, 130, 2, 2, 0), (3, 301, 3, 3, 0),
+                                                            (1, 3, 1, 1, 0), (2, 300, 3, 2, 4), (1, 130, 2, 3, 4)])
+def test_whole_layer_calls_give_the_bits_of_the_separate_steps(batch, seq, layers, heads, experts):
     """One native call per layer and direction against one autograd node per step: the same kernels on the same operands, so
     losses agree bit for bit and matrix gradients up to the order in which split-K sums meet.  130 rows take the separate
     rotation kernel (products below the 2-CTA tiles), 993 end inside a tile, 903 x 3 leaves the row statistics at odd offsets."""
-    from autoresearch_b200.config import ModelConfig
+    from autoresearch_b200.config import ModelConfig, MoEConfig
     from autoresearch_b200.ops import kernels as K
+    moe = MoEConfig(n_experts=experts, top_k=2, mlp_dim_e=512 * heads, capacity_factor=1.25) if experts else None
     cfg = ModelConfig(vocab=1024, seq_len=512, d_model=128 * heads, n_head=heads, head_dim=128, mlp_dim=512 * heads,
-                      n_layer=layers)
+                      n_layer=layers, moe=moe)
     torch.manual_seed(3)
     mod = _build("sm100", cfg, torch.bfloat16)
     ids = torch.randint(0, cfg.vocab, (batch, seq), device="cuda", dtype=torch.int32)
