@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(1024) emb_plan_scan_k(const int* __restrict__ 
   grid_enter();
   __shared__ int wsum[2][32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int row0 = 0, it0 = 0;                             // rows and items of the ids below this round's
+  int row0 = 0, it0 = 0;                             // rows and items of the ids before v0
   for (int v0 = 0; v0 < vocab; v0 += 1024) {
     const int v = v0 + tid;
     const int n = v < vocab ? counts[v] : 0, it = (n + R - 1) / R;
