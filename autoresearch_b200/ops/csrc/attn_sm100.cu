@@ -785,8 +785,8 @@ attn_bwd_dkv_k(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
 // delta[b,h,t] = sum_d dO[b,t,h,d] * O[b,t,h,d]; one warp per token, a half-warp per head (16-byte loads, two heads
 // per iteration), the token arithmetic done once per warp
-__global__ void __launch_bounds__(256) attn_delta_k(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                                    float* __restrict__ delta, int B, int T, int H, long long ldo, long long lddo) {
+__global__ void __launch_bounds__(256) attn_delta_k(const __nv_bfloat16* o, const __nv_bfloat16* d_o,
+                                                    float* delta, int B, int T, int H, long long ldo, long long lddo) {
   grid_enter();
   const long long bt = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;

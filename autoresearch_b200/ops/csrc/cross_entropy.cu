@@ -14,8 +14,8 @@ constexpr int CE_THREADS = 256;
 // The soft-capped logits lie in [-cap, cap], so exp(s - cap) can neither overflow nor vanish in fp32 (cap = 15 gives
 // e^-30 at worst): the row maximum and its block-wide reduction are not needed.  One barrier per row.
 template <int VPT>  // 8-element vectors per thread
-__global__ void __launch_bounds__(CE_THREADS) softcap_ce_k(__nv_bfloat16* __restrict__ logits, long long ld,
-                                                           const int* __restrict__ targets, float* __restrict__ loss,
+__global__ void __launch_bounds__(CE_THREADS) softcap_ce_k(__nv_bfloat16* logits, long long ld,
+                                                           const int* targets, float* loss,
                                                            int V, float cap, float gscale) {
   grid_enter();
   __shared__ float red[CE_THREADS / 32];

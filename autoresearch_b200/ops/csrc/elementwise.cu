@@ -41,7 +41,7 @@ constexpr int ROWS_PER_CTA = 8;  // 8 warps, one row each
 
 // ---------------------------------------------------------------------------------------------
 template <int NV>
-__global__ void __launch_bounds__(256) rmsnorm_fwd_k(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
+__global__ void __launch_bounds__(256) rmsnorm_fwd_k(const __nv_bfloat16* x, __nv_bfloat16* y,
                                                      long long rows, int D, float eps) {
   grid_enter();
   const int lane = threadIdx.x & 31;
@@ -74,8 +74,8 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_k(const __nv_bfloat16* __rest
 
 // gx = (add_to ? add_to : 0) + r*(g - x*(g.x)/D*r^2)
 template <int NV>
-__global__ void __launch_bounds__(256) rmsnorm_bwd_k(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
-                                                     const __nv_bfloat16* __restrict__ add_to, __nv_bfloat16* __restrict__ gx,
+__global__ void __launch_bounds__(256) rmsnorm_bwd_k(const __nv_bfloat16* x, const __nv_bfloat16* g,
+                                                     const __nv_bfloat16* add_to, __nv_bfloat16* gx,
                                                      long long rows, int D, float eps) {
   grid_enter();
   const int lane = threadIdx.x & 31;
@@ -136,9 +136,9 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_k(const __nv_bfloat16* __rest
 
 // x' = lr*x + l0*x0 (stored bf16) ; xn = rmsnorm(x')
 template <int NV, bool SCALE>
-__global__ void __launch_bounds__(256) resid_norm_fwd_k(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ x0,
-                                                        const __nv_bfloat16* __restrict__ lam_r, const __nv_bfloat16* __restrict__ lam_0,
-                                                        int idx, __nv_bfloat16* __restrict__ xo, __nv_bfloat16* __restrict__ xn,
+__global__ void __launch_bounds__(256) resid_norm_fwd_k(const __nv_bfloat16* x, const __nv_bfloat16* x0,
+                                                        const __nv_bfloat16* lam_r, const __nv_bfloat16* lam_0,
+                                                        int idx, __nv_bfloat16* xo, __nv_bfloat16* xn,
                                                         long long rows, int D, float eps) {
   grid_enter();
   const int lane = threadIdx.x & 31;
@@ -161,15 +161,15 @@ __global__ void __launch_bounds__(256) resid_norm_fwd_k(const __nv_bfloat16* __r
         v[i][j] = bf16_round(lr * v[i][j] + l0 * b[j]);
         ss += v[i][j] * v[i][j];
       }
-      st8(xo + row * D + c * 8, v[i]);
     }
   }
   ss = warp_sum(ss);
   const float r = rsqrtf(ss / D + eps);
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
+  for (int i = 0; i < NV; ++i) {                     // stores only: all loads of the row are under way above
     const int c = lane + 32 * i;
     if (c < nch) {
+      st8(xo + row * D + c * 8, v[i]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[i][j] *= r;
       st8(xn + row * D + c * 8, v[i]);
@@ -178,12 +178,12 @@ __global__ void __launch_bounds__(256) resid_norm_fwd_k(const __nv_bfloat16* __r
 }
 
 template <int NV>
-__global__ void __launch_bounds__(256) resid_norm_bwd_k(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ x0,
-                                                        const __nv_bfloat16* __restrict__ lam_r, const __nv_bfloat16* __restrict__ lam_0,
-                                                        int idx, const __nv_bfloat16* __restrict__ g_xs, const __nv_bfloat16* __restrict__ g_xn,
-                                                        __nv_bfloat16* __restrict__ d_x, __nv_bfloat16* d_x0,
+__global__ void __launch_bounds__(256) resid_norm_bwd_k(const __nv_bfloat16* x, const __nv_bfloat16* x0,
+                                                        const __nv_bfloat16* lam_r, const __nv_bfloat16* lam_0,
+                                                        int idx, const __nv_bfloat16* g_xs, const __nv_bfloat16* g_xn,
+                                                        __nv_bfloat16* d_x, __nv_bfloat16* d_x0,
                                                         const __nv_bfloat16* d_x0_acc,
-                                                        float* __restrict__ dlam_r, float* __restrict__ dlam_0,
+                                                        float* dlam_r, float* dlam_0,
                                                         long long rows, int D, float eps) {
   grid_enter();
   // d_x0_acc (may equal d_x0): the x0 gradient of the layers above, added here instead of by a separate pass
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(256) resid_norm_bwd_k(const __nv_bfloat16* __r
 }
 
 // ---------------------------------------------------------------------------------------------
-__global__ void residual_add_k(const uint4* __restrict__ a, const uint4* __restrict__ b, uint4* __restrict__ o, long long n8) {
+__global__ void residual_add_k(const uint4* a, const uint4* b, uint4* o, long long n8) {
   grid_enter();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
     float x[8], y[8];
@@ -322,7 +322,7 @@ __global__ void add_cols_k(__nv_bfloat16* dst, long long ld_dst, const __nv_bflo
 
 // ---------------------------------------------------------------------------------------------
 // embedding
-__global__ void embedding_fwd_k(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
+__global__ void embedding_fwd_k(const int* ids, const __nv_bfloat16* w, __nv_bfloat16* out,
                                 long long N, int D, int vocab) {
   grid_enter();
   const int nch = D >> 3;
@@ -361,10 +361,10 @@ __global__ void embedding_bwd_k(const int* __restrict__ ids, const __nv_bfloat16
 // in flight, and the groups' sums meet in shared memory in group order.  (One group of D / 8 threads walking all 64 rows of an
 // item took 18 us for 1024 tokens of width 256, whose gradient is 0.5 MB.)
 constexpr int EMB_THREADS = 256;
-__global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_sorted_k(const long long* __restrict__ perm, const int* __restrict__ item_id,
-                                                              const int* __restrict__ item_start, const int* __restrict__ seg_start,
-                                                              const int* __restrict__ seg_count, const __nv_bfloat16* __restrict__ g,
-                                                              float* __restrict__ dw, float* __restrict__ partial, int n_items_max,
+__global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_sorted_k(const long long* perm, const int* item_id,
+                                                              const int* item_start, const int* seg_start,
+                                                              const int* seg_count, const __nv_bfloat16* g,
+                                                              float* dw, float* partial, int n_items_max,
                                                               int D, int R, int vocab) {
   grid_enter();
   __shared__ __align__(16) float red[EMB_THREADS][8];
@@ -424,8 +424,8 @@ __global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_sorted_k(const long
     *reinterpret_cast<float4*>(dst + 4) = b;
   }
 }
-__global__ void __launch_bounds__(128) embedding_bwd_combine_k(const int* __restrict__ item_start, const int* __restrict__ seg_count,
-                                                               const float* __restrict__ partial, float* __restrict__ dw, int D, int R) {
+__global__ void __launch_bounds__(128) embedding_bwd_combine_k(const int* item_start, const int* seg_count,
+                                                               const float* partial, float* dw, int D, int R) {
   grid_enter();
   const int id = blockIdx.x;
   const int cnt = seg_count[id];
@@ -451,7 +451,7 @@ constexpr int PLAN_CHUNK = 1024;
 constexpr int PLAN_MAX_VOCAB = 49152;                // one counter per id in shared memory
 __device__ __forceinline__ int plan_id(const int* ids, long long i, int vocab) { return min(max(ids[i], 0), vocab - 1); }
 
-__global__ void __launch_bounds__(256) emb_plan_hist_k(const int* __restrict__ ids, long long N, int vocab, int* __restrict__ hist) {
+__global__ void __launch_bounds__(256) emb_plan_hist_k(const int* ids, long long N, int vocab, int* hist) {
   grid_enter();
   extern __shared__ int plan_cnt[];
   for (int v = threadIdx.x; v < vocab; v += 256) plan_cnt[v] = 0;
@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(256) emb_plan_hist_k(const int* __restrict__ i
   __syncthreads();
   for (int v = threadIdx.x; v < vocab; v += 256) hist[(long long)blockIdx.x * vocab + v] = plan_cnt[v];
 }
-__global__ void __launch_bounds__(64) emb_plan_chunks_k(int* __restrict__ hist, int n_chunks, int vocab, int* __restrict__ counts) {
+__global__ void __launch_bounds__(64) emb_plan_chunks_k(int* hist, int n_chunks, int vocab, int* counts) {
   grid_enter();
   const int v = blockIdx.x * 64 + threadIdx.x;
   if (v >= vocab) return;
@@ -478,9 +478,9 @@ __global__ void __launch_bounds__(64) emb_plan_chunks_k(int* __restrict__ hist, 
   for (; c < n_chunks; ++c) { const int x = h[(long long)c * vocab]; h[(long long)c * vocab] = sum; sum += x; }
   counts[v] = sum;
 }
-__global__ void __launch_bounds__(1024) emb_plan_scan_k(const int* __restrict__ counts, int vocab, int R, int n_items_max,
-                                                        int* __restrict__ seg_start, int* __restrict__ item_start,
-                                                        int* __restrict__ item_id) {
+__global__ void __launch_bounds__(1024) emb_plan_scan_k(const int* counts, int vocab, int R, int n_items_max,
+                                                        int* seg_start, int* item_start,
+                                                        int* item_id) {
   grid_enter();
   __shared__ int wsum[2][32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -515,8 +515,8 @@ __global__ void __launch_bounds__(1024) emb_plan_scan_k(const int* __restrict__ 
   }
   for (int i = it0 + tid; i < n_items_max; i += 1024) item_id[i] = -1;
 }
-__global__ void __launch_bounds__(256) emb_plan_place_k(const int* __restrict__ ids, long long N, int vocab, const int* __restrict__ hist,
-                                                        const int* __restrict__ seg_start, long long* __restrict__ perm) {
+__global__ void __launch_bounds__(256) emb_plan_place_k(const int* ids, long long N, int vocab, const int* hist,
+                                                        const int* seg_start, long long* perm) {
   grid_enter();
   extern __shared__ int plan_cnt[];                  // next sorted position of every id
   for (int v = threadIdx.x; v < vocab; v += 256) plan_cnt[v] = seg_start[v] + hist[(long long)blockIdx.x * vocab + v];
@@ -555,11 +555,11 @@ __device__ __forceinline__ void st4(__nv_bfloat16* p, const float (&f)[4]) {
 // One warp per token: the cos/sin row of the token is loaded once and reused by all 2H q/k heads, the
 // token-index arithmetic is done once, and two heads are in flight per iteration.  (One warp per
 // (token, head) made these kernels instruction-bound: 2-3 million warps, each with two 64-bit divisions.)
-__global__ void __launch_bounds__(256) qkv_post_fwd_k(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ cos_t,
-                                                      const __nv_bfloat16* __restrict__ sin_t, float* __restrict__ rstd_qk,
-                                                      const __nv_bfloat16* __restrict__ xn, const int* __restrict__ ids,
-                                                      const __nv_bfloat16* __restrict__ ve_w, const __nv_bfloat16* __restrict__ gate_w,
-                                                      float* __restrict__ gate_out, long long N, int T, int H, int D_model,
+__global__ void __launch_bounds__(256) qkv_post_fwd_k(__nv_bfloat16* qkv, const __nv_bfloat16* cos_t,
+                                                      const __nv_bfloat16* sin_t, float* rstd_qk,
+                                                      const __nv_bfloat16* xn, const int* ids,
+                                                      const __nv_bfloat16* ve_w, const __nv_bfloat16* gate_w,
+                                                      float* gate_out, long long N, int T, int H, int D_model,
                                                       int gate_ch, float eps) {
   grid_enter();
   const int lane = threadIdx.x & 31;
@@ -619,12 +619,12 @@ __global__ void __launch_bounds__(256) qkv_post_fwd_k(__nv_bfloat16* __restrict_
   }
 }
 
-__global__ void __launch_bounds__(256) qkv_post_bwd_k(__nv_bfloat16* __restrict__ dqkv, const __nv_bfloat16* __restrict__ qkv,
-                                                      const __nv_bfloat16* __restrict__ cos_t, const __nv_bfloat16* __restrict__ sin_t,
-                                                      const float* __restrict__ rstd_qk, const __nv_bfloat16* __restrict__ xn,
-                                                      const int* __restrict__ ids, const __nv_bfloat16* __restrict__ ve_w,
-                                                      const __nv_bfloat16* __restrict__ gate_w, const float* __restrict__ gate,
-                                                      __nv_bfloat16* __restrict__ d_ve, float* __restrict__ d_gate_logit,
+__global__ void __launch_bounds__(256) qkv_post_bwd_k(__nv_bfloat16* dqkv, const __nv_bfloat16* qkv,
+                                                      const __nv_bfloat16* cos_t, const __nv_bfloat16* sin_t,
+                                                      const float* rstd_qk, const __nv_bfloat16* xn,
+                                                      const int* ids, const __nv_bfloat16* ve_w,
+                                                      const __nv_bfloat16* gate_w, const float* gate,
+                                                      __nv_bfloat16* d_ve, float* d_gate_logit,
                                                       long long N, int T, int H) {
   grid_enter();
   const int lane = threadIdx.x & 31;
@@ -689,9 +689,9 @@ __global__ void __launch_bounds__(256) qkv_post_bwd_k(__nv_bfloat16* __restrict_
 // memory by all threads, then thread (h, j) walks down its column there.  (With the walk over global memory, 512 dependent
 // steps of two loads on N / 512 CTAs, the kernel took 85 us for 2048 tokens and 119 us for 32768.)
 constexpr int VE_CHUNK = 64;
-__global__ void __launch_bounds__(256) ve_gate_bwd_k(const float* __restrict__ dgl, const __nv_bfloat16* __restrict__ xn,
-                                                     const __nv_bfloat16* __restrict__ gate_w, float* __restrict__ d_gate_w,
-                                                     __nv_bfloat16* __restrict__ d_xn_gate, long long N, int H, int D_model,
+__global__ void __launch_bounds__(256) ve_gate_bwd_k(const float* dgl, const __nv_bfloat16* xn,
+                                                     const __nv_bfloat16* gate_w, float* d_gate_w,
+                                                     __nv_bfloat16* d_xn_gate, long long N, int H, int D_model,
                                                      int ch, int tok_per_cta, int chunk) {
   grid_enter();
   extern __shared__ float ve_sm[];

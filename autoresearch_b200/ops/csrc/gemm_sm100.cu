@@ -414,7 +414,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, 2 * BN); }
 }
 
-// One head (128 accumulator columns of one row) of the packed q|k|v projection, in place.
+// One head (128 accumulator columns of one row) of the packed q|k|v projection, in place.  Ordinary loads: xn is what the kernel
+// before this one, which may still run when this one starts, has written (ptx.cuh).
 __device__ __forceinline__ void qkv_post_head(float (&f)[128], const QkvPostArgs& q, int row, int col_h) {
   const int Dl = q.H * 128;
   const int sec = col_h / Dl;                       // 0 query, 1 key, 2 value
@@ -426,7 +427,7 @@ __device__ __forceinline__ void qkv_post_head(float (&f)[128], const QkvPostArgs
     float ss = 0.f;
 #pragma unroll
     for (int g = 0; g < 8; ++g) {
-      const uint4 cu = __ldg(cp + g), su = __ldg(sp + g);
+      const uint4 cu = cp[g], su = sp[g];
       const uint32_t cw[4] = {cu.x, cu.y, cu.z, cu.w}, sw[4] = {su.x, su.y, su.z, su.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -448,7 +449,7 @@ __device__ __forceinline__ void qkv_post_head(float (&f)[128], const QkvPostArgs
     const __nv_bfloat16* gw = q.gate_w + head * q.gate_ch;
     float gl = 0.f;
     for (int j = 0; j < q.gate_ch; j += 8) {
-      const uint4 xu = __ldg(reinterpret_cast<const uint4*>(xr + j)), gu = __ldg(reinterpret_cast<const uint4*>(gw + j));
+      const uint4 xu = *reinterpret_cast<const uint4*>(xr + j), gu = *reinterpret_cast<const uint4*>(gw + j);
       const uint32_t xw[4] = {xu.x, xu.y, xu.z, xu.w}, gg[4] = {gu.x, gu.y, gu.z, gu.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -461,7 +462,7 @@ __device__ __forceinline__ void qkv_post_head(float (&f)[128], const QkvPostArgs
     const uint4* vp = reinterpret_cast<const uint4*>(q.ve + (long long)q.ids[row] * Dl + head * 128);
 #pragma unroll
     for (int g = 0; g < 16; ++g) {
-      const uint4 eu = __ldg(vp + g);
+      const uint4 eu = vp[g];
       const uint32_t ew[4] = {eu.x, eu.y, eu.z, eu.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {

@@ -68,6 +68,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 // writes are visible.  grid_trigger() lets the successor start; a kernel that allocates TMEM triggers behind its allocation, so
 // that a waiting successor can never hold columns its predecessor still needs.  Every thread passes grid_wait(), early exits
 // included: a kernel's completion thereby implies that of everything before it.
+// Such a kernel takes no __restrict__ pointers and no __ldg: both promise data that do not change while the kernel runs, which would
+// let the compiler move their loads above the wait and read them past the caches that the predecessor's writes go through.  Where
+// that costs the order of loads and stores, the loads are written ahead of the stores by hand.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_enter() { grid_trigger(); grid_wait(); }
