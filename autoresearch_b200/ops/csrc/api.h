@@ -156,6 +156,8 @@ int arb_embedding_bwd_sorted(const long long* perm, const int* item_id, const in
 // counts / seg_start / item_start [vocab], item_id [n_items_max >= N / R + vocab].  vocab <= 49152.
 int arb_embedding_plan(const int* ids, long long N, int vocab, int R, int n_items_max, int* hist, long long* perm, int* counts,
                        int* seg_start, int* item_start, int* item_id, cudaStream_t s);
+// Id of the graph capture that the stream takes part in, 0 outside of one.
+int arb_capture_id(unsigned long long* id, cudaStream_t s);
 int arb_add_cols(void* dst, long long ld_dst, const void* src, long long rows, int cols, cudaStream_t s);
 int arb_cast_f32_to_bf16(const float* src, void* dst, long long n, float scale, cudaStream_t s);
 int arb_accum_bf16_into_f32(const void* src, float* dst, long long n, cudaStream_t s);

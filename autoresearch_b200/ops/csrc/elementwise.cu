@@ -895,6 +895,14 @@ int arb_embedding_plan(const int* ids, long long N, int vocab, int R, int n_item
   launch_dependent(true, emb_plan_place_k, chunks, 256, smem, s, ids, N, vocab, hist, seg_start, perm);
   return int(cudaGetLastError());
 }
+int arb_capture_id(unsigned long long* id, cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long n = 0;
+  cudaError_t e = cudaStreamGetCaptureInfo(s, &status, &n);
+  if (e == cudaErrorStreamCaptureImplicit) { cudaGetLastError(); e = cudaSuccess; }   // another stream captures, not this one
+  *id = e == cudaSuccess && status == cudaStreamCaptureStatusActive ? n : 0;
+  return int(e);
+}
 int arb_add_cols(void* dst, long long ld_dst, const void* src, long long rows, int cols, cudaStream_t s) {
   if (rows <= 0 || cols <= 0) return -3;
   launch_dependent(rows * cols * 2 <= EARLY_BYTES, add_cols_k, grid_for(rows * cols, 256), 256, 0, s, (bf16*)dst, ld_dst, (const bf16*)src, rows, cols);

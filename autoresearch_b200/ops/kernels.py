@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import struct
+import weakref
 from typing import Optional
 
 import torch
@@ -83,6 +84,7 @@ def _signatures() -> dict:
         "arb_embedding_bwd": [vp, vp, vp, i64, i32, i32, vp],
         "arb_embedding_bwd_sorted": [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp],
         "arb_embedding_plan": [vp, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp],
+        "arb_capture_id": [vp, vp],
         "arb_add_cols": [vp, i64, vp, i64, i32, vp],
         "arb_cast_f32_to_bf16": [vp, vp, i64, f32, vp],
         "arb_accum_bf16_into_f32": [vp, vp, i64, vp],
@@ -397,37 +399,37 @@ def embedding_fwd(ids, w):
 
 EMB_BWD_DETERMINISTIC = True   # sorted, atomic-free embedding gradient (False: fp32 atomics)
 EMB_BWD_ROWS_PER_ITEM = 64
-_emb_plan = {}
-
-
 EMB_PLAN_MAX_VOCAB = 49152     # one shared-memory counter per id (csrc/elementwise.cu)
+# {object of a forward pass: {what a plan was made from: plan}}: the gradients of one backward pass share a plan, and it goes with
+# the pass.  Nothing is kept from one pass for the next: that the same tensor holds the same ids cannot be seen from outside (a
+# graph replay or a kernel that writes through a pointer does not raise its version).
+_emb_plan = weakref.WeakKeyDictionary()
+
+
+def _capture_id() -> int:
+    """Id of the graph capture that the current stream takes part in, 0 outside of one."""
+    n = C.c_ulonglong(0)
+    rc = lib().arb_capture_id(C.addressof(n), _stream())
+    if rc != 0:
+        raise KernelError(f"arb_capture_id failed with code {rc}")
+    return n.value
 
 
 def _embedding_plan(ids, vocab: int):
-    """Sort order and work-item tables of one batch of token ids; kept until other ids come, since the word-embedding and
-    every value-embedding gradient of a micro-batch use the same ids.  The entry holds the id tensor itself, so that its
-    address cannot be handed to another one meanwhile, and serves the stream it was made on.  Fixed-size tensors only (no host sync)."""
-    slot = ("plan", ids.device.index)
-    key = (ids.data_ptr(), ids._version, ids.numel(), ids.dtype, vocab, _stream())
-    hit = _emb_plan.get(slot)
-    # a graph that is being captured holds its own plan kernels: the ids are other ones when it is replayed
-    if hit is not None and hit[0] == key and not torch.cuda.is_current_stream_capturing():
-        return hit[1]
+    """Sort order and work-item tables of one batch of token ids.  Fixed-size tensors only (no host sync)."""
     R = EMB_BWD_ROWS_PER_ITEM
     N = ids.numel()
     n_max = N // R + vocab + 1                                                     # upper bound of the item count
     n_chunks = (N + 1023) // 1024
     if vocab <= EMB_PLAN_MAX_VOCAB and n_chunks * vocab <= 1 << 25 and ids.dtype is torch.int32 and ids.is_contiguous():
         perm = torch.empty(N, dtype=torch.int64, device=ids.device)
-        counts, seg_start, item_start, item_id, hist = torch.empty(
-            3 * vocab + n_max + n_chunks * vocab, dtype=torch.int32, device=ids.device).split(
-            (vocab, vocab, vocab, n_max, n_chunks * vocab))
+        counts, seg_start, item_start, item_id = torch.empty(3 * vocab + n_max, dtype=torch.int32, device=ids.device).split(
+            (vocab, vocab, vocab, n_max))
+        hist = torch.empty(n_chunks * vocab, dtype=torch.int32, device=ids.device)
         _check(lib().arb_embedding_plan(ids.data_ptr(), N, vocab, R, n_max, hist.data_ptr(), perm.data_ptr(), counts.data_ptr(),
                                         seg_start.data_ptr(), item_start.data_ptr(), item_id.data_ptr(), _stream()),
                "embedding_plan")
-        plan = (perm, item_id, item_start, seg_start, counts, n_max)
-        _emb_plan[slot] = (key, plan, ids)
-        return plan
+        return perm, item_id, item_start, seg_start, counts, n_max
     flat = ids.reshape(-1).long().clamp(0, vocab - 1)
     perm = torch.sort(flat, stable=True).indices.contiguous()                     # int64 [N]
     # (torch.bincount reads the largest id back to the host to size its result: a sync per micro-batch)
@@ -439,19 +441,36 @@ def _embedding_plan(ids, vocab: int):
     item = torch.arange(n_max, device=ids.device)
     item_id = torch.searchsorted(it_end, item, right=True)
     item_id = torch.where(item < it_end[-1], item_id, torch.full_like(item_id, -1)).to(torch.int32)
-    plan = (perm, item_id.contiguous(), item_start.contiguous(), seg_start.contiguous(), counts.to(torch.int32).contiguous(), n_max)
-    _emb_plan[slot] = (key, plan, ids)
-    return plan
+    return perm, item_id.contiguous(), item_start.contiguous(), seg_start.contiguous(), counts.to(torch.int32).contiguous(), n_max
 
 
-def embedding_bwd(ids, g, dw_f32):
-    """dw[id] += sum of the rows of g whose token is id."""
+def _plan_of_pass(ids, vocab: int, of_pass):
+    """The plan of these ids within the forward pass ``of_pass`` (None: a plan of its own).  It serves the stream it was made on;
+    one made under graph capture serves that capture only, since its kernels run at replay."""
+    if of_pass is None:
+        return _embedding_plan(ids, vocab)
+    plans = _emb_plan.setdefault(of_pass, {})
+    key = (ids.data_ptr(), None if ids.is_inference() else ids._version, ids.numel(), ids.dtype, vocab, _stream(), _capture_id())
+    if key not in plans:
+        plans[key] = _embedding_plan(ids, vocab)
+    return plans[key]
+
+
+def forget_embedding_plans(of_pass) -> None:
+    """The plans of a pass whose last embedding gradient has been launched."""
+    if of_pass is not None:
+        _emb_plan.pop(of_pass, None)
+
+
+def embedding_bwd(ids, g, dw_f32, of_pass=None):
+    """dw[id] += sum of the rows of g whose token is id.  ``of_pass``: an object that lives as long as the forward pass the
+    gradient belongs to; gradients with the same one share their plan."""
     D, vocab = g.shape[-1], dw_f32.shape[0]
     if not EMB_BWD_DETERMINISTIC:
         _check(lib().arb_embedding_bwd(ids.data_ptr(), g.data_ptr(), dw_f32.data_ptr(), ids.numel(), D, vocab, _stream()),
                "embedding_bwd")
         return
-    perm, item_id, item_start, seg_start, counts, n_max = _embedding_plan(ids, vocab)
+    perm, item_id, item_start, seg_start, counts, n_max = _plan_of_pass(ids, vocab, of_pass)
     scratch = torch.empty(n_max * D, dtype=torch.float32, device=g.device)
     _check(lib().arb_embedding_bwd_sorted(perm.data_ptr(), item_id.data_ptr(), item_start.data_ptr(), seg_start.data_ptr(),
                                           counts.data_ptr(), g.data_ptr(), dw_f32.data_ptr(), scratch.data_ptr(), n_max, D,

@@ -223,13 +223,15 @@ class LinearRelu2Fn(torch.autograd.Function):
         return dx, dw
 
 
-class _X0GradChain:
-    """The x0 gradient of one forward pass: every layer of a stage adds its share to one buffer inside its
-    backward kernel, and only the stage's first layer (the last to run backward) hands the sum to autograd."""
-    __slots__ = ("buf",)
+class _ForwardPass:
+    """What the nodes of one forward pass share: the x0 gradient (every layer of a stage adds its share to one buffer inside its
+    backward kernel, and only the stage's first layer, the last to run backward, hands the sum to autograd) and, through
+    ``kernels.embedding_bwd``, the sort order of its token ids."""
+    __slots__ = ("buf", "in_layers", "__weakref__")
 
     def __init__(self):
         self.buf = None
+        self.in_layers = False      # its first layer has been visited
 
 
 class ResidScaleNormFn(torch.autograd.Function):
@@ -265,29 +267,28 @@ class ResidScaleNormFn(torch.autograd.Function):
 
 class EmbeddingFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, ids, w):
+    def forward(ctx, ids, w, of_pass=None):
         ctx.save_for_backward(ids, w)
+        ctx.of_pass = of_pass
         return K.embedding_fwd(ids, w)
 
     @staticmethod
     def backward(ctx, g):
         ids, w = ctx.saved_tensors
         mg = _main_grad(w)
-        if mg is not None:
-            K.embedding_bwd(ids, g.contiguous(), mg)
-            return None, None
-        tmp = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
-        K.embedding_bwd(ids, g.contiguous(), tmp)
-        return None, tmp.to(w.dtype)
+        acc = mg if mg is not None else torch.zeros(w.shape, dtype=torch.float32, device=w.device)
+        K.embedding_bwd(ids, g.contiguous(), acc, ctx.of_pass)
+        K.forget_embedding_plans(ctx.of_pass)         # everything above has run
+        return None, None if mg is not None else acc.to(w.dtype), None
 
 
 class AttnPreFn(torch.autograd.Function):
     """packed qkv = post(xn @ wqkv^T): RoPE + QK-norm on q, k; value embedding on v."""
 
     @staticmethod
-    def forward(ctx, xn, wqkv, ids, ve_w, gate_w, cos, sin, T, H, gate_ch, eps, tp=None):
+    def forward(ctx, xn, wqkv, ids, ve_w, gate_w, cos, sin, T, H, gate_ch, eps, tp=None, of_pass=None):
         # tp (a FusedTPContext): xn is this rank's sequence shard; the gather is overlapped with the GEMM
-        ctx.tp = tp
+        ctx.tp, ctx.of_pass = tp, of_pass
         if tp is None and K.qkv_post_fusable(xn.shape[0], wqkv.shape[0]):
             # RoPE, QK-norm and the value embedding run in the epilogue of the projection: qkv is written once
             N, D = xn.shape
@@ -353,14 +354,14 @@ class AttnPreFn(torch.autograd.Function):
             K.add_cols_(dxn, d_xn_gate)
             mgv = _main_grad(ve_w)
             if mgv is not None:
-                K.embedding_bwd(ids, d_ve, mgv)
+                K.embedding_bwd(ids, d_ve, mgv, ctx.of_pass)
             else:
                 tmp = torch.zeros(ve_w.shape, dtype=torch.float32, device=xn.device)
-                K.embedding_bwd(ids, d_ve, tmp)
+                K.embedding_bwd(ids, d_ve, tmp, ctx.of_pass)
                 g_ve = tmp.to(ve_w.dtype)
             if _main_grad(gate_w) is None:
                 g_gate = dgw.to(gate_w.dtype)
-        return dxn, dw, None, g_ve, g_gate, None, None, None, None, None, None, None
+        return dxn, dw, None, g_ve, g_gate, None, None, None, None, None, None, None, None
 
 
 class AttentionFn(torch.autograd.Function):
@@ -450,7 +451,7 @@ def _layer_backward(ctx, g, g_xn):
         d_ve = work[lo:lo + N * D].view(N, D)
         mgv = _main_grad(ve)
         acc = mgv if mgv is not None else torch.zeros(ve.shape, dtype=torch.float32, device=dev)
-        K.embedding_bwd(ids, d_ve, acc)
+        K.embedding_bwd(ids, d_ve, acc, chain)
         g_ve = None if mgv is not None else acc.to(ve.dtype)
     chain.buf = dx0
     if idx != 0:
@@ -691,7 +692,7 @@ class Sm100Backend(OracleBackend):
         self.attn = attn
         self.big_ce_chunk = 16384
         self.layer_calls = True       # False: one autograd node and one native call per step of a layer
-        self._x0_chain = None
+        self._pass = None
 
     def optim_kernels(self):
         if getattr(self, "_optim_kernels", None) is None:
@@ -699,16 +700,18 @@ class Sm100Backend(OracleBackend):
         return self._optim_kernels
 
     def embedding(self, ids, w):
-        return EmbeddingFn.apply(ids.contiguous(), w)
+        self._pass = _ForwardPass()                  # a forward pass begins here, or with the first layer of its stage
+        return EmbeddingFn.apply(ids.contiguous(), w, self._pass)
 
     def rmsnorm(self, x):
         return RMSNormFn.apply(x.contiguous(), self.eps)
 
     def _chain(self, i):
-        # layers are visited in order within one forward pass: index 0 opens a new x0-gradient chain
-        if i == 0 or self._x0_chain is None:
-            self._x0_chain = _X0GradChain()
-        return self._x0_chain
+        # layers are visited in order within one forward pass
+        if self._pass is None or (i == 0 and self._pass.in_layers):
+            self._pass = _ForwardPass()
+        self._pass.in_layers = True
+        return self._pass
 
     def resid_scale_norm(self, x, x0, lam_r, lam_0, i):
         return ResidScaleNormFn.apply(x.contiguous(), x0.contiguous(), lam_r, lam_0, i, self.eps, self._chain(i))
@@ -774,7 +777,7 @@ class Sm100Backend(OracleBackend):
         if cfg.head_dim != 128:
             raise ValueError("the sm100 kernels support head_dim = 128 only")
         qkv = AttnPreFn.apply(xn, blk.wqkv, ids_flat, blk.ve, blk.ve_gate, cos, sin, T, H, cfg.ve_gate_ch, self.eps,
-                              fused_tp)
+                              fused_tp, self._pass)
         fn = AttentionFn if self.attn == "own" else LibraryAttentionFn
         return fn.apply(qkv, B, T, H, window)
 

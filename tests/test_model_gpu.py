@@ -148,3 +148,119 @@ def test_captured_pass_follows_its_inputs():
         for p, g in zip(mod.parameters(), got[1]):
             assert (p.main_grad - g).norm() <= 1e-3 * p.main_grad.norm() + 1e-9
     K.check_err_flag()
+
+
+class _TrainingPass:
+    """A small model with value embeddings in half of its layers and fp32 main gradients; ``run`` is one forward and backward pass
+    on the staged ids."""
+
+    def __init__(self, seed=5):
+        from autoresearch_b200.config import model_preset
+        self.cfg = model_preset("small")
+        torch.manual_seed(seed)
+        self.mod = _build("sm100", self.cfg, torch.bfloat16)
+        for p in self.mod.parameters():
+            p.main_grad = torch.zeros(p.shape, dtype=torch.float32, device="cuda")
+        self.ids, self.tgt = self.batch(), self.batch()
+
+    def batch(self):
+        return torch.randint(0, self.cfg.vocab, (2, 200), device="cuda", dtype=torch.int32)
+
+    def run(self):
+        for p in self.mod.parameters():
+            p.main_grad.zero_()
+        loss, _ = self.mod(self.ids, self.tgt, grad_scale=1.0 / self.ids.numel())
+        loss.backward()
+
+    def embedding_grads(self):
+        names = {n: p.main_grad for n, p in self.mod.named_parameters() if n == "wte" or n.endswith(".ve")}
+        assert len(names) > 1
+        return {n: g.clone() for n, g in names.items()}
+
+
+def _assert_same_embedding_grads(got, want):
+    for n in want:      # their sums have a fixed order; what they sum differs by the order of split-K sums below
+        assert (got[n] - want[n]).norm() <= 1e-3 * want[n].norm() + 1e-9, n
+
+
+def test_direct_pass_on_the_capture_stream_does_not_take_the_captured_plan():
+    """Capture on an explicit stream, then the same pass directly on that stream, ids untouched, before any replay: every captured
+    or direct pass makes one plan of its own, shared by the word and the value embeddings."""
+    from autoresearch_b200.ops import kernels as K
+    t = _TrainingPass()
+    side = torch.cuda.Stream()
+    made, make = [], K._embedding_plan
+    K._embedding_plan = lambda ids, vocab: made.append(torch.cuda.is_current_stream_capturing()) or make(ids, vocab)
+    try:
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            t.run()
+            want = t.embedding_grads()
+            graph = torch.cuda.CUDAGraph()
+            graph.capture_begin()
+            t.run()
+            graph.capture_end()
+            t.run()
+            got = t.embedding_grads()
+            graph.replay()
+            replayed = t.embedding_grads()
+        side.synchronize()
+    finally:
+        K._embedding_plan = make
+    assert made == [False, True, False]
+    assert len(K._emb_plan) == 0
+    _assert_same_embedding_grads(got, want)
+    _assert_same_embedding_grads(replayed, want)
+    K.check_err_flag()
+
+
+def test_direct_pass_after_a_replay_that_refills_the_ids():
+    """The captured pass copies its ids in, which raises no version at replay; a direct pass then sees the new ids."""
+    from autoresearch_b200.ops import kernels as K
+    t = _TrainingPass()
+    source = t.ids.clone()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        t.run()
+        graph = torch.cuda.CUDAGraph()
+        graph.capture_begin()
+        t.ids.copy_(source)
+        t.run()
+        graph.capture_end()
+        graph.replay()
+        t.run()
+        source.copy_(t.batch())
+        graph.replay()
+        replayed = t.embedding_grads()
+        t.run()
+        got = t.embedding_grads()
+        t.ids = t.ids.clone()
+        t.run()
+        want = t.embedding_grads()
+    side.synchronize()
+    _assert_same_embedding_grads(replayed, want)
+    _assert_same_embedding_grads(got, want)
+    K.check_err_flag()
+
+
+def test_two_streams_with_one_set_of_ids():
+    """Passes of two models on the same ids, queued on two streams without waiting for each other."""
+    from autoresearch_b200.ops import kernels as K
+    a, b = _TrainingPass(5), _TrainingPass(6)
+    b.ids, b.tgt = a.ids, a.tgt
+    want = []
+    for t in (a, b):
+        t.run()
+        want.append(t.embedding_grads())
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+    for _ in range(3):
+        for t, s in zip((a, b), streams):
+            with torch.cuda.stream(s):
+                t.run()
+    torch.cuda.synchronize()
+    for t, w in zip((a, b), want):
+        _assert_same_embedding_grads(t.embedding_grads(), w)
+    K.check_err_flag()
