@@ -42,6 +42,20 @@ def _acc_weight_grad(w, dy, x):
     return tmp.to(w.dtype)
 
 
+def _grad_buffer(p):
+    """(dense fp32 buffer of p's shape for kernels that are given a pointer only, main gradient that takes it up afterwards or None).
+    What the GEMM takes as its output is taken here: fp32 rows at any stride."""
+    mg = _main_grad(p)
+    if mg is None:
+        return torch.zeros(p.shape, dtype=torch.float32, device=p.device), None
+    dense = mg.is_contiguous()
+    if mg.dtype is not torch.float32 or mg.shape != p.shape or mg.device != p.device or not (dense or mg.stride(-1) == 1):
+        raise ValueError(f"main_grad of a {tuple(p.shape)} parameter must be fp32 of that shape with unit inner stride")
+    if dense:
+        return mg, None
+    return torch.zeros(p.shape, dtype=torch.float32, device=p.device), mg
+
+
 class LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w):
@@ -434,8 +448,8 @@ def _layer_backward(ctx, g, g_xn):
         K.flush_pending_pulls()
     g, g_xn = (t.contiguous() if t is not None else None for t in (g, g_xn))
     params = (lam_r, lam_0, wqkv, wo, wfc, wdn, gate_w)
-    mains = [_main_grad(p) if p is not None else None for p in params]
-    accs = [m if m is not None or p is None else torch.zeros(p.shape, dtype=torch.float32, device=dev) for m, p in zip(mains, params)]
+    bufs = [_grad_buffer(p) if p is not None else (None, None) for p in params]
+    accs = [b for b, _ in bufs]
     wide = M + 4 * D if group else max(M, 4 * D)
     work = torch.empty(N * (wide + 2 * D + gate_ch) + 8 + 2 * ((N * H + 3) // 4 * 8), dtype=torch.bfloat16, device=dev)
     dx = torch.empty_like(x)
@@ -458,7 +472,10 @@ def _layer_backward(ctx, g, g_xn):
         dx0 = None              # still being summed; layer 0 of the stage returns it
     else:
         chain.buf = None
-    gp = [None if m is not None or p is None else a.to(p.dtype) for m, a, p in zip(mains, accs, params)]
+    for a, m in bufs:
+        if m is not None:
+            m.add_(a)
+    gp = [None if p is None or _main_grad(p) is not None else a.to(p.dtype) for a, p in zip(accs, params)]
     return dx, dx0, gp[:6], g_ve, gp[6]
 
 
