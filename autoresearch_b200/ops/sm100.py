@@ -650,8 +650,8 @@ class OptimKernels:
         if min(m, n) < self.MIN_GEMM_DIM or pv.dtype != torch.bfloat16 or (m % 8) or (n % 8):
             if isinstance(grad, PeerGrad):
                 raise RuntimeError("small Muon groups take the unfused path: reduce them first")
-            if (pv.dtype == torch.bfloat16 and grad.dtype == torch.float32 and min(m, n) <= 64 and m * n <= 16384 and ns_steps <= 5 and
-                    all(t.is_contiguous() for t in (grad, pv, *st.values()))):
+            if (pv.dtype == torch.bfloat16 and min(m, n) <= 64 and m * n <= 16384 and ns_steps <= 5 and grad.numel() and pv.is_contiguous() and
+                    all(t.dtype == torch.float32 and t.is_contiguous() and t.device == pv.device for t in (grad, *st.values()))):
                 abc = (C.c_float * 15)(*[c for step in MA.POLAR_EXPRESS for c in step])
                 K._check(K.lib().arb_muon_small(st["momentum"].data_ptr(), grad.data_ptr(), st["second"].data_ptr(),
                                                 st["master"].data_ptr(), pv.data_ptr(), G, m, n, mu, lr, wd, beta2, abc,
