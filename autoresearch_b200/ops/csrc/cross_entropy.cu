@@ -92,11 +92,10 @@ extern "C" int arb_softcap_ce(void* logits, long long ld, const int* targets, fl
   const int vpt = (nch + CE_THREADS - 1) / CE_THREADS;
   __nv_bfloat16* p = reinterpret_cast<__nv_bfloat16*>(logits);
   const bool early = rows * V * 2 <= EARLY_BYTES;
-  if (vpt <= 1) launch_dependent(early, softcap_ce_k<1>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
-  else if (vpt <= 2) launch_dependent(early, softcap_ce_k<2>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
-  else if (vpt <= 4) launch_dependent(early, softcap_ce_k<4>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
-  else if (vpt <= 8) launch_dependent(early, softcap_ce_k<8>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
-  else if (vpt <= 16) launch_dependent(early, softcap_ce_k<16>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
+  if (vpt <= 1) return launch_dependent(early, softcap_ce_k<1>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
+  else if (vpt <= 2) return launch_dependent(early, softcap_ce_k<2>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
+  else if (vpt <= 4) return launch_dependent(early, softcap_ce_k<4>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
+  else if (vpt <= 8) return launch_dependent(early, softcap_ce_k<8>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
+  else if (vpt <= 16) return launch_dependent(early, softcap_ce_k<16>, unsigned(rows), CE_THREADS, 0, s, p, ld, targets, loss, V, softcap, dlogits_scale);
   else return -3;  // vocabularies above 32768 are not supported by this kernel
-  return int(cudaGetLastError());
 }

@@ -742,11 +742,11 @@ static inline int grid_for(long long n, int threads, int cap = 148 * 16) {
 #define ROW_DISPATCH(KERNEL, ...)                                                        \
   do {                                                                                     \
     const int blocks = int((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA);                      \
-    if (D <= 256) launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<1>, blocks, 256, 0, s, __VA_ARGS__);                           \
-    else if (D <= 512) launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<2>, blocks, 256, 0, s, __VA_ARGS__);                      \
-    else if (D <= 1024) launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<4>, blocks, 256, 0, s, __VA_ARGS__);                     \
-    else if (D <= 2048) launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<8>, blocks, 256, 0, s, __VA_ARGS__);                     \
-    else launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<16>, blocks, 256, 0, s, __VA_ARGS__);                                   \
+    if (D <= 256) return launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<1>, blocks, 256, 0, s, __VA_ARGS__);                           \
+    else if (D <= 512) return launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<2>, blocks, 256, 0, s, __VA_ARGS__);                      \
+    else if (D <= 1024) return launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<4>, blocks, 256, 0, s, __VA_ARGS__);                     \
+    else if (D <= 2048) return launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<8>, blocks, 256, 0, s, __VA_ARGS__);                     \
+    else return launch_dependent(rows * D * 2 <= EARLY_BYTES, KERNEL<16>, blocks, 256, 0, s, __VA_ARGS__);                                   \
   } while (0)
 
 static inline int check_row_args(long long rows, int D) {
@@ -765,37 +765,33 @@ extern "C" {
 int arb_rmsnorm_fwd(const void* x, void* y, long long rows, int D, float eps, cudaStream_t s) {
   if (check_row_args(rows, D) || misaligned(x) || misaligned(y)) return -3;
   ROW_DISPATCH(rmsnorm_fwd_k, (const bf16*)x, (bf16*)y, rows, D, eps);
-  return int(cudaGetLastError());
 }
 int arb_rmsnorm_bwd(const void* x, const void* g, const void* add_to, void* gx, long long rows, int D, float eps, cudaStream_t s) {
   if (check_row_args(rows, D) || misaligned(x) || misaligned(g) || misaligned(gx) || misaligned(add_to)) return -3;
   ROW_DISPATCH(rmsnorm_bwd_k, (const bf16*)x, (const bf16*)g, (const bf16*)add_to, (bf16*)gx, rows, D, eps);
-  return int(cudaGetLastError());
 }
 int arb_resid_scale_norm_fwd(const void* x, const void* x0, const void* lam_r, const void* lam_0, int idx, void* x_out,
                              void* xn_out, long long rows, int D, float eps, cudaStream_t s) {
   if (check_row_args(rows, D) || misaligned(x) || misaligned(x0) || misaligned(x_out) || misaligned(xn_out)) return -3;
 #define RSN(NV) resid_norm_fwd_k<NV, true>
   const int blocks = int((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA);
-  if (D <= 256) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(1), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 512) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(2), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 1024) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(4), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 2048) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(8), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(16), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  if (D <= 256) return launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(1), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 512) return launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(2), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 1024) return launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(4), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 2048) return launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(8), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else return launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(16), blocks, 256, 0, s, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
 #undef RSN
-  return int(cudaGetLastError());
 }
 int arb_add_norm_fwd(const void* x, const void* proj, void* x_out, void* xn_out, long long rows, int D, float eps, cudaStream_t s) {
   if (check_row_args(rows, D) || misaligned(x) || misaligned(proj) || misaligned(x_out) || misaligned(xn_out)) return -3;
 #define RSN(NV) resid_norm_fwd_k<NV, false>
   const int blocks = int((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA);
-  if (D <= 256) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(1), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 512) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(2), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 1024) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(4), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else if (D <= 2048) launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(8), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
-  else launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(16), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  if (D <= 256) return launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(1), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 512) return launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(2), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 1024) return launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(4), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else if (D <= 2048) return launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(8), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
+  else return launch_dependent(rows * D * 2 <= EARLY_BYTES, RSN(16), blocks, 256, 0, s, (const bf16*)x, (const bf16*)proj, nullptr, nullptr, 0, (bf16*)x_out, (bf16*)xn_out, rows, D, eps);
 #undef RSN
-  return int(cudaGetLastError());
 }
 int arb_resid_scale_norm_bwd(const void* x, const void* x0, const void* lam_r, const void* lam_0, int idx, const void* g_xs,
                              const void* g_xn, void* d_x, void* d_x0, const void* d_x0_acc, float* dlam_r, float* dlam_0,
@@ -805,12 +801,10 @@ int arb_resid_scale_norm_bwd(const void* x, const void* x0, const void* lam_r, c
     return -3;
   ROW_DISPATCH(resid_norm_bwd_k, (const bf16*)x, (const bf16*)x0, (const bf16*)lam_r, (const bf16*)lam_0, idx, (const bf16*)g_xs,
                (const bf16*)g_xn, (bf16*)d_x, (bf16*)d_x0, (const bf16*)d_x0_acc, dlam_r, dlam_0, rows, D, eps);
-  return int(cudaGetLastError());
 }
 int arb_residual_add(const void* a, const void* b, void* out, long long n, cudaStream_t s) {
   if (n <= 0 || (n & 7) || misaligned(a) || misaligned(b) || misaligned(out)) return -3;
-  launch_dependent(n * 2 <= EARLY_BYTES, residual_add_k, grid_for(n / 8, 256), 256, 0, s, (const uint4*)a, (const uint4*)b, (uint4*)out, n / 8);
-  return int(cudaGetLastError());
+  return launch_dependent(n * 2 <= EARLY_BYTES, residual_add_k, grid_for(n / 8, 256), 256, 0, s, (const uint4*)a, (const uint4*)b, (uint4*)out, n / 8);
 }
 int arb_relu_sq_fwd(const void* x, void* y, long long n, cudaStream_t s) {
   if (n <= 0 || (n & 7) || misaligned(x) || misaligned(y)) return -3;
@@ -827,19 +821,17 @@ int arb_qkv_post_fwd(void* qkv, const void* cos_t, const void* sin_t, float* rst
                      int gate_ch, float eps, cudaStream_t s) {
   if (N <= 0 || T <= 0 || H <= 0 || misaligned(qkv) || (reinterpret_cast<uintptr_t>(cos_t) & 7) || (reinterpret_cast<uintptr_t>(sin_t) & 7)) return -3;
   if (ve_w && (!gate_w || !gate_out || !xn || !ids || misaligned(ve_w))) return -3;
-  launch_dependent(N * H * 768 <= EARLY_BYTES, qkv_post_fwd_k, int((N + 7) / 8), 256, 0, s, (bf16*)qkv, (const bf16*)cos_t, (const bf16*)sin_t, rstd_qk, (const bf16*)xn, ids,
+  return launch_dependent(N * H * 768 <= EARLY_BYTES, qkv_post_fwd_k, int((N + 7) / 8), 256, 0, s, (bf16*)qkv, (const bf16*)cos_t, (const bf16*)sin_t, rstd_qk, (const bf16*)xn, ids,
                                                       (const bf16*)ve_w, (const bf16*)gate_w, gate_out, N, T, H, D_model, gate_ch, eps);
-  return int(cudaGetLastError());
 }
 int arb_qkv_post_bwd(void* d_qkv, const void* qkv, const void* cos_t, const void* sin_t, const float* rstd_qk, const void* xn,
                      const int* ids, const void* ve_w, const void* gate_w, const float* gate, void* d_ve, float* d_gate_w,
                      void* d_xn_gate, float* dgl, long long N, int T, int H, int D_model, int gate_ch, cudaStream_t s) {
   if (N <= 0 || T <= 0 || H <= 0 || misaligned(d_qkv) || misaligned(qkv)) return -3;
   if (ve_w && (!gate_w || !gate || !xn || !ids || !d_ve || !d_gate_w || !d_xn_gate || !dgl)) return -3;
-  launch_dependent(N * H * 768 <= EARLY_BYTES, qkv_post_bwd_k, int((N + 7) / 8), 256, 0, s, (bf16*)d_qkv, (const bf16*)qkv, (const bf16*)cos_t, (const bf16*)sin_t, rstd_qk,
+  int rc = launch_dependent(N * H * 768 <= EARLY_BYTES, qkv_post_bwd_k, int((N + 7) / 8), 256, 0, s, (bf16*)d_qkv, (const bf16*)qkv, (const bf16*)cos_t, (const bf16*)sin_t, rstd_qk,
                                                       (const bf16*)xn, ids, (const bf16*)ve_w, (const bf16*)gate_w, gate, (bf16*)d_ve,
                                                       dgl, N, T, H);
-  int rc = int(cudaGetLastError());
   if (ve_w) {
     // two slabs per SM, at least 16 tokens each (a slab ends with H * gate_ch atomic adds)
     long long tpc = (N + 295) / 296;
@@ -848,15 +840,15 @@ int arb_qkv_post_bwd(void* d_qkv, const void* qkv, const void* cos_t, const void
     if (chunk > VE_CHUNK) chunk = VE_CHUNK;
     if (chunk < 1) return -3;
     if (chunk > tpc) chunk = int(tpc);
-    launch_dependent(N * gate_ch * 2 <= EARLY_BYTES, ve_gate_bwd_k, unsigned((N + tpc - 1) / tpc), 256, size_t(chunk) * 4 * (gate_ch + H), s, dgl, (const bf16*)xn, (const bf16*)gate_w, d_gate_w, (bf16*)d_xn_gate, N, H, D_model, gate_ch, int(tpc), chunk);
-    if (!rc) rc = int(cudaGetLastError());
+    const int gate_rc = launch_dependent(N * gate_ch * 2 <= EARLY_BYTES, ve_gate_bwd_k, unsigned((N + tpc - 1) / tpc), 256, size_t(chunk) * 4 * (gate_ch + H), s, dgl,
+                                         (const bf16*)xn, (const bf16*)gate_w, d_gate_w, (bf16*)d_xn_gate, N, H, D_model, gate_ch, int(tpc), chunk);
+    if (!rc) rc = gate_rc;
   }
   return rc;
 }
 int arb_embedding_fwd(const int* ids, const void* w, void* out, long long N, int D, int vocab, cudaStream_t s) {
   if (N <= 0 || (D & 7) || misaligned(w) || misaligned(out)) return -3;
-  launch_dependent(N * D * 2 <= EARLY_BYTES, embedding_fwd_k, grid_for(N * (D / 8), 256), 256, 0, s, ids, (const bf16*)w, (bf16*)out, N, D, vocab);
-  return int(cudaGetLastError());
+  return launch_dependent(N * D * 2 <= EARLY_BYTES, embedding_fwd_k, grid_for(N * (D / 8), 256), 256, 0, s, ids, (const bf16*)w, (bf16*)out, N, D, vocab);
 }
 int arb_embedding_bwd(const int* ids, const void* g, float* dw, long long N, int D, int vocab, cudaStream_t s) {
   if (N <= 0 || (D & 7) || misaligned(g) || misaligned(dw)) return -3;
@@ -871,12 +863,10 @@ int arb_embedding_bwd_sorted(const long long* perm, const int* item_id, const in
                              const int* seg_count, const void* g, float* dw, float* partial, int n_items_max, int D, int R,
                              int vocab, cudaStream_t s) {
   if (n_items_max <= 0 || (D & 7) || R <= 0 || vocab <= 0 || misaligned(g) || misaligned(dw) || misaligned(partial)) return -3;
-  launch_dependent((long long)(n_items_max - vocab) * R * D * 2 <= EARLY_BYTES, embedding_bwd_sorted_k, n_items_max, EMB_THREADS, 0, s, perm, item_id, item_start, seg_start, seg_count, (const bf16*)g, dw, partial,
+  const int rc = launch_dependent((long long)(n_items_max - vocab) * R * D * 2 <= EARLY_BYTES, embedding_bwd_sorted_k, n_items_max, EMB_THREADS, 0, s, perm, item_id, item_start, seg_start, seg_count, (const bf16*)g, dw, partial,
                                                      n_items_max, D, R, vocab);
-  int rc = int(cudaGetLastError());
   if (rc) return rc;
-  launch_dependent((long long)(n_items_max - vocab) * D * 4 <= EARLY_BYTES, embedding_bwd_combine_k, vocab, 128, 0, s, item_start, seg_count, partial, dw, D, R);
-  return int(cudaGetLastError());
+  return launch_dependent((long long)(n_items_max - vocab) * D * 4 <= EARLY_BYTES, embedding_bwd_combine_k, vocab, 128, 0, s, item_start, seg_count, partial, dw, D, R);
 }
 int arb_embedding_plan(const int* ids, long long N, int vocab, int R, int n_items_max, int* hist, long long* perm, int* counts,
                        int* seg_start, int* item_start, int* item_id, cudaStream_t s) {
@@ -889,11 +879,11 @@ int arb_embedding_plan(const int* ids, long long N, int vocab, int R, int n_item
     if (e == cudaSuccess) e = cudaFuncSetAttribute(emb_plan_place_k, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_MAX_VOCAB * 4);
     if (e != cudaSuccess) return int(e);
   }
-  launch_dependent(true, emb_plan_hist_k, chunks, 256, smem, s, ids, N, vocab, hist);
-  launch_dependent(true, emb_plan_chunks_k, (vocab + 63) / 64, 64, 0, s, hist, int(chunks), vocab, counts);
-  launch_dependent(true, emb_plan_scan_k, 1, 1024, 0, s, counts, vocab, R, n_items_max, seg_start, item_start, item_id);
-  launch_dependent(true, emb_plan_place_k, chunks, 256, smem, s, ids, N, vocab, hist, seg_start, perm);
-  return int(cudaGetLastError());
+  int rc = launch_dependent(true, emb_plan_hist_k, chunks, 256, smem, s, ids, N, vocab, hist);
+  if (!rc) rc = launch_dependent(true, emb_plan_chunks_k, (vocab + 63) / 64, 64, 0, s, hist, int(chunks), vocab, counts);
+  if (!rc) rc = launch_dependent(true, emb_plan_scan_k, 1, 1024, 0, s, counts, vocab, R, n_items_max, seg_start, item_start, item_id);
+  if (!rc) rc = launch_dependent(true, emb_plan_place_k, chunks, 256, smem, s, ids, N, vocab, hist, seg_start, perm);
+  return rc;
 }
 int arb_capture_id(unsigned long long* id, cudaStream_t s) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
@@ -905,8 +895,7 @@ int arb_capture_id(unsigned long long* id, cudaStream_t s) {
 }
 int arb_add_cols(void* dst, long long ld_dst, const void* src, long long rows, int cols, cudaStream_t s) {
   if (rows <= 0 || cols <= 0) return -3;
-  launch_dependent(rows * cols * 2 <= EARLY_BYTES, add_cols_k, grid_for(rows * cols, 256), 256, 0, s, (bf16*)dst, ld_dst, (const bf16*)src, rows, cols);
-  return int(cudaGetLastError());
+  return launch_dependent(rows * cols * 2 <= EARLY_BYTES, add_cols_k, grid_for(rows * cols, 256), 256, 0, s, (bf16*)dst, ld_dst, (const bf16*)src, rows, cols);
 }
 int arb_cast_f32_to_bf16(const float* src, void* dst, long long n, float scale, cudaStream_t s) {
   if (n <= 0 || (n & 3) || misaligned(src) || (reinterpret_cast<uintptr_t>(dst) & 7)) return -3;

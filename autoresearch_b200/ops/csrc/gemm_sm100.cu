@@ -1138,7 +1138,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
   pair_launch_config(cfg, attr, clusters, Smem2<EPI>::TOTAL, st);
   GemmArgs args = a;
   if (int r = arm_pull(args, clusters * 2)) return r;
-  return int(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tx, args));
+  return launch_status(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tx, args));
 }
 
 template <bool A_MN, bool B_MN>
@@ -1248,7 +1248,7 @@ extern "C" int arb_gemm_dw_group(const void* const* dy, const void* const* x, fl
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   pair_launch_config(cfg, attr, clusters, SMEM, stream);
-  return int(cudaLaunchKernelEx(&cfg, gemm_dw_group_kernel, maps, a));
+  return launch_status(cudaLaunchKernelEx(&cfg, gemm_dw_group_kernel, maps, a));
 }
 
 extern "C" int arb_gemm_set_mode(int mode) {

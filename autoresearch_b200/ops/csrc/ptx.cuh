@@ -80,6 +80,12 @@ __device__ __forceinline__ void grid_enter() { grid_trigger(); grid_wait(); }
 // bytes in flight for HBM (119.5 M model, 64 x 2048 tokens, 134 MB per tensor: training pass 133.3 -> 134.7 ms with the early
 // start everywhere; 1 x 2048 tokens: 7.90 -> 6.96).
 constexpr long long EARLY_BYTES = 48ll << 20;
+// The code of a launch, which then leaves nothing behind: the runtime also keeps it as the thread's last error, and the next entry
+// point that asks for the status of its own launch would report it.
+inline int launch_status(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return int(e);
+}
 template <typename... Formal, typename... Actual>
 inline int launch_dependent(bool early, void (*kern)(Formal...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Actual&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -92,7 +98,7 @@ inline int launch_dependent(bool early, void (*kern)(Formal...), dim3 grid, dim3
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = early ? 1 : 0;
-  return int(cudaLaunchKernelEx(&cfg, kern, static_cast<Formal>(args)...));
+  return launch_status(cudaLaunchKernelEx(&cfg, kern, static_cast<Formal>(args)...));
 }
 
 // ---- TMA -------------------------------------------------------------------------------

@@ -46,3 +46,11 @@ def test_no_read_only_loads_where_early_started_kernels_live():
     for name, text in _sources():
         if re.search(r"\bgrid_(enter|wait)\s*\(", text):
             assert not re.findall(r"__ldg\s*\(|\.nc\b", text), name
+
+
+def test_no_launch_leaves_its_error_for_the_next_entry_point():
+    """cudaLaunchKernelEx returns its error and leaves it as the thread's last one: every such launch goes through launch_status(), and
+    no entry point asks for the last error after one."""
+    for name, text in _sources():
+        assert len(re.findall(r"\bcudaLaunchKernelEx\(", text)) == len(re.findall(r"\blaunch_status\(cudaLaunchKernelEx\(", text)), name
+        assert not re.findall(r"[;{})]\s*launch_dependent\(", text), name            # its code is used

@@ -357,3 +357,16 @@ def test_kernels_are_bitwise_reproducible_and_stay_inside_their_outputs():
     assert torch.equal(y1, y2)
     torch.cuda.synchronize()
     K.check_err_flag()
+
+
+def test_a_refused_launch_does_not_fail_the_next_call():
+    """More blocks than a grid can have (the runtime refuses them on the host, nothing starts), then a call that is in order."""
+    from autoresearch_b200.ops import kernels as K
+    x = _bf(16, 128)
+    p, err = x.data_ptr(), K.err_flag(x.device).data_ptr()
+    B, T = 65535, 262152                                    # delta rows: B * T / 8 blocks
+    assert (B * T + 7) // 8 > 2 ** 31 - 1
+    rc = K.lib().arb_attn_bwd(*[p] * 11, B, T, 1, *[128] * 8, T, 1.0, err, K._stream())
+    assert rc != 0
+    _close(K.relu_sq_fwd(x), torch.relu(x.float()) ** 2)
+    _close(K.residual_add(x, x), 2 * x.float())
