@@ -116,14 +116,14 @@ class GPT(nn.Module):
                 x.register_hook(lambda g, cb=cb, b=b: cb(b))
             with nvtx_range(f"layer {l}"):
                 one_call = whole_layer if blk.router is None else first_half
-                if one_call is not None:
-                    y = one_call(x, x0, self.resid_lambdas, self.x0_lambdas, bi, blk, ids_flat, B, T, cfg, self.rope_cos,
-                                 self.rope_sin, cfg.window(l))
-                    if y is not None and blk.router is None:
-                        x = y
-                        continue
-                if one_call is not None and y is not None:
+                y = one_call(x, x0, self.resid_lambdas, self.x0_lambdas, bi, blk, ids_flat, B, T, cfg, self.rope_cos, self.rope_sin,
+                             cfg.window(l)) if one_call is not None else None
+                if y is not None and blk.router is None:
+                    x = y
+                    continue
+                if y is not None:
                     x, xn = y
+                    del y                    # the next layer's call would still hold this layer's tensors
                 else:
                     x, xn = be.resid_scale_norm(x, x0, self.resid_lambdas, self.x0_lambdas, bi)
                     a = be.attention_block(xn, blk, ids_flat, B, T, cfg, self.rope_cos, self.rope_sin,

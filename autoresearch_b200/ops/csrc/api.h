@@ -262,11 +262,12 @@ typedef struct {
   void *work, *d_x, *d_x0;
   const void* d_x0_acc;
   void *g_lam_r, *g_lam_0, *g_wqkv, *g_wo, *g_wfc, *g_wdn, *g_gate;
-  long long B, T, H, M, window, idx, gate_ch, fuse_post, group_dw, half;
+  long long B, T, H, M, window, idx, gate_ch, fuse_post, group_dw, half, scoring;
   double eps, scale;
 } ArbLayer;
 // half: the layer up to its second norm (what comes before the experts of an expert layer): out = the residual stream, out2 = its
 // norm, M = 0, kept without their copies; backward: out as input, g and g_xn their gradients (either may be null, not both).
+// scoring: no backward call follows; kept is then scratch of max(5 D and the statistics, 2 D + M) columns.
 int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s);
 int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s);
 

@@ -18,11 +18,18 @@ namespace {
 struct Kept {
   char *xs, *xn, *qkv, *att, *xs2, *xn2, *act;
   float *lse, *rstd, *gate;
-  Kept(void* base, long long N, long long D, long long M, long long H, bool half) {
+  Kept(void* base, long long N, long long D, long long M, long long H, bool half, bool scoring) {
     char* p = static_cast<char*>(base);
     auto take = [&](long long cols) { char* q = p; p += N * cols * 2; return q; };
-    xs = take(D); xn = take(D); qkv = take(3 * D); att = take(D);
-    xs2 = take(half ? 0 : D); xn2 = take(half ? 0 : D); act = take(half ? 0 : M);
+    if (scoring) {
+      // no backward pass follows: q|k|v 3 D, xs D, xn D and, over it when the projection has read it, the attention's output; what
+      // comes behind the attention lies over what is dead by then
+      qkv = take(3 * D); xs = take(D); xn = att = take(D);
+      xs2 = qkv; xn2 = xs2 + N * D * 2; act = xn2 + N * D * 2;
+    } else {
+      xs = take(D); xn = take(D); qkv = take(3 * D); att = take(D);
+      xs2 = take(half ? 0 : D); xn2 = take(half ? 0 : D); act = take(half ? 0 : M);
+    }
     const long long nh = (N * H + 3) / 4 * 4;
     lse = reinterpret_cast<float*>(p); rstd = lse + nh; gate = rstd + 2 * nh;
   }
@@ -56,7 +63,7 @@ extern "C" int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s
   const ArbLayer& a = *args;
   if (bad_sizes(a) || !a.kept || !a.out || (a.half && !a.out2)) return -3;
   const long long N = a.B * a.T, D = a.H * 128;
-  const Kept k(a.kept, N, D, a.M, a.H, a.half);
+  const Kept k(a.kept, N, D, a.M, a.H, a.half, a.scoring);
   const Gemm g{static_cast<int*>(a.err), s};
   const float eps = float(a.eps);
   const int* ids = static_cast<const int*>(a.ids);
@@ -91,9 +98,9 @@ extern "C" int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s
 // On return the value embedding's row gradients [N, D] lie behind the first 3 N D elements.
 extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s) {
   const ArbLayer& a = *args;
-  if (bad_sizes(a) || !a.kept || !a.work || !a.d_x || !a.d_x0 || (a.half ? !a.out || (!a.g && !a.g_xn) : !a.g)) return -3;
+  if (bad_sizes(a) || !a.kept || !a.work || !a.d_x || !a.d_x0 || a.scoring || (a.half ? !a.out || (!a.g && !a.g_xn) : !a.g)) return -3;
   const long long N = a.B * a.T, D = a.H * 128;
-  const Kept k(a.kept, N, D, a.M, a.H, a.half);
+  const Kept k(a.kept, N, D, a.M, a.H, a.half, false);
   const Gemm g{static_cast<int*>(a.err), s};
   const float eps = float(a.eps);
   const int* ids = static_cast<const int*>(a.ids);

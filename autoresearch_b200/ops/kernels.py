@@ -307,7 +307,7 @@ def flush_pending_pulls() -> None:
     _check(lib().arb_pull_ranges(src, dst, nb, n, _stream()), "pull_ranges")
 
 
-_LAYER = struct.Struct("=40q2d")        # ArbLayer of csrc/api.h: 30 pointers, 10 sizes, eps and scale
+_LAYER = struct.Struct("=41q2d")        # ArbLayer of csrc/api.h: 30 pointers, 11 sizes, eps and scale
 
 
 def layer_call(entry: str, pointers, sizes, eps: float, scale: float) -> None:

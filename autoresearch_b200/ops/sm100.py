@@ -420,27 +420,30 @@ class AttentionFn(torch.autograd.Function):
 GROUP_DW_FLOPS = 6e10
 
 
-def _layer_forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, B, T, window, idx, gate_ch, eps, chain, out2):
+def _layer_forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, B, T, window, idx, gate_ch, eps, chain, scoring, out2):
     """Forward launches of a layer, or with ``out2`` (and no MLP matrices) of its half up to the second norm."""
     N, D = x.shape
     half = out2 is not None
     M, H = 0 if half else wfc.shape[0], D // 128
     stat = (N * H + 3) // 4 * 8                            # fp32 [N, H] in bf16 elements; lse, rstd of q and k, gate
-    kept = torch.empty(N * ((6 if half else 8) * D + M) + 4 * stat, dtype=torch.bfloat16, device=x.device)
+    # without a backward pass the parts lie over each other (csrc/layer.cu): as much as the separate steps hold at their peak
+    cells = max(5 * N * D + 4 * stat, 2 * N * D + N * M) if scoring else N * ((6 if half else 8) * D + M) + 4 * stat
+    kept = torch.empty(cells, dtype=torch.bfloat16, device=x.device)
     out = torch.empty_like(x)
     group = int(2 * N * D * (4 * D + 2 * M) <= GROUP_DW_FLOPS)
-    sizes = (B, T, H, M, window, idx, gate_ch, int(K.qkv_post_fusable(N, 3 * D)), group, int(half))
+    sizes = (B, T, H, M, window, idx, gate_ch, int(K.qkv_post_fusable(N, 3 * D)), group, int(half), int(scoring))
     ptrs = [t.data_ptr() if t is not None else 0 for t in (x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin)]
     ptrs += (kept.data_ptr(), out.data_ptr(), out2.data_ptr() if half else 0, K.err_flag(x.device).data_ptr())
     K.layer_call("arb_layer_fwd", ptrs + [0] * 13, sizes, eps, 1.0 / math.sqrt(128.0))
-    ctx.save_for_backward(x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept, out if half else None)
-    ctx.sizes, ctx.eps, ctx.chain = sizes, eps, chain
+    if not scoring:
+        ctx.save_for_backward(x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept, out if half else None)
+        ctx.sizes, ctx.eps, ctx.chain = sizes, eps, chain
     return out
 
 
 def _layer_backward(ctx, g, g_xn):
     x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin, kept, out = ctx.saved_tensors
-    B, T, H, M, _, idx, gate_ch, _, group, half = ctx.sizes
+    B, T, H, M, _, idx, gate_ch, _, group, half, _ = ctx.sizes
     chain = ctx.chain
     N, D = x.shape
     dev = x.device
@@ -491,7 +494,7 @@ class DenseLayerFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         dx, dx0, gp, g_ve, g_gate = _layer_backward(ctx, g, None)
-        return (dx, dx0, *gp, g_ve, g_gate) + (None,) * 10
+        return (dx, dx0, *gp, g_ve, g_gate) + (None,) * 11
 
 
 class AttentionHalfFn(torch.autograd.Function):
@@ -505,7 +508,7 @@ class AttentionHalfFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_xs, g_xn):
         dx, dx0, gp, g_ve, g_gate = _layer_backward(ctx, g_xs, g_xn)
-        return (dx, dx0, *gp[:4], g_ve, g_gate) + (None,) * 10
+        return (dx, dx0, *gp[:4], g_ve, g_gate) + (None,) * 11
 
 
 class LibraryAttentionFn(torch.autograd.Function):
@@ -756,19 +759,26 @@ class Sm100Backend(OracleBackend):
         return (N == B * T and D % 128 == 0 and cfg.head_dim == 128 and cos.shape[0] >= T and ids_flat.dtype is torch.int32 and
                 ids_flat.shape == (N,) and ids_flat.device == dev and ids_flat.is_contiguous() and x.is_cuda)
 
+    @staticmethod
+    def _scoring(*inputs):
+        """No backward pass can follow a call on these inputs."""
+        return not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in inputs))
+
     def dense_layer(self, x, x0, lam_r, lam_0, i, blk, ids_flat, B, T, cfg, cos, sin, window):
         """A dense layer through DenseLayerFn: its output, or None where its steps have to run one by one."""
         if blk.router is not None or not self._one_call(x, x0, lam_r, lam_0, blk, ids_flat, B, T, cfg, cos, sin):
             return None
         return DenseLayerFn.apply(x, x0, lam_r, lam_0, blk.wqkv, blk.wo, blk.wfc, blk.wdn, blk.ve, blk.ve_gate, ids_flat, cos, sin,
-                                  B, T, window, i, cfg.ve_gate_ch, self.eps, self._chain(i))
+                                  B, T, window, i, cfg.ve_gate_ch, self.eps, self._chain(i),
+                                  self._scoring(x, x0, lam_r, lam_0, blk.wqkv, blk.wo, blk.wfc, blk.wdn, blk.ve, blk.ve_gate))
 
     def attention_half(self, x, x0, lam_r, lam_0, i, blk, ids_flat, B, T, cfg, cos, sin, window):
         """An expert layer up to the input of its experts: (residual stream, its norm), or None as in dense_layer."""
         if blk.router is None or not self._one_call(x, x0, lam_r, lam_0, blk, ids_flat, B, T, cfg, cos, sin):
             return None
         return AttentionHalfFn.apply(x, x0, lam_r, lam_0, blk.wqkv, blk.wo, blk.ve, blk.ve_gate, ids_flat, cos, sin,
-                                     B, T, window, i, cfg.ve_gate_ch, self.eps, self._chain(i))
+                                     B, T, window, i, cfg.ve_gate_ch, self.eps, self._chain(i),
+                                     self._scoring(x, x0, lam_r, lam_0, blk.wqkv, blk.wo, blk.ve, blk.ve_gate))
 
     def linear_col(self, x, w):
         return LinearFn.apply(x, w)

@@ -34,7 +34,7 @@ def call(monkeypatch):
             ps[n].main_grad = m
         x, aux = torch.zeros(N, D, dtype=torch.bfloat16), torch.zeros(64, dtype=torch.bfloat16)
         ctx = SimpleNamespace(saved_tensors=(x, x, *ps.values(), None, None, None, aux, aux, aux, None), eps=1e-5,
-                              sizes=(1, N, 1, M, N, 0, 32, 0, 1, 0), chain=SimpleNamespace(buf=None))
+                              sizes=(1, N, 1, M, N, 0, 32, 0, 1, 0, 0), chain=SimpleNamespace(buf=None))
         return dict(zip(PARAMS, sm100._layer_backward(ctx, x, None)[2]))
     return backward
 

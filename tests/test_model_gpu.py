@@ -264,3 +264,31 @@ def test_two_streams_with_one_set_of_ids():
     for t, w in zip((a, b), want):
         _assert_same_embedding_grads(t.embedding_grads(), w)
     K.check_err_flag()
+
+
+@pytest.mark.parametrize("heads,mlp,experts", [(2, 1024, 0), (3, 768, 0), (1, 1024, 0), (2, 1024, 4)])
+def test_scoring_pass_holds_no_more_memory_than_the_separate_steps(heads, mlp, experts):
+    """Peak of the layers of a pass without gradients, whole-layer calls against one call per step, and the same bits: MLPs of four,
+    two and eight widths, and experts.  The row statistics lie over the MLP part unless that is narrow: 16 bytes a row and head."""
+    from autoresearch_b200.config import ModelConfig, MoEConfig
+    moe = MoEConfig(n_experts=experts, top_k=2, mlp_dim_e=mlp, capacity_factor=1.25) if experts else None
+    cfg = ModelConfig(vocab=512, seq_len=2048, d_model=128 * heads, n_head=heads, head_dim=128, mlp_dim=mlp, n_layer=3, moe=moe)
+    torch.manual_seed(7)
+    mod = _build("sm100", cfg, torch.bfloat16)
+    B, T = 8, 2048
+    ids = torch.randint(0, cfg.vocab, (B, T), device="cuda", dtype=torch.int32)
+    peak, out = {}, {}
+    with torch.no_grad():
+        x = mod.embed(ids)
+        for whole in (True, False):
+            mod.backend.layer_calls = whole
+            for _ in range(2):                   # first pass: lazily made buffers
+                torch.cuda.synchronize()
+                torch.cuda.reset_peak_memory_stats()
+                before = torch.cuda.memory_allocated()
+                out[whole] = None
+                out[whole] = mod.run_layers(x, x, ids, B, T)
+                torch.cuda.synchronize()
+                peak[whole] = torch.cuda.max_memory_allocated() - before
+    assert torch.equal(out[True], out[False])
+    assert peak[True] <= peak[False] + 16 * B * T * heads + (1 << 21), peak
