@@ -123,7 +123,8 @@ int arb_rmsnorm_bwd(const void* x, const void* g, const void* add_to, void* gx, 
 int arb_resid_scale_norm_fwd(const void* x, const void* x0, const void* lam_r, const void* lam_0, int idx,
                              void* x_out, void* xn_out, long long rows, int D, float eps, cudaStream_t s);
 // t = g_xs + rmsnorm_bwd(x', g_xn);  d_x = lam_r*t;  d_x0 = lam_0*t (+ d_x0_acc when given; it may be d_x0 itself);
-// dlam_r[idx] += sum(x*t);  dlam_0[idx] += sum(x0*t)   (fp32 atomics, one per CTA)
+// dlam_r[idx] += sum(x*t);  dlam_0[idx] += sum(x0*t)   (fp32 atomics, one per CTA).  d_x may be g_xn: a thread reads its part of a row
+// before it writes it.
 int arb_resid_scale_norm_bwd(const void* x, const void* x0, const void* lam_r, const void* lam_0, int idx,
                              const void* g_xs, const void* g_xn, void* d_x, void* d_x0, const void* d_x0_acc,
                              float* dlam_r, float* dlam_0, long long rows, int D, float eps, cudaStream_t s);
@@ -253,7 +254,7 @@ int arb_moe_combine_bwd(const void* d_out, void* const* y_bufs, const void* y_ro
 
 // ---- one dense layer per call (layer.cu): the same kernels as the entry points above, started from native code ----
 typedef struct {
-  // forward: inputs, parameters, the buffer for what the layer keeps (bf16 [N, 8 D + M] then four times
+  // forward: inputs, parameters, the buffer for what the layer keeps (bf16 [N, 7 D + M] then four times
   // fp32 [N, H], each rounded up to 4 floats), output [N, D]
   const void *x, *x0, *lam_r, *lam_0, *wqkv, *wo, *wfc, *wdn, *ve, *gate_w, *ids, *cos_t, *sin_t;
   void *kept, *out, *out2, *err;
@@ -267,7 +268,7 @@ typedef struct {
 } ArbLayer;
 // half: the layer up to its second norm (what comes before the experts of an expert layer): out = the residual stream, out2 = its
 // norm, M = 0, kept without their copies; backward: out as input, g and g_xn their gradients (either may be null, not both).
-// scoring: no backward call follows; kept is then scratch of max(5 D and the statistics, 2 D + M) columns.
+// scoring: no backward call follows; kept is then scratch of max(4 D and the statistics, 2 D + M) columns.
 int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s);
 int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s);
 

@@ -14,23 +14,26 @@ namespace {
 
 // The activations that a layer keeps, carved out of one buffer (bf16 [N, cols] each, then the fp32 row statistics).
 // N * D is a multiple of 128 elements, so every bf16 part starts on a 256-byte boundary; the statistics are padded to four
-// floats each, because the kernels read them as pairs.
+// floats each, because the kernels read them as pairs.  The layer's input after scaling, xs, is read by the output projection and by
+// nothing later (the backward pass forms it again from x and x0): it lies where an output of the call is written last.
 struct Kept {
   char *xs, *xn, *qkv, *att, *xs2, *xn2, *act;
   float *lse, *rstd, *gate;
-  Kept(void* base, long long N, long long D, long long M, long long H, bool half, bool scoring) {
-    char* p = static_cast<char*>(base);
+  explicit Kept(const ArbLayer& a) {
+    const long long N = a.B * a.T, D = a.H * 128;
+    char* p = static_cast<char*>(a.kept);
     auto take = [&](long long cols) { char* q = p; p += N * cols * 2; return q; };
-    if (scoring) {
-      // no backward pass follows: q|k|v 3 D, xs D, xn D and, over it when the projection has read it, the attention's output; what
-      // comes behind the attention lies over what is dead by then
-      qkv = take(3 * D); xs = take(D); xn = att = take(D);
+    xs = static_cast<char*>(a.half ? a.out2 : a.out);
+    if (a.scoring) {
+      // no backward pass follows: q|k|v 3 D, xn D and, over it when the projection has read it, the attention's output; what comes
+      // behind the attention lies over what is dead by then
+      qkv = take(3 * D); xn = att = take(D);
       xs2 = qkv; xn2 = xs2 + N * D * 2; act = xn2 + N * D * 2;
     } else {
-      xs = take(D); xn = take(D); qkv = take(3 * D); att = take(D);
-      xs2 = take(half ? 0 : D); xn2 = take(half ? 0 : D); act = take(half ? 0 : M);
+      xn = take(D); qkv = take(3 * D); att = take(D);
+      xs2 = take(a.half ? 0 : D); xn2 = take(a.half ? 0 : D); act = take(a.half ? 0 : a.M);
     }
-    const long long nh = (N * H + 3) / 4 * 4;
+    const long long nh = (N * a.H + 3) / 4 * 4;
     lse = reinterpret_cast<float*>(p); rstd = lse + nh; gate = rstd + 2 * nh;
   }
 };
@@ -63,7 +66,7 @@ extern "C" int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s
   const ArbLayer& a = *args;
   if (bad_sizes(a) || !a.kept || !a.out || (a.half && !a.out2)) return -3;
   const long long N = a.B * a.T, D = a.H * 128;
-  const Kept k(a.kept, N, D, a.M, a.H, a.half, a.scoring);
+  const Kept k(a);
   const Gemm g{static_cast<int*>(a.err), s};
   const float eps = float(a.eps);
   const int* ids = static_cast<const int*>(a.ids);
@@ -93,14 +96,14 @@ extern "C" int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s
 }
 
 // a.group_dw: the four weight gradients leave in one launch at the end; d_h then has a place of its own.
-// a.work: bf16 [N, max(M, 4 D) + 2 D] (with group_dw [N, M + 4 D + 2 D], the value rows' gradients behind M + 3 D), then d_xn_gate [N, gate_ch], then (16-byte aligned, as is dgl) fp32 delta and dgl
-// [N, H] each.
+// a.work: bf16 [N, max(M, 4 D) + D] (with group_dw [N, M + 4 D + D], the value rows' gradients behind M + 3 D), then d_xn_gate
+// [N, gate_ch], then (16-byte aligned, as is dgl) fp32 delta and dgl [N, H] each.  a.d_x also holds d_xn2, d_att and d_xn in turn.
 // On return the value embedding's row gradients [N, D] lie behind the first 3 N D elements.
 extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s) {
   const ArbLayer& a = *args;
   if (bad_sizes(a) || !a.kept || !a.work || !a.d_x || !a.d_x0 || a.scoring || (a.half ? !a.out || (!a.g && !a.g_xn) : !a.g)) return -3;
   const long long N = a.B * a.T, D = a.H * 128;
-  const Kept k(a.kept, N, D, a.M, a.H, a.half, false);
+  const Kept k(a);
   const Gemm g{static_cast<int*>(a.err), s};
   const float eps = float(a.eps);
   const int* ids = static_cast<const int*>(a.ids);
@@ -109,7 +112,7 @@ extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s
   const long long wide = a.group_dw ? a.M + 4 * D : a.M > 4 * D ? a.M : 4 * D;
   char *dh = w, *dqkv = w + (a.group_dw ? N * a.M * 2 : 0);   // else d_h is dead when the attention backward writes d_qkv
   char* dve = dqkv + N * 3 * D * 2;
-  char *t1 = w + N * wide * 2, *g2 = t1 + N * D * 2;          // t1: d_xn2, then d_att, then d_xn
+  char *t1 = static_cast<char*>(a.d_x), *g2 = w + N * wide * 2;
   char* dxg = g2 + N * D * 2;
   float *delta = reinterpret_cast<float*>(dxg + (N * ch * 2 + 15) / 16 * 16), *dgl = delta + (N * H + 3) / 4 * 4;
   int n = 0;

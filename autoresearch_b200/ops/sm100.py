@@ -427,7 +427,7 @@ def _layer_forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids
     M, H = 0 if half else wfc.shape[0], D // 128
     stat = (N * H + 3) // 4 * 8                            # fp32 [N, H] in bf16 elements; lse, rstd of q and k, gate
     # without a backward pass the parts lie over each other (csrc/layer.cu): as much as the separate steps hold at their peak
-    cells = max(5 * N * D + 4 * stat, 2 * N * D + N * M) if scoring else N * ((6 if half else 8) * D + M) + 4 * stat
+    cells = max(4 * N * D + 4 * stat, 2 * N * D + N * M) if scoring else N * ((5 if half else 7) * D + M) + 4 * stat
     kept = torch.empty(cells, dtype=torch.bfloat16, device=x.device)
     out = torch.empty_like(x)
     group = int(2 * N * D * (4 * D + 2 * M) <= GROUP_DW_FLOPS)
@@ -454,7 +454,7 @@ def _layer_backward(ctx, g, g_xn):
     bufs = [_grad_buffer(p) if p is not None else (None, None) for p in params]
     accs = [b for b, _ in bufs]
     wide = M + 4 * D if group else max(M, 4 * D)
-    work = torch.empty(N * (wide + 2 * D + gate_ch) + 8 + 2 * ((N * H + 3) // 4 * 8), dtype=torch.bfloat16, device=dev)
+    work = torch.empty(N * (wide + D + gate_ch) + 8 + 2 * ((N * H + 3) // 4 * 8), dtype=torch.bfloat16, device=dev)
     dx = torch.empty_like(x)
     acc0 = chain.buf
     dx0 = acc0 if acc0 is not None else torch.empty_like(x)

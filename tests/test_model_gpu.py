@@ -292,3 +292,39 @@ def test_scoring_pass_holds_no_more_memory_than_the_separate_steps(heads, mlp, e
                 peak[whole] = torch.cuda.max_memory_allocated() - before
     assert torch.equal(out[True], out[False])
     assert peak[True] <= peak[False] + 16 * B * T * heads + (1 << 21), peak
+
+
+@pytest.mark.parametrize("group", [0.0, 6e10])
+def test_training_pass_keeps_no_more_per_layer_than_the_separate_steps(monkeypatch, group):
+    """Peak of forward and backward through six layers: what a layer keeps may not exceed what the separate steps keep (a width of D
+    more in each would be six).  Beside it the call in progress holds its scratch, M + 5 D columns (ungrouped max(M, 4 D) + D), the gate's
+    32, the statistics and two input gradients, where the separate steps' widest moment is d_h and its product, 5 D: with M = 4 D and
+    D = 256 that is 6 widths (2) and less than a quarter."""
+    from autoresearch_b200.config import ModelConfig
+    from autoresearch_b200.ops import sm100
+    monkeypatch.setattr(sm100, "GROUP_DW_FLOPS", group)
+    heads, B, T = 2, 8, 2048
+    D = 128 * heads
+    cfg = ModelConfig(vocab=512, seq_len=T, d_model=D, n_head=heads, head_dim=128, mlp_dim=4 * D, n_layer=6)
+    mod = _build("sm100", cfg, torch.bfloat16)
+    for p in mod.parameters():
+        p.main_grad = torch.zeros(p.shape, dtype=torch.float32, device="cuda")
+    ids = torch.randint(0, cfg.vocab, (B, T), device="cuda", dtype=torch.int32)
+    x = torch.randn(B * T, D, device="cuda").to(torch.bfloat16).requires_grad_()
+    g = torch.randn(B * T, D, device="cuda").to(torch.bfloat16)
+    kept, peak = {}, {}
+    for whole in (True, False):
+        mod.backend.layer_calls = whole
+        for _ in range(2):
+            x.grad = None
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            out = mod.run_layers(x, x, ids, B, T)
+            kept[whole] = torch.cuda.memory_allocated() - before
+            out.backward(g)
+            del out
+            torch.cuda.synchronize()
+            peak[whole] = torch.cuda.max_memory_allocated() - before
+    width = B * T * D * 2
+    assert kept[True] <= kept[False] + width // 4, (kept, width)
+    assert peak[True] <= peak[False] + (6 if group else 2) * width + width // 4 + (1 << 21), (peak, width)
