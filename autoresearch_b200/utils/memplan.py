@@ -120,12 +120,18 @@ def plan(mcfg: ModelConfig, micro_batch: int, *, dp: int = 1, tp: int = 1, ep: i
         p.step.append(("final norm in/out, d_xf, losses", 3 * Ns * D * a + Ns * 4))
         p.step.append(("logits chunk", min(ce_chunk, Ns) * V * a))
     # widest moment of the backward pass: d(out), d(hidden) or d(qkv) with the attention statistics, and two
-    # residual-stream gradients
+    # residual-stream gradients; the native call of a small layer holds d(hidden) beside d(qkv), for one launch of its weight gradients
+    from ..ops.sm100 import GROUP_DW_FLOPS
+    grouped = tp == 1 and 2 * N * D * (4 * D + 2 * M) <= GROUP_DW_FLOPS
     bwd = max(N * Ml * a + 2 * N * Dl * a, 2 * N * 3 * Dl * a + N * Dl * a + N * Hl * 4) + 4 * Ns * D * a
+    if grouped:
+        bwd = max(bwd, N * (M + 8 * D + m.ve_gate_ch) * a + 2 * N * H * 4 + 64)
     if tp > 1:
         bwd += 2 * N * D * a
     p.step.append(("backward temporaries", bwd))
-    p.step.append(("embedding-gradient plan + scratch", N * 24 + (N // 64 + V + 1) * D * 4))
+    # sort order, tables and per-chunk counts of the ids (the library operations of a large vocabulary take more per token)
+    tables = max(N * 24, N * 8 + (4 * V + N // 64 + 1) * 4 + (N + 1023) // 1024 * V * 4)
+    p.step.append(("embedding-gradient plan + scratch", tables + (N // 64 + V + 1) * D * 4))
     return p
 
 

@@ -58,3 +58,19 @@ def test_a_configuration_that_cannot_fit_is_refused_before_step_zero():
     with pytest.raises(MemoryError) as e:
         Trainer(cfg, t, device="cuda", quiet=True)
     assert "BATCH_SIZE" in str(e.value)
+
+
+@pytest.mark.parametrize("heads,batch,seq,vocab", [(2, 2, 512, 1024), (4, 1, 2048, 8192), (8, 4, 32768, 8192), (8, 16, 8192, 32768)])
+def test_plan_covers_what_the_layer_call_and_the_embedding_plan_take(heads, batch, seq, vocab):
+    """The scratch of one backward layer call with its incoming gradient and two input gradients, grouped weight gradients (small
+    layers) or not, and the tables of the embedding gradients: as ops/sm100.py and ops/kernels.py allocate them."""
+    from autoresearch_b200.config import ModelConfig
+    from autoresearch_b200.ops import sm100
+    D, N = 128 * heads, batch * seq
+    cfg = ModelConfig(vocab=vocab, seq_len=seq, d_model=D, n_head=heads, head_dim=128, mlp_dim=4 * D, n_layer=6)
+    step = dict(memplan.plan(cfg, batch).step)
+    grouped = 2 * N * D * (4 * D + 2 * 4 * D) <= sm100.GROUP_DW_FLOPS
+    work = N * ((8 * D if grouped else 4 * D) + D + cfg.ve_gate_ch) + 4 * N * heads
+    assert step["backward temporaries"] >= 2 * (work + 3 * N * D)
+    tables = 8 * N + 4 * (3 * vocab + N // 64 + vocab + 1) + 4 * ((N + 1023) // 1024) * vocab
+    assert step["embedding-gradient plan + scratch"] >= tables + (N // 64 + vocab + 1) * D * 4
