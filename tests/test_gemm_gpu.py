@@ -273,12 +273,20 @@ def test_few_tiles_and_just_too_many(M, N, Kd):
     K.check_err_flag()
 
 
+@pytest.mark.parametrize("own_stream", [False, True])
 @pytest.mark.parametrize("Kd,shapes", [(1, [(8, 8)]), (130, [(256, 256), (264, 512)]), (2048, [(1536, 512), (2048, 512), (512, 2048), (512, 512)]),
                                        (993, [(1152, 384), (1536, 384), (384, 1536), (384, 384)]), (8000, [(128, 128), (384, 128), (512, 128)])])
-def test_grouped_weight_gradients(Kd, shapes):
+def test_grouped_weight_gradients(Kd, shapes, own_stream):
     """One launch against 64 bits: one row, ragged tiles and K, splits that do and do not divide the K blocks; fp32 sums of Kd
-    products of bf16 values, and rows around the outputs that stay untouched."""
+    products of bf16 values, and rows around the outputs that stay untouched; on the default stream and on another, whose operands are
+    made on it just before."""
     import ctypes as C
+    from contextlib import nullcontext
+    with torch.cuda.stream(torch.cuda.Stream()) if own_stream else nullcontext():
+        _grouped_weight_gradients(C, Kd, shapes)
+
+
+def _grouped_weight_gradients(C, Kd, shapes):
     from autoresearch_b200.ops import kernels as K
     torch.manual_seed(Kd)
     dy = [torch.randn(Kd, m, device="cuda").bfloat16() for m, _ in shapes]

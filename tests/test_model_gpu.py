@@ -66,17 +66,8 @@ def test_training_step_sm100_loss_decreases():
     assert losses[-1] < losses[0] - 0.3, losses
 
 
-@pytest.mark.parametrize("batch,seq,layers,heads,experts", [(1, 512, 4, 2, 0), (3, 331, 6, 2, 0), (1, 130, 2, 2, 0), (3, 301, 3, 3, 0),
-                                                            (1, 3, 1, 1, 0), (2, 300, 3, 2, 4), (1, 130, 2, 3, 4)])
-def test_whole_layer_calls_give_the_bits_of_the_separate_steps(batch, seq, layers, heads, experts):
-    """One native call per layer and direction against one autograd node per step: the same kernels on the same operands, so
-    losses agree bit for bit and matrix gradients up to the order in which split-K sums meet.  130 rows take the separate
-    rotation kernel (products below the 2-CTA tiles), 993 end inside a tile, 903 x 3 leaves the row statistics at odd offsets."""
-    from autoresearch_b200.config import ModelConfig, MoEConfig
+def _assert_whole_layers_match_the_steps(cfg, batch, seq):
     from autoresearch_b200.ops import kernels as K
-    moe = MoEConfig(n_experts=experts, top_k=2, mlp_dim_e=512 * heads, capacity_factor=1.25) if experts else None
-    cfg = ModelConfig(vocab=1024, seq_len=512, d_model=128 * heads, n_head=heads, head_dim=128, mlp_dim=512 * heads,
-                      n_layer=layers, moe=moe)
     torch.manual_seed(3)
     mod = _build("sm100", cfg, torch.bfloat16)
     ids = torch.randint(0, cfg.vocab, (batch, seq), device="cuda", dtype=torch.int32)
@@ -108,6 +99,32 @@ def test_whole_layer_calls_give_the_bits_of_the_separate_steps(batch, seq, layer
             else:
                 # fp32 split-K sums meet in L2 in any order: a few units in the last place of the largest partial sum
                 assert (x.float() - y.float()).norm() <= (1e-5 if with_main else 4e-3) * y.float().norm(), n
+
+
+def _layers_cfg(heads, layers, mlp, experts):
+    from autoresearch_b200.config import ModelConfig, MoEConfig
+    moe = MoEConfig(n_experts=experts, top_k=2, mlp_dim_e=mlp, capacity_factor=1.25) if experts else None
+    return ModelConfig(vocab=1024, seq_len=512, d_model=128 * heads, n_head=heads, head_dim=128, mlp_dim=mlp, n_layer=layers, moe=moe)
+
+
+@pytest.mark.parametrize("batch,seq,layers,heads,experts", [(1, 512, 4, 2, 0), (3, 331, 6, 2, 0), (1, 130, 2, 2, 0), (3, 301, 3, 3, 0),
+                                                            (1, 3, 1, 1, 0), (2, 300, 3, 2, 4), (1, 130, 2, 3, 4)])
+def test_whole_layer_calls_give_the_bits_of_the_separate_steps(batch, seq, layers, heads, experts):
+    """One native call per layer and direction against one autograd node per step: the same kernels on the same operands (the weight
+    gradients of layers as small as these leave in one grouped launch), so losses agree bit for bit and matrix gradients up to the
+    order in which split-K sums meet.  130 rows take the separate rotation kernel (products below the 2-CTA tiles), 993 end inside a
+    tile, 903 x 3 leaves the row statistics at odd offsets."""
+    _assert_whole_layers_match_the_steps(_layers_cfg(heads, layers, 512 * heads, experts), batch, seq)
+
+
+@pytest.mark.parametrize("group", [0.0, float("inf")])
+@pytest.mark.parametrize("heads,mlp,experts", [(2, 1024, 0), (2, 1288, 0), (2, 520, 0), (1, 2048, 0), (2, 1024, 4)])
+def test_whole_layer_calls_with_grouped_and_separate_weight_gradients(monkeypatch, group, heads, mlp, experts):
+    """Both scratch layouts of the backward call, with MLPs of four widths, wider and narrower: d_h over d_qkv and the value rows, or in
+    a place of its own."""
+    from autoresearch_b200.ops import sm100
+    monkeypatch.setattr(sm100, "GROUP_DW_FLOPS", group)
+    _assert_whole_layers_match_the_steps(_layers_cfg(heads, 3, mlp, experts), 3, 331)
 
 
 def test_captured_pass_follows_its_inputs():
