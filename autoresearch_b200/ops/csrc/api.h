@@ -186,11 +186,11 @@ int arb_muon_nesterov_rs(float* buf, const void* const* peer_buckets, int world,
 int arb_adamw_rs(float* master, const void* const* peer_buckets, int world, int rank, const void* mc_bucket,
                  long long bucket_offset, float grad_scale, float* m, float* v, void* shadow_bf16, long long n,
                  float lr, float beta1, float beta2, float eps, float wd, float bc1, float bc2, cudaStream_t s);
-// x = u / (sqrt(sum of partials[mat][0..63])*1.02 + 1e-6)
 // The whole step of n_mat small matrices (short side <= 64, at most 16384 elements): momentum, normalisation, `steps`
 // Newton-Schulz iterations with coefficients abc[3 * steps] (host), NorMuon, cautious update of master and bf16 parameter.
 int arb_muon_small(float* buf, const float* grad, float* second, float* master, void* shadow_bf16, int n_mat, int m, int n, float mu,
                    float lr, float wd, float beta2, const float* abc, int steps, cudaStream_t s);
+// x = u / (sqrt(sum of partials[mat][0..63])*1.02 + 1e-6)
 int arb_muon_frob_scale(void* u_bf16, const float* partials, long long per_mat, int n_mat, cudaStream_t s);
 // NorMuon statistics + cautious update, per matrix [m, n]; reduce over columns if m >= n.
 int arb_normuon_stats(const void* x_bf16, float* v_mean, int n_mat, int m, int n, cudaStream_t s);
@@ -252,7 +252,8 @@ int arb_moe_combine_bwd(const void* d_out, void* const* y_bufs, const void* y_ro
                         const int* idx, const int* row, const float* gates, float* d_gates, long long N, int K, int D,
                         int E, cudaStream_t s);
 
-// ---- one dense layer per call (layer.cu): the same kernels as the entry points above, started from native code ----
+// ---- a layer per call (layer.cu): the launches of the entry points above from native code; the weight gradients of a small layer
+//      in one launch (group_dw) ----
 typedef struct {
   // forward: inputs, parameters, the buffer for what the layer keeps (bf16 [N, 7 D + M] then four times
   // fp32 [N, H], each rounded up to 4 floats), output [N, D]
@@ -267,7 +268,7 @@ typedef struct {
   double eps, scale;
 } ArbLayer;
 // half: the layer up to its second norm (what comes before the experts of an expert layer): out = the residual stream, out2 = its
-// norm, M = 0, kept without their copies; backward: out as input, g and g_xn their gradients (either may be null, not both).
+// norm, M = 0, kept without their copies; backward: out as input, g and g_xn their gradients.
 // scoring: no backward call follows; kept is then scratch of max(4 D and the statistics, 2 D + M) columns.
 int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s);
 int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s);

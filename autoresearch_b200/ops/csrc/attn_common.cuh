@@ -26,9 +26,10 @@ struct AttnArgs {
 
 // Which tile of which head a CTA of the flat grid takes.  The (sequence, head) pairs go in groups of p.group; inside a group the
 // pair changes fastest and the tile rank (0 = most work) slowest, so the long tiles of a whole group start first and its last
-// wave is made of short ones.  One pair after the other instead leaves the last pair's long tiles for the end: full causal,
-// B=1 H=16 T=8192: 328 us, grouped 277; B=1 H=16 T=4096: 120, 82.  All pairs in one group lose their K and V between a tile and
-// the next once they outgrow L2: B=64 H=4 T=2048: 403 us, one after the other 361.
+// wave is made of short ones.  Full causal, us, one pair after the other / groups of attn_group() / all pairs interleaved: B=1 H=16
+// T=8192 328 / 305 / 277; B=1 H=16 T=4096 120 / 80 / 82 (one group in both); B=64 H=4 T=2048 361 / 342 / 403.  One pair after the
+// other leaves the last pair's long tiles for the end; all pairs interleaved lose their K and V between a tile and the next once
+// they outgrow L2.  The first of these shapes would still gain from one group (K and V of 64 MB), where the rule makes 12 and 4.
 struct AttnTile { int rank, h, b; };
 __device__ __forceinline__ AttnTile attn_tile(const AttnArgs& p, int n_tiles, int block = int(blockIdx.x)) {
   const int per = p.group * n_tiles, g = block / per, i = block - g * per;

@@ -1,11 +1,12 @@
-// One dense transformer layer per call: the launch sequences of the forward and the backward pass of a layer that is
-// neither tensor- nor expert-parallel.  Host code only; every kernel it starts is the one that the separate entry points
-// start, in the same order and with the same arguments, so results do not change.
+// A transformer layer per call: the launch sequences of the forward and the backward pass of a dense layer that is not
+// tensor-parallel, and of what precedes the experts of an expert layer.  Host code only.  The kernels are those that the separate
+// entry points start, in the same order and on the same operands, with one exception: the weight gradients of a small layer
+// (group_dw) leave in one launch at the end of the backward pass (gemm_sm100.cu), whose K splits add up in another order.
 //
-// Why: a layer is 7 launches forward and 17 to 21 backward.  Through one Python call and one autograd node per kernel a launch
-// cost 25 us of host time, four times what a kernel of a small batch runs.  Measured, per step -> per layer: training pass of
-// the 119.5 M model on one sequence of 2048 15.4 -> 8.6 ms (GPU work 7.4); small model, 512 tokens scored 0.95 -> 0.46 ms, 1024
-// tokens trained 2.70 -> 1.32 ms.
+// Why: a dense layer is 7 launches forward (8 with the rotation as its own kernel) and 13 backward (15 with a value embedding; three
+// fewer with grouped weight gradients).  Through one Python call and one autograd node per kernel a launch cost 25 us of host
+// time, four times what a kernel of a small batch runs.  Measured, per step -> per layer (ungrouped): training pass of the 119.5 M model on one sequence of 2048 15.4 -> 8.6 ms (GPU work 7.4); small
+// model, 512 tokens scored 0.95 -> 0.46 ms, 1024 tokens trained 2.70 -> 1.32 ms.
 //
 // Math and order: brain/src/forward.rs:359-739, brain/src/backward.rs:203-877.
 #include "api.h"
@@ -101,7 +102,7 @@ extern "C" int arb_layer_fwd(const ArbLayer* args, int* launches, cudaStream_t s
 // On return the value embedding's row gradients [N, D] lie behind the first 3 N D elements.
 extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s) {
   const ArbLayer& a = *args;
-  if (bad_sizes(a) || !a.kept || !a.work || !a.d_x || !a.d_x0 || a.scoring || (a.half ? !a.out || (!a.g && !a.g_xn) : !a.g)) return -3;
+  if (bad_sizes(a) || !a.kept || !a.work || !a.d_x || !a.d_x0 || !a.g || a.scoring || (a.half && (!a.out || !a.g_xn))) return -3;
   const long long N = a.B * a.T, D = a.H * 128;
   const Kept k(a);
   const Gemm g{static_cast<int*>(a.err), s};
@@ -116,10 +117,8 @@ extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s
   char* dxg = g2 + N * D * 2;
   float *delta = reinterpret_cast<float*>(dxg + (N * ch * 2 + 15) / 16 * 16), *dgl = delta + (N * H + 3) / 4 * 4;
   int n = 0;
-  const void* gs = g2;                                        // gradient of xs2
   if (a.half) {
-    if (a.g_xn) ARB_TRY(arb_rmsnorm_bwd(a.out, a.g_xn, a.g, g2, N, int(D), eps, s));
-    else gs = a.g;
+    ARB_TRY(arb_rmsnorm_bwd(a.out, a.g_xn, a.g, g2, N, int(D), eps, s));
   } else {
     // MLP: out = xs2 + relu(xn2 wfc^T)^2 wdn^T
     ARB_TRY(g.nn(a.g, a.wdn, dh, k.act, N, a.M, D, EPI_RELU2_BWD));
@@ -130,9 +129,9 @@ extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s
     ARB_TRY(g.nn(dh, a.wfc, t1, nullptr, N, D, a.M, EPI_STORE_BF16));
     ARB_TRY(arb_rmsnorm_bwd(k.xs2, t1, a.g, g2, N, int(D), eps, s));
   }
-  // attention: xs2 = xs + att wo^T
-  ARB_TRY(g.nn(gs, a.wo, t1, nullptr, N, D, D, EPI_STORE_BF16));
-  if (!a.group_dw) ARB_TRY(g.dw(gs, k.att, a.g_wo, D, D, N));
+  // attention: xs2 = xs + att wo^T; g2 is the gradient of xs2
+  ARB_TRY(g.nn(g2, a.wo, t1, nullptr, N, D, D, EPI_STORE_BF16));
+  if (!a.group_dw) ARB_TRY(g.dw(g2, k.att, a.g_wo, D, D, N));
   ARB_TRY(arb_attn_bwd(k.qkv, k.qkv + 2 * D, k.qkv + 4 * D, k.att, t1, k.lse, dqkv, dqkv + 2 * D, dqkv + 4 * D, delta, nullptr, int(a.B),
                        T, H, 3 * D, 3 * D, 3 * D, D, D, 3 * D, 3 * D, 3 * D, int(a.window), float(a.scale), g.err, s));
   ARB_TRY(arb_qkv_post_bwd(dqkv, k.qkv, a.cos_t, a.sin_t, k.rstd, k.xn, ids, a.ve, a.ve ? a.gate_w : nullptr, a.ve ? k.gate : nullptr,
@@ -141,10 +140,10 @@ extern "C" int arb_layer_bwd(const ArbLayer* args, int* launches, cudaStream_t s
   if (!a.group_dw) ARB_TRY(g.dw(dqkv, k.xn, a.g_wqkv, 3 * D, D, N));
   ARB_TRY(g.nn(dqkv, a.wqkv, t1, nullptr, N, D, 3 * D, EPI_STORE_BF16));
   if (a.ve) ARB_TRY(arb_add_cols(t1, D, dxg, N, ch, s));
-  ARB_TRY(arb_resid_scale_norm_bwd(a.x, a.x0, a.lam_r, a.lam_0, int(a.idx), gs, t1, a.d_x, a.d_x0, a.d_x0_acc,
+  ARB_TRY(arb_resid_scale_norm_bwd(a.x, a.x0, a.lam_r, a.lam_0, int(a.idx), g2, t1, a.d_x, a.d_x0, a.d_x0_acc,
                                    static_cast<float*>(a.g_lam_r), static_cast<float*>(a.g_lam_0), N, int(D), eps, s));
   if (a.group_dw) {
-    const void *dy[4] = {dqkv, gs, a.g, dh}, *x[4] = {k.xn, k.att, k.act, k.xn2};
+    const void *dy[4] = {dqkv, g2, a.g, dh}, *x[4] = {k.xn, k.att, k.act, k.xn2};
     float* c[4] = {static_cast<float*>(a.g_wqkv), static_cast<float*>(a.g_wo), static_cast<float*>(a.g_wdn), static_cast<float*>(a.g_wfc)};
     const int d = int(D), f = int(a.M), rows[4] = {3 * d, d, d, f}, cols[4] = {d, d, f, d};
     ARB_TRY(arb_gemm_dw_group(dy, x, c, rows, cols, a.half ? 2 : 4, int(N), g.err, s));

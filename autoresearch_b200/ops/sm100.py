@@ -449,7 +449,7 @@ def _layer_backward(ctx, g, g_xn):
     dev = x.device
     if K.pending_pulls:
         K.flush_pending_pulls()
-    g, g_xn = (t.contiguous() if t is not None else None for t in (g, g_xn))
+    g, g_xn = g.contiguous(), g_xn.contiguous() if half else None
     params = (lam_r, lam_0, wqkv, wo, wfc, wdn, gate_w)
     bufs = [_grad_buffer(p) if p is not None else (None, None) for p in params]
     accs = [b for b, _ in bufs]
@@ -483,9 +483,9 @@ def _layer_backward(ctx, g, g_xn):
 
 
 class DenseLayerFn(torch.autograd.Function):
-    """A whole dense layer, launched by one native call per direction (csrc/layer.cu): the kernels, their order and their
-    arguments are those of ResidScaleNormFn, AttnPreFn, AttentionFn, LinearAddNormFn and MLPFn in a row.  What the layer
-    keeps for its backward pass is one buffer."""
+    """A whole dense layer, launched by one native call per direction (csrc/layer.cu): the kernels and their order are those of
+    ResidScaleNormFn, AttnPreFn, AttentionFn, LinearAddNormFn and MLPFn in a row, except that a small layer's weight gradients leave in
+    one launch at the end of the backward call.  What the layer keeps for its backward pass is one buffer."""
 
     @staticmethod
     def forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, *rest):
