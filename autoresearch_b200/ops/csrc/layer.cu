@@ -5,8 +5,8 @@
 //
 // Why: a dense layer is 7 launches forward (8 with the rotation as its own kernel) and 13 backward (15 with a value embedding; three
 // fewer with grouped weight gradients).  Through one Python call and one autograd node per kernel a launch cost 25 us of host
-// time, four times what a kernel of a small batch runs.  Measured, per step -> per layer (ungrouped): training pass of the 119.5 M model on one sequence of 2048 15.4 -> 8.6 ms (GPU work 7.4); small
-// model, 512 tokens scored 0.95 -> 0.46 ms, 1024 tokens trained 2.70 -> 1.32 ms.
+// time, four times what a kernel of a small batch runs.  Measured, per step -> per layer (ungrouped): training pass of the 119.5 M model on one sequence of
+// 2048 15.4 -> 8.6 ms (GPU work 7.4); small model, 512 tokens scored 0.95 -> 0.46 ms, 1024 tokens trained 2.70 -> 1.32 ms.
 //
 // Math and order: brain/src/forward.rs:359-739, brain/src/backward.rs:203-877.
 #include "api.h"
