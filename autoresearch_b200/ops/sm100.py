@@ -712,7 +712,8 @@ class Sm100Backend(OracleBackend):
         self.attn = attn
         self.big_ce_chunk = 16384
         self.layer_calls = True       # False: one autograd node and one native call per step of a layer
-        self._pass = None
+        self._pass = None             # the forward pass in progress, and the same for the layer whose steps run one by one
+        self._layer_pass = None
 
     def optim_kernels(self):
         if getattr(self, "_optim_kernels", None) is None:
@@ -734,7 +735,8 @@ class Sm100Backend(OracleBackend):
         return self._pass
 
     def resid_scale_norm(self, x, x0, lam_r, lam_0, i):
-        return ResidScaleNormFn.apply(x.contiguous(), x0.contiguous(), lam_r, lam_0, i, self.eps, self._chain(i))
+        self._layer_pass = self._chain(i)
+        return ResidScaleNormFn.apply(x.contiguous(), x0.contiguous(), lam_r, lam_0, i, self.eps, self._layer_pass)
 
     def _one_call(self, x, x0, lam_r, lam_0, blk, ids_flat, B, T, cfg, cos, sin):
         """Whether a layer can go through one native call: not under tensor parallelism, with the library attention or while
@@ -803,8 +805,10 @@ class Sm100Backend(OracleBackend):
         H = blk.wqkv.shape[0] // (3 * cfg.head_dim)
         if cfg.head_dim != 128:
             raise ValueError("the sm100 kernels support head_dim = 128 only")
+        # taken once: a block that is called by itself, outside of a pass through the layers, shares nothing with an earlier one
+        of_pass, self._layer_pass = self._layer_pass, None
         qkv = AttnPreFn.apply(xn, blk.wqkv, ids_flat, blk.ve, blk.ve_gate, cos, sin, T, H, cfg.ve_gate_ch, self.eps,
-                              fused_tp, self._pass)
+                              fused_tp, of_pass)
         fn = AttentionFn if self.attn == "own" else LibraryAttentionFn
         return fn.apply(qkv, B, T, H, window)
 

@@ -231,6 +231,24 @@ def test_direct_pass_on_the_capture_stream_does_not_take_the_captured_plan():
     K.check_err_flag()
 
 
+def test_steps_of_one_pass_share_a_plan_and_a_block_called_by_itself_makes_its_own(monkeypatch):
+    from autoresearch_b200.ops import kernels as K
+    t = _TrainingPass()
+    be, cfg = t.mod.backend, t.cfg
+    be.layer_calls = False
+    made, make = [], K._embedding_plan
+    monkeypatch.setattr(K, "_embedding_plan", lambda ids, vocab: made.append(1) or make(ids, vocab))
+    t.run()
+    assert len(made) == 1
+    blk = next(b for b in t.mod.blocks if b.ve is not None)
+    B, T = t.ids.shape
+    for n in (2, 3):
+        xn = torch.randn(B * T, cfg.d_model, device="cuda").to(torch.bfloat16).requires_grad_()
+        be.attention_block(xn, blk, t.ids.reshape(-1), B, T, cfg, t.mod.rope_cos, t.mod.rope_sin, T).float().sum().backward()
+        assert len(made) == n and len(K._emb_plan) == 0
+    K.check_err_flag()
+
+
 def test_direct_pass_after_a_replay_that_refills_the_ids():
     """The captured pass copies its ids in, which raises no version at replay; a direct pass then sees the new ids."""
     from autoresearch_b200.ops import kernels as K
