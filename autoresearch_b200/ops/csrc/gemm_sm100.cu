@@ -1314,9 +1314,9 @@ extern "C" int arb_gemm_bf16_ragged(const void* A, const void* B, void* C, const
   if (sym) {
     // The caller vouches for a symmetric result.  Mirrored from four tiles a side: 428 M model (1024 a side), optimizer update
     // 11.12 -> 10.40 ms; at two a side (3 of 4 tiles left, main loops of 8 K blocks) the transposed stores cost more than the
-    // skipped tile: 119.5 M model 2.25 -> 2.39 ms.
+    // skipped tile: 119.5 M model 2.25 -> 2.39 ms.  The transposes are written two rows at a time: even sides only.
     if (M != N || m_valid || k_valid || (a_mn_major != b_mn_major)) return -3;
-    if (!pair || M <= 768 || (epi == EPI_SYM_NS_COMBINE && a_mn_major)) epi = epi == EPI_SYM_STORE ? EPI_STORE_BF16 : EPI_NS_COMBINE;
+    if (!pair || M <= 768 || (M & 1) || (epi == EPI_SYM_NS_COMBINE && a_mn_major)) epi = epi == EPI_SYM_STORE ? EPI_STORE_BF16 : EPI_NS_COMBINE;
   }
   const int bm_eff = pair ? 256 : BM;
   GemmArgs a;

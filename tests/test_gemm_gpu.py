@@ -304,3 +304,23 @@ def _grouped_weight_gradients(C, Kd, shapes):
         ref = 0.25 + a.double().t() @ b.double()
         assert (c.double() - ref).abs().max() <= 2e-6 * (a.double().abs().t() @ b.double().abs()).max() + 1e-6
         assert (full[0] == 0.25).all() and (full[-1] == 0.25).all()
+
+
+def test_symmetric_product_of_an_odd_side_writes_what_the_plain_product_writes():
+    """The transposes are stored as pairs of rows: with an odd side the last pair would reach into the padding of a row.  Every tile is
+    computed then, and the bits are those of the plain product, in the padding (whose rest of 16 bytes a tile store fills) too."""
+    from autoresearch_b200.ops import kernels as K
+    torch.manual_seed(11)
+    d, ld = 1001, 1008
+    x = (torch.randn(d, 128, device="cuda") * 0.1).to(torch.bfloat16)
+    buf, aux, full = (torch.full((d, ld), 3.0, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    K.gemm(x, x, out=full[:, :d])
+    K.gemm(x, x, out=buf[:, :d], epi=K.EPI_SYM_STORE)
+    assert torch.equal(buf, full)
+    aux[:, :d] = full[:, :d]
+    got = []
+    for epi in (K.EPI_NS_COMBINE, K.EPI_SYM_NS_COMBINE):
+        got.append(torch.full_like(buf, 3.0))
+        K.gemm(full[:, :d], full[:, :d], out=got[-1][:, :d], epi=epi, aux=aux[:, :d], alpha=3.4, beta=-4.7, gamma=2.0)
+    assert torch.equal(*got)
+    K.check_err_flag()
