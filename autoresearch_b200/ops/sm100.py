@@ -430,7 +430,7 @@ def _layer_forward(ctx, x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids
     cells = max(4 * N * D + 4 * stat, 2 * N * D + N * M) if scoring else N * ((5 if half else 7) * D + M) + 4 * stat
     kept = torch.empty(cells, dtype=torch.bfloat16, device=x.device)
     out = torch.empty_like(x)
-    group = int(2 * N * D * (4 * D + 2 * M) <= GROUP_DW_FLOPS)
+    group = int(K._gemm_mode != 1 and 2 * N * D * (4 * D + 2 * M) <= GROUP_DW_FLOPS)      # the grouped launch has 2-CTA tiles
     sizes = (B, T, H, M, window, idx, gate_ch, int(K.qkv_post_fusable(N, 3 * D)), group, int(half), int(scoring))
     ptrs = [t.data_ptr() if t is not None else 0 for t in (x, x0, lam_r, lam_0, wqkv, wo, wfc, wdn, ve, gate_w, ids, cos, sin)]
     ptrs += (kept.data_ptr(), out.data_ptr(), out2.data_ptr() if half else 0, K.err_flag(x.device).data_ptr())

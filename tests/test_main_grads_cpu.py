@@ -54,3 +54,18 @@ def test_strided_main_gradients_take_the_sum_and_nothing_beside_them_changes(cal
 def test_main_gradients_that_the_products_cannot_add_into_are_refused(call, main):
     with pytest.raises(ValueError):
         call(dict(wo=main))
+
+
+@pytest.mark.parametrize("mode,grouped", [(0, True), (1, False), (2, True)])
+def test_grouped_weight_gradients_follow_the_tile_mode(monkeypatch, mode, grouped):
+    """The grouped launch has 2-CTA tiles: with the mode that asks for 1-CTA tiles the gradients stay separate products."""
+    seen = []
+    monkeypatch.setattr(K, "layer_call", lambda entry, pointers, sizes, eps, scale: seen.append(sizes))
+    monkeypatch.setattr(K, "err_flag", lambda device=None: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(K, "_gemm_mode", mode)
+    D, M = 128, 512
+    w = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    ctx = SimpleNamespace(save_for_backward=lambda *t: None)
+    sm100._layer_forward(ctx, w(4, D), w(4, D), w(1), w(1), w(3 * D, D), w(D, D), w(M, D), w(D, M), None, None, w(4), w(4, 64), w(4, 64),
+                         1, 4, 4, 0, 32, 1e-5, None, False, None)
+    assert [s[8] for s in seen] == [int(grouped)]
